@@ -6,14 +6,21 @@
 // stack: popping node X allots node records to X's inner children (left, then
 // right) and appends the Woop triangles of X's leaf children (left, then
 // right, each followed by a 0x80000000 terminator).  Nodes are therefore
-// popped in right-first preorder.  Here:
-//   1. bottom-up: per node, inner-node count of its subtree I, its number of
-//      inner children, and the Woop entries of its leaf children;
-//   2. pointer jumping over inner nodes: pop rank
-//        rank(X) = sum over the path of 1 + [X' is a left child] * I(sibling),
-//      depth, and whether a leaf of the collapsed tree lies above (unreached);
-//   3. scatter by rank, two exclusive scans -> node slot and Woop offset;
-//   4. one thread per reachable inner node writes its 64-byte record and its
+// popped in right-first preorder, and everything popped before a node X is its
+// ancestors and, for every node of its path that is an inner left child, the
+// right sibling's whole subtree.  A subtree of I inner nodes allots I - 1
+// records below its root's, so the two running totals at X -- records allotted
+// (S) and Woop entries written (W) before X is popped -- are sums over X's path
+// of per-node steps that need subtree totals only:
+//   S(c) = S(P) + inner children of P + [c left, sibling r inner] (I(r) - 1)
+//   W(c) = W(P) + entries of P's leaf children + [c left, r inner] TW(r)
+// and X's own record is 1 + S(P), plus one for a right child beside an inner
+// left one.  Hence three passes and no scan, rank order or jump rounds:
+//   1. bottom-up: subtree totals (I, TW); the thread that finishes a node
+//      writes its inner children's steps;
+//   2. the nodes with at least kTopInner inner nodes below sum their whole path;
+//   3. every other node walks up to the nearest of those (a few links), and the
+//      thread of each reachable inner node writes its 64-byte record and its
 //      leaf children's Woop triangles.
 // The Woop transform restates FW::MatrixBase::inverted
 // (gpu-ray-traversal/src/framework/base/Math.hpp:961-983, 3x3 determinant
@@ -24,13 +31,11 @@
 
 namespace atr {
 
-int exclusive_scan_u32(atr_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* d_total);
-
 namespace {
 
-constexpr int kPendingWord = 8;    // flags[8 + r * kPendingStride]: jumps left after round r (r < 34)
-constexpr int kPendingStride = 8;  // one 32-byte sector per round
-constexpr size_t kFlagBytes = 4 * (kPendingWord + 34 * kPendingStride);
+// Nodes whose subtree holds at least this many inner nodes sum their path to
+// the root once (pass 2); the walks of pass 3 stop at the nearest of them.
+constexpr uint32_t kTopInner = 32;
 
 struct FlatRefs {
     const int32_t* parent;
@@ -62,166 +67,128 @@ __device__ __forceinline__ SegPos seg_pos(const Segs& segs, uint32_t gi) {
 }
 
 __device__ __forceinline__ bool c_leaf(const FlatRefs& t, int nb, int x) { return t.data[nb + x] >= 0; }
-__device__ __forceinline__ uint32_t woop_entries(const FlatRefs& t, int nb, int x) {
-    const int c = t.count[nb + x];
-    return 3u * (uint32_t)(c > 1 ? c : 1) + 1u;
+
+// A node's step from its parent: x the parent (local; -1 at the root), y the
+// S step (-1: the parent is a leaf of the collapsed tree, so nothing below it
+// is part of the layout), z the W step, w the inner nodes of the node's
+// subtree, with kRightOfInner set for a right child beside an inner left one.
+// Written for inner nodes only, so a walk must not start at a collapsed leaf.
+constexpr uint32_t kRightOfInner = 0x80000000u;
+__device__ __forceinline__ uint32_t step_inner(const int4& s) { return (uint32_t)s.w & ~kRightOfInner; }
+
+// Pass 1.  A child's totals reach its parent through the parent's 64-bit slot
+// (bit 63 marks them present, then I, then TW): the first arrival exchanges
+// its totals in and stops, the second takes the sibling's out of the exchange.
+// A leaf's I is 0 and an inner node's at least 1, so the totals also tell the
+// two apart and a child's own arrays are not read.  Nothing else read here is
+// written by this pass, so the exchanges need no ordering, and the next node's
+// links load while the exchange is in flight.
+__device__ __forceinline__ unsigned long long pack_totals(uint32_t inner, uint32_t tw) {
+    return (1ull << 63) | ((unsigned long long)inner << 32) | tw;
 }
 
-// Pass 1: per inner node, inner nodes in its subtree, inner children, Woop
-// entries of its leaf children (inner arrays are indexed cb + local index).
-// A child's inner-node count reaches its parent through the parent's 64-bit
-// slot (bit 32 marks it present): the first arrival exchanges its count in
-// and stops, the second takes the sibling's out of the exchange.  Nothing
-// else read here is written by this pass, so the exchanges need no ordering,
-// and the next node's links load while the exchange is in flight.
-__global__ void __launch_bounds__(256) k_flat_counts(FlatRefs t, Segs segs, uint32_t* __restrict__ icnt,
-                                                      uint32_t* __restrict__ ic, uint32_t* __restrict__ tw,
-                                                      unsigned long long* __restrict__ slots) {
+__global__ void __launch_bounds__(256) k_flat_counts(FlatRefs t, Segs segs, int4* __restrict__ step,
+                                                      unsigned long long* __restrict__ slots,
+                                                      int64_t* __restrict__ nodes_out, int64_t* __restrict__ woop_out,
+                                                      int64_t* __restrict__ depth_out) {
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gi == 0) *depth_out = 0;
     if (gi >= segs.n) return;
     const SegPos q = seg_pos(segs, gi);
     int ch = (int)q.li + (int)q.n - 1;
     int cur = t.parent[q.nb + ch];
     if (cur < 0) return;
-    uint32_t mine = 0u;  // inner nodes below ch counted by the parent (none under a leaf)
-    int l = t.left[q.nb + cur], r = t.right[q.nb + cur], up = t.parent[q.nb + cur];
-    bool cleaf = c_leaf(t, q.nb, cur);
+    uint32_t mi = 0u, mw = 4u;  // inner nodes and Woop entries below ch: one triangle and its terminator
+    int l = t.left[q.nb + cur], r = t.right[q.nb + cur], up = t.parent[q.nb + cur], dat = t.data[q.nb + cur];
     while (true) {
-        int nl = 0, nr = 0, nup = -1;
-        bool ncleaf = false;
+        int nl = 0, nr = 0, nup = -1, ndat = -1;
         if (up >= 0) {
             nl = t.left[q.nb + up];
             nr = t.right[q.nb + up];
             nup = t.parent[q.nb + up];
-            ncleaf = c_leaf(t, q.nb, up);
+            ndat = t.data[q.nb + up];
         }
-        const bool ll = c_leaf(t, q.nb, l), rl = c_leaf(t, q.nb, r);
-        const unsigned long long other = atomicExch(slots + q.cb + cur, (1ull << 32) | mine);
+        const unsigned long long other = atomicExch(slots + q.cb + cur, pack_totals(mi, mw));
         if (other == 0ull) return;
-        const uint32_t sib = (uint32_t)other;
+        const uint32_t si = (uint32_t)(other >> 32) & 0x7fffffffu, sw = (uint32_t)other;
         const bool from_left = ch == l;
-        const uint32_t il = from_left ? mine : sib, ir = from_left ? sib : mine;
-        const uint32_t v = cleaf ? 0u : 1u + il + ir;
-        icnt[q.cb + cur] = v;
-        ic[q.cb + cur] = (ll ? 0u : 1u) + (rl ? 0u : 1u);
-        tw[q.cb + cur] = (ll ? woop_entries(t, q.nb, l) : 0u) + (rl ? woop_entries(t, q.nb, r) : 0u);
-        if (up < 0) return;
-        mine = v;
+        const uint32_t il = from_left ? mi : si, ir = from_left ? si : mi;
+        const uint32_t wl = from_left ? mw : sw, wr = from_left ? sw : mw;
+        const bool cleaf = dat >= 0 && up >= 0;
+        const int ds = (il ? 1 : 0) + (ir ? 1 : 0);
+        const uint32_t dw = (il ? 0u : wl) + (ir ? 0u : wr);
+        if (il)
+            step[q.cb + l] = make_int4(cur, cleaf ? -1 : ds + (ir ? (int)ir - 1 : 0), (int)(dw + (ir ? wr : 0u)), (int)il);
+        if (ir) step[q.cb + r] = make_int4(cur, cleaf ? -1 : ds, (int)dw, (int)(ir | (il ? kRightOfInner : 0u)));
+        if (cleaf) {
+            const int c = t.count[q.nb + cur];
+            mi = 0u;
+            mw = 3u * (uint32_t)(c > 1 ? c : 1) + 1u;
+        } else {
+            mi = 1u + il + ir;
+            mw = wl + wr;
+        }
+        if (up < 0) {
+            step[q.cb + cur] = make_int4(-1, 0, 0, (int)mi);
+            nodes_out[q.m] = (int64_t)mi;
+            woop_out[q.m] = (int64_t)mw;
+            return;
+        }
         ch = cur;
         cur = up;
         l = nl;
         r = nr;
         up = nup;
-        cleaf = ncleaf;
+        dat = ndat;
     }
 }
 
-// Pointer-jumping initialisation; thread gi owns inner node li of its mesh.
-// .x: pop-rank contribution; .y: depth in the low 16 bits, bit 30 set when a
-// leaf of the collapsed tree lies on the path (the node itself included).
-__global__ void __launch_bounds__(256) k_flat_jump_init(FlatRefs t, Segs segs, const uint32_t* __restrict__ icnt,
-                                                         int2* __restrict__ acc, int* __restrict__ jmp) {
+// Where a node stands: S, W, its depth (root 1), and whether it is part of
+// the layout (w = 0) or below a leaf of the collapsed tree (w = 1).
+// Pass 2: the nodes with large subtrees, over their whole path.
+__global__ void __launch_bounds__(256) k_flat_top(Segs segs, const int4* __restrict__ step, int4* __restrict__ place,
+                                                   const int32_t* __restrict__ data) {
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     if (gi >= segs.n) return;
     const SegPos q = seg_pos(segs, gi);
     if (q.li >= q.n - 1) return;
     const int x = (int)q.li;
-    const int gx = q.cb + x;
-    const int p = t.parent[q.nb + x];
-    if (p < 0) {
-        acc[gx] = make_int2(0, 0);
-        jmp[gx] = -1;
-        return;
+    if (data[q.nb + x] >= 0) return;  // a collapsed leaf has no step
+    int4 s = __ldg(step + q.cb + x);
+    if (step_inner(s) < kTopInner) return;
+    int4 at = make_int4(0, 0, 1, 0);
+    while (s.x >= 0) {
+        if (s.y < 0) {
+            at.w = 1;
+            break;
+        }
+        at.x += s.y;
+        at.y += s.z;
+        at.z += 1;
+        s = __ldg(step + q.cb + s.x);
     }
-    const bool is_left = t.left[q.nb + p] == x;
-    const int sib = is_left ? t.right[q.nb + p] : t.left[q.nb + p];
-    const int sib_inner = c_leaf(t, q.nb, sib) ? 0 : (int)icnt[q.cb + sib];
-    const int val = 1 + (is_left ? sib_inner : 0);
-    const int blocked = c_leaf(t, q.nb, x) ? (1 << 30) : 0;
-    acc[gx] = make_int2(val, 1 | blocked);
-    jmp[gx] = q.cb + p;
+    place[q.cb + x] = at;
 }
 
-// Round r of pointer jumping reads buffer r & 1 and writes buffer (r + 1) & 1;
-// pending[r * kPendingStride] records whether any jump is left after it (one
-// 32-byte sector per round, one store per block).  A round whose predecessor
-// left none does nothing, except the first such round of odd index, which
-// moves the finished sums into buffer 0: the host launches a fixed number of
-// rounds and never waits, and the result is always in buffer 0.  A node whose
-// jump ran out (-1) copies its sums into the other buffer once and marks both
-// jump words -2; later rounds skip it.  Readers of its jump word see -1 or -2,
-// both "no further ancestor".
-__global__ void __launch_bounds__(256) k_flat_jump(uint32_t m, int round, const int2* __restrict__ acc_in,
-                                                    int* jmp_in, int2* __restrict__ acc_out,
-                                                    int* __restrict__ jmp_out, uint32_t* __restrict__ pending) {
-    __shared__ int s_state;  // 0 jump, 1 idle, 2 idle and move buffer 1 to buffer 0
-    __shared__ int s_any;
-    if (threadIdx.x == 0) {
-        int st = 0;
-        if (round > 0 && pending[(round - 1) * kPendingStride] == 0u)
-            st = (round & 1) && (round == 1 || pending[(round - 2) * kPendingStride] != 0u) ? 2 : 1;
-        s_state = st;
-        s_any = 0;
-    }
-    __syncthreads();
-    const int st = s_state;
-    if (st == 1) return;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    bool any = false;
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < m; x += stride) {
-        if (st == 2) {
-            acc_out[x] = acc_in[x];
-            continue;
+// The place of inner node x (local), whose step is s.
+__device__ __forceinline__ int4 walk_up(const int4* __restrict__ step, const int4* __restrict__ place, int x, int4 s) {
+    int4 at = make_int4(0, 0, 0, 0);
+    while (true) {
+        if (step_inner(s) >= kTopInner) {
+            const int4 p = __ldg(place + x);
+            return make_int4(at.x + p.x, at.y + p.y, at.z + p.z, p.w);
         }
-        const int j = jmp_in[x];
-        if (j < 0) {
-            if (j == -1) {
-                acc_out[x] = acc_in[x];
-                jmp_out[x] = -2;
-                jmp_in[x] = -2;
-            }
-            continue;
+        at.z += 1;
+        if (s.x < 0) return at;
+        if (s.y < 0) {
+            at.w = 1;
+            return at;
         }
-        int2 a = acc_in[x];
-        const int2 b = acc_in[j];
-        a.x += b.x;
-        a.y = ((a.y & 0xffff) + (b.y & 0xffff)) | ((a.y | b.y) & (1 << 30));
-        const int nj = jmp_in[j];
-        acc_out[x] = a;
-        jmp_out[x] = nj < 0 ? -1 : nj;
-        any |= nj >= 0;
+        at.x += s.y;
+        at.y += s.z;
+        x = s.x;
+        s = __ldg(step + x);
     }
-    if (st != 0) return;
-    if (any) s_any = 1;
-    __syncthreads();
-    if (threadIdx.x == 0 && s_any) pending[round * kPendingStride] = 1u;
-}
-
-// Inner nodes of the layout are the reachable ones (no collapsed-tree leaf on
-// their path); scatter their inner-child counts and Woop sizes by pop rank.
-__global__ void __launch_bounds__(256) k_flat_scatter(Segs segs, const int2* __restrict__ acc,
-                                                       const uint32_t* __restrict__ ic,
-                                                       const uint32_t* __restrict__ tw,
-                                                       uint32_t* __restrict__ ic_by_rank,
-                                                       uint32_t* __restrict__ tw_by_rank,
-                                                       int* __restrict__ max_depth) {
-    const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
-    int depth = 0;
-    if (gi < segs.n) {
-        const SegPos q = seg_pos(segs, gi);
-        if (q.li < q.n - 1) {
-            const int gx = q.cb + (int)q.li;
-            const int2 a = acc[gx];
-            if (!(a.y & (1 << 30))) {
-                ic_by_rank[q.cb + a.x] = ic[gx];
-                tw_by_rank[q.cb + a.x] = tw[gx];
-                depth = (a.y & 0xffff) + 1;
-            }
-        }
-    }
-    // One atomic per warp on the shared maximum.
-    depth = __reduce_max_sync(0xffffffffu, depth);
-    if ((threadIdx.x & 31) == 0 && depth > 0) atomicMax(max_depth, depth);
 }
 
 __device__ __forceinline__ float det3(const float s[3][3]) {
@@ -275,25 +242,7 @@ __device__ void woopify(const float4* __restrict__ v, int tri, float4* __restric
     out[2] = make_float4(R[1][0], R[1][1], R[1][2], R[1][3]);
 }
 
-__global__ void __launch_bounds__(256) k_flat_slots(FlatRefs t, Segs segs, const int2* __restrict__ acc,
-                                                     const uint32_t* __restrict__ s_by_rank,
-                                                     int* __restrict__ slot_of) {
-    const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gi >= segs.n) return;
-    const SegPos q = seg_pos(segs, gi);
-    if (q.li >= q.n - 1) return;
-    const int x = (int)q.li;
-    const int2 a = acc[q.cb + x];
-    if (a.y & (1 << 30)) return;
-    if (t.parent[q.nb + x] < 0) slot_of[q.cb + x] = 0;
-    const int l = t.left[q.nb + x], r = t.right[q.nb + x];
-    const uint32_t base = 1u + s_by_rank[q.cb + a.x] - s_by_rank[q.cb];
-    const bool li = !c_leaf(t, q.nb, l), ri = !c_leaf(t, q.nb, r);
-    if (li) slot_of[q.cb + l] = (int)base;
-    if (ri) slot_of[q.cb + r] = (int)(base + (li ? 1u : 0u));
-}
-
-// One thread per reachable inner node: its 64-byte record in the mesh's node
+// Pass 3.  One thread per reachable inner node: its 64-byte record in the mesh's node
 // slice (first node 4 * cb in float4 units), the terminators of its leaf
 // children's Woop lists in the mesh's Woop slice (first entry 4 * s0).  The
 // Woop triangles of a warp's leaf children are then spread over the warp's
@@ -303,10 +252,10 @@ __global__ void __launch_bounds__(256) k_flat_slots(FlatRefs t, Segs segs, const
 constexpr int kWriteThreads = 128;
 
 __global__ void __launch_bounds__(kWriteThreads) k_flat_write(FlatRefs t, Segs segs, const float4* __restrict__ verts,
-                                                     const int2* __restrict__ acc,
-                                                     const uint32_t* __restrict__ w_by_rank,
-                                                     const int* __restrict__ slot_of, int4* __restrict__ nodes,
-                                                     float4* __restrict__ woop, int32_t* __restrict__ tri_index) {
+                                                     const int4* __restrict__ step, const int4* __restrict__ place,
+                                                     int4* __restrict__ nodes, float4* __restrict__ woop,
+                                                     int32_t* __restrict__ tri_index,
+                                                     unsigned long long* __restrict__ depth_out) {
     constexpr int W = kWriteThreads / 32;
     __shared__ uint32_t s_pre[W][32], s_n0[W][32], s_w[W][2][32], s_s0[W][32];
     __shared__ int32_t s_d[W][2][32];
@@ -316,22 +265,30 @@ __global__ void __launch_bounds__(kWriteThreads) k_flat_write(FlatRefs t, Segs s
     int32_t dk[2] = {0, 0};
     uint32_t s0 = 0;
     bool multi[2] = {false, false};
+    uint32_t depth = 0;
     if (gi < segs.n) {
         const SegPos q = seg_pos(segs, gi);
         s0 = q.s0;
         const int x = (int)q.li;
-        const int2 a = q.li < q.n - 1 ? acc[q.cb + x] : make_int2(0, 1 << 30);
-        if (!(a.y & (1 << 30))) {
+        int4 st = make_int4(-1, 0, 0, 0), at = make_int4(0, 0, 0, 1);
+        // The root is part of the layout whatever its data says.
+        if (q.li < q.n - 1 && (t.data[q.nb + x] < 0 || t.parent[q.nb + x] < 0)) {
+            st = __ldg(step + q.cb + x);
+            at = walk_up(step + q.cb, place + q.cb, x, st);
+        }
+        if (at.w == 0) {
+            depth = (uint32_t)at.z;
             float4* mw = woop + 4 * (size_t)q.s0;
             int32_t* mt = tri_index + 4 * (size_t)q.s0;
             const int ch[2] = {t.left[q.nb + x], t.right[q.nb + x]};
             int cref[2];
-            uint32_t w = w_by_rank[q.cb + a.x] - w_by_rank[q.cb];
+            uint32_t w = (uint32_t)at.y;
+            int slot = 1 + at.x;  // of the next inner child
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const int c = ch[k];
                 if (!c_leaf(t, q.nb, c)) {
-                    cref[k] = 4 * slot_of[q.cb + c];
+                    cref[k] = 4 * slot++;
                     continue;
                 }
                 cref[k] = ~(int)w;
@@ -348,13 +305,17 @@ __global__ void __launch_bounds__(kWriteThreads) k_flat_write(FlatRefs t, Segs s
             }
             const float4 lm = t.bmin[q.nb + ch[0]], lx = t.bmax[q.nb + ch[0]];
             const float4 rm = t.bmin[q.nb + ch[1]], rx = t.bmax[q.nb + ch[1]];
-            int4* dst = nodes + 4 * ((size_t)q.cb + (size_t)slot_of[q.cb + x]);
+            const int own = st.x < 0 ? 0 : 1 + at.x - st.y + (st.w < 0 ? 1 : 0);
+            int4* dst = nodes + 4 * ((size_t)q.cb + (size_t)own);
             dst[0] = make_int4(__float_as_int(lm.x), __float_as_int(lx.x), __float_as_int(lm.y), __float_as_int(lx.y));
             dst[1] = make_int4(__float_as_int(rm.x), __float_as_int(rx.x), __float_as_int(rm.y), __float_as_int(rx.y));
             dst[2] = make_int4(__float_as_int(lm.z), __float_as_int(lx.z), __float_as_int(rm.z), __float_as_int(rx.z));
             dst[3] = make_int4(cref[0], cref[1], 0, 0);
         }
     }
+    // One atomic per warp on the shared maximum.
+    depth = __reduce_max_sync(kFull, depth);
+    if (lane == 0 && depth > 0) atomicMax(depth_out, (unsigned long long)depth);
     // Items of this lane: items[0] triangles of the left leaf child, then
     // items[1] of the right.
     const uint32_t mine = items[0] + items[1];
@@ -398,22 +359,6 @@ __global__ void __launch_bounds__(kWriteThreads) k_flat_write(FlatRefs t, Segs s
     }
 }
 
-// Per-mesh sizes: inner nodes = 1 + inner children, Woop entries.
-__global__ void k_flat_sizes(Segs segs, const uint32_t* __restrict__ ic_scan, const uint32_t* __restrict__ tw_scan,
-                             const uint32_t* __restrict__ totals, const int* __restrict__ max_depth,
-                             int64_t* __restrict__ nodes_out, int64_t* __restrict__ woop_out,
-                             int64_t* __restrict__ depth_out) {
-    const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m == 0) *depth_out = *max_depth;
-    if (m >= segs.count) return;
-    const int cb = segs.inner_base(m);
-    const bool last = m + 1 == segs.count;
-    const uint32_t ic_end = last ? totals[0] : ic_scan[segs.inner_base(m + 1)];
-    const uint32_t tw_end = last ? totals[1] : tw_scan[segs.inner_base(m + 1)];
-    nodes_out[m] = 1 + (int64_t)(ic_end - ic_scan[cb]);
-    woop_out[m] = (int64_t)(tw_end - tw_scan[cb]);
-}
-
 }  // namespace
 
 // Compact2 layout of every mesh of segs into per-mesh slices of nodes (mesh m
@@ -427,62 +372,25 @@ int flatten_segs(atr_ctx* ctx, const Segs& segs, const CollapsedOut& c, const fl
     const uint32_t m = n - segs.count;  // inner nodes over all meshes
     cudaStream_t s = ctx->stream;
     void* scratch = nullptr;
-    const size_t bm = align256((size_t)m * 4), b2 = align256((size_t)m * 8);
-    ATR_TRY(ctx->alloc(&scratch, 9 * bm + 2 * b2 + kFlagBytes));
+    const size_t b4 = align256((size_t)m * 16);
+    ATR_TRY(ctx->alloc(&scratch, 2 * b4 + align256((size_t)m * 8)));
     char* p = static_cast<char*>(scratch);
-    uint32_t* icnt = reinterpret_cast<uint32_t*>(p); p += bm;
-    uint32_t* ic = reinterpret_cast<uint32_t*>(p); p += bm;
-    uint32_t* tw = reinterpret_cast<uint32_t*>(p); p += bm;
-    p += bm;  // spare word per inner node: the scratch keeps its size (and its place in the pool)
-    int* jmp0 = reinterpret_cast<int*>(p); p += bm;
-    int* jmp1 = reinterpret_cast<int*>(p); p += bm;
-    int* slot_of = reinterpret_cast<int*>(p); p += bm;
-    int2* acc0 = reinterpret_cast<int2*>(p); p += b2;
-    int2* acc1 = reinterpret_cast<int2*>(p); p += b2;
-    uint32_t* ic_r = reinterpret_cast<uint32_t*>(p); p += bm;
-    uint32_t* tw_r = reinterpret_cast<uint32_t*>(p); p += bm;
-    uint32_t* flags = reinterpret_cast<uint32_t*>(p);  // [1] max depth, [2..3] totals, then pending
-    FlatRefs t{c.parent, c.left, c.right, c.data, c.count, c.bmin, c.bmax, c.tri_indices};
-    const unsigned gb = (n + 255) / 256, gm = (m + 255) / 256;
-    // The exchange slots of pass 1 (8 B per inner node) live in acc0, which
-    // k_flat_jump_init overwrites for every inner node afterwards.
-    unsigned long long* const slots = reinterpret_cast<unsigned long long*>(acc0);
+    int4* step = reinterpret_cast<int4*>(p); p += b4;
+    int4* place = reinterpret_cast<int4*>(p); p += b4;
+    unsigned long long* slots = reinterpret_cast<unsigned long long*>(p);
+    const FlatRefs t{c.parent, c.left, c.right, c.data, c.count, c.bmin, c.bmax, c.tri_indices};
+    const unsigned gb = (n + 255) / 256;
+    int64_t* const depth_out = d_sizes + 2 * segs.count;
     // The count climb reads a zero slot as "no sibling yet": a failed clear must stop here.
-    cudaError_t me = cudaMemsetAsync(slots, 0, (size_t)m * 8, s);
-    if (me == cudaSuccess) me = cudaMemsetAsync(ic_r, 0, 2 * bm, s);
-    if (me == cudaSuccess) me = cudaMemsetAsync(flags, 0, kFlagBytes, s);
-    if (me != cudaSuccess) {
-        ctx->release(scratch);
-        return cuda_fail(me, "flatten scratch clear", __FILE__, __LINE__);
-    }
-    k_flat_counts<<<gb, 256, 0, s>>>(t, segs, icnt, ic, tw, slots);
-    k_flat_jump_init<<<gb, 256, 0, s>>>(t, segs, icnt, acc0, jmp0);
-    ctx->launches += 2;
-    // Depth <= m, and after round r every jump spans 2^(r+1) ancestors, so the
-    // last working round is below bits(m) and round bits(m) + 1 is idle.
-    if (m > 0) {
-        const int rounds = 34 - __builtin_clz(m);
-        int2* acc[2] = {acc0, acc1};
-        int* jmp[2] = {jmp0, jmp1};
-        const unsigned gj = std::min(gm, (unsigned)ctx->num_sms * 8u);
-        for (int r = 0; r < rounds; ++r)
-            k_flat_jump<<<gj, 256, 0, s>>>(m, r, acc[r & 1], jmp[r & 1], acc[(r + 1) & 1], jmp[(r + 1) & 1],
-                                           flags + kPendingWord);
-        ctx->launches += rounds;
-    }
-    const int2* ai = acc0;
-    k_flat_scatter<<<gb, 256, 0, s>>>(segs, ai, ic, tw, ic_r, tw_r, reinterpret_cast<int*>(flags + 1));
-    ctx->launches += 1;
-    int st = exclusive_scan_u32(ctx, ic_r, ic_r, m, flags + 2);
-    if (st == ATR_OK) st = exclusive_scan_u32(ctx, tw_r, tw_r, m, flags + 3);
+    int st = zero_words_async(ctx, reinterpret_cast<uint32_t*>(slots), (size_t)m * 2);
     if (st == ATR_OK) {
-        k_flat_slots<<<gb, 256, 0, s>>>(t, segs, ai, ic_r, slot_of);
-        k_flat_write<<<(n + kWriteThreads - 1) / kWriteThreads, kWriteThreads, 0, s>>>(t, segs, verts, ai, tw_r,
-                                                                                       slot_of, nodes, woop, tri_index);
-        k_flat_sizes<<<(segs.count + 255) / 256, 256, 0, s>>>(segs, ic_r, tw_r, flags + 2,
-                                                             reinterpret_cast<const int*>(flags + 1), d_sizes,
-                                                             d_sizes + segs.count, d_sizes + 2 * segs.count);
+        k_flat_counts<<<gb, 256, 0, s>>>(t, segs, step, slots, d_sizes, d_sizes + segs.count, depth_out);
+        k_flat_top<<<gb, 256, 0, s>>>(segs, step, place, c.data);
+        k_flat_write<<<(n + kWriteThreads - 1) / kWriteThreads, kWriteThreads, 0, s>>>(
+            t, segs, verts, step, place, nodes, woop, tri_index, reinterpret_cast<unsigned long long*>(depth_out));
         ctx->launches += 3;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) st = cuda_fail(e, "flatten kernels", __FILE__, __LINE__);
     }
     ctx->release(scratch);
     return st;
