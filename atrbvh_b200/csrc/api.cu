@@ -125,8 +125,9 @@ int atr_ctx_create(int device, void* stream, atr_ctx** out) {
         delete c;
         return atr::cuda_fail(e, "cudaMemPoolCreate", __FILE__, __LINE__);
     }
-    e = cudaMalloc(&c->d_error, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(c->d_error, 0, sizeof(uint32_t));
+    e = cudaMalloc(&c->d_error, 128);
+    if (e == cudaSuccess) e = cudaMemset(c->d_error, 0, 128);
+    if (e == cudaSuccess) c->d_trace = reinterpret_cast<unsigned long long*>(c->d_error + 16);
     if (e == cudaSuccess && atr::lbvh_prepare() != ATR_OK) e = cudaErrorInvalidValue;
     if (e == cudaSuccess && atr::atrbvh_prepare() != ATR_OK) e = cudaErrorInvalidValue;
     if (e != cudaSuccess) {

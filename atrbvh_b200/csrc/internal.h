@@ -86,6 +86,9 @@ struct atr_ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     uint32_t* d_error = nullptr;  // device error bits
+    // Traversal's ray counter and finished-warp counter, zero between launches
+    // (in d_error's allocation).
+    unsigned long long* d_trace = nullptr;
     uint64_t launches = 0;        // kernels enqueued by this context
     bool timing = false;
     // Launch tuning (atr_ctx_set_tuning): ATRBVH warps per block (2, 4, 8);

@@ -12,10 +12,18 @@
 // Woop dot products as fma chains, IEEE reciprocal; the CPU oracle uses the
 // same operations.
 //
-// Warps are persistent and refill terminated lanes from a global ray counter
-// (warp-aggregated atomic), breaking out to refill whenever fewer than 20
-// lanes of a warp are still traversing (the reference's dynamic fetch).
-
+// Warps are persistent: lanes whose ray is done wait until fewer than 20 lanes
+// of the warp have work (the reference's dynamic fetch), then take new rays
+// from a global counter.  Between two fetches the warp steps as one, every step
+// either a descent or a leaf test, chosen by vote: left to diverge, the lanes
+// of a warp met again only by chance and an instruction served 6.6 of 32 lanes
+// (1M sorted incoherent rays; 8.8 for pinhole rays); voting serves 11 and 13.
+// What a ray does, and in which order, does not depend on the schedule.  Bound
+// by issue (0.65 per cycle and scheduler) and by L1/L2 latency: 1M sorted
+// incoherent rays 1.07 -> 0.84 ms, 2.07M pinhole rays 0.57 -> 0.46 ms, a bounce of
+// each 0.66 -> 0.48 ms (4.2M triangles).  Measured and not kept: 12 or 16 blocks a
+// SM (spills), prefetching the pushed child, fetching at 12 or 28 lanes.
+//
 #include "common.cuh"
 #include "internal.h"
 
@@ -49,154 +57,240 @@ __device__ __forceinline__ float span_end(float a0, float a1, float b0, float b1
     return __int_as_float(imin(imin(__float_as_int(fmaxf(a0, a1)), __float_as_int(fmaxf(b0, b1))), t));
 }
 
-template <int kStack>
-__global__ void __launch_bounds__(128) k_trace(const float4* __restrict__ nodes_all,
+// A node's 64 bytes in two 32-byte loads: the lanes of a warp visit different
+// nodes, so each load instruction costs the L1 one lookup per lane (1M sorted
+// incoherent rays: 1.12 -> 1.07 ms against four 16-byte loads).
+__device__ __forceinline__ void ld32(const float4* p, float4& a, float4& b) {
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
+}
+
+constexpr int kTraceThreads = 128;
+constexpr int kSharedStack = 16;
+constexpr int kLeafWeight = 2;
+
+template <int kStack, bool kMapped>
+__global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restrict__ nodes_all,
                                                const float4* __restrict__ woop_all,
                                                const int* __restrict__ tri_all, RayMeshMap map,
                                                const float4* __restrict__ rays, int64_t nrays, int any_hit,
                                                int4* __restrict__ results, unsigned long long* __restrict__ counter,
-                                               uint32_t* __restrict__ err) {
-    int stack[kStack];
+                                               int lanes, uint32_t* __restrict__ err) {
+    // The stack's top entry is held in a register (top), so a pop does not
+    // wait for a load; of the sp entries below it the first kSharedStack are
+    // in shared memory (one bank per lane whatever the lanes' depths), the
+    // rest in local memory (16 entries take 5 % off incoherent rays; 4 or 8 less).
+    __shared__ int s_stack[kSharedStack][kTraceThreads];
+    int stack[kStack > kSharedStack ? kStack - kSharedStack : 1];
     const int lane = threadIdx.x & 31;
+    if (lane >= lanes) return;
+    const unsigned team = lanes == 32 ? kFull : (1u << lanes) - 1u;
+    const int fetch = (kDynamicFetch * lanes + 31) / 32;
+    int top = kSentinel;
     float ox = 0, oy = 0, oz = 0, tmin = 0, dx = 0, dy = 0, dz = 0, hitT = 0;
     float idx = 0, idy = 0, idz = 0, oodx = 0, oody = 0, oodz = 0;
     int nodeAddr = kSentinel, leafAddr = 0, hitIndex = -1, sp = 0;
     long long rayidx = 0;
-    bool overflow = false;
+    bool has = false, overflow = false;
+    bool more = true;  // the same in every lane: rays are left to fetch
     const float4* nodes = nodes_all;
     const float4* woop = woop_all;
     const int* tri_index = tri_all;
 
-    while (true) {
-        const bool terminated = nodeAddr == kSentinel;
-        const unsigned active = __activemask();
-        const unsigned mt = __ballot_sync(active, terminated);
-        if (terminated) {
-            const int leader = __ffs(mt) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(mt));
-            base = __shfl_sync(mt, base, leader);
-            rayidx = (long long)base + __popc(mt & lanemask_lt());
-            if (rayidx >= nrays) break;
-            if (map.groups) {
-                uint32_t lo = 0, hi = map.groups;
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if ((long long)__ldg(map.ray_off + mid) <= rayidx) lo = mid; else hi = mid;
+    auto pop = [&]() {
+        nodeAddr = top;
+        if (--sp >= 0) top = sp < kSharedStack ? s_stack[sp][threadIdx.x] : stack[max(sp - kSharedStack, 0)];
+    };
+    // Both children of the inner node nodeAddr against the ray: on to the
+    // nearer one, the farther one pushed; the first leaf met is set aside.
+    auto node_step = [&]() {
+        float4 n0, n1, nz, cn;
+        ld32(nodes + nodeAddr, n0, n1);
+        ld32(nodes + nodeAddr + 2, nz, cn);
+        int c0 = __float_as_int(cn.x), c1 = __float_as_int(cn.y);
+        const float c0lox = __fmaf_rn(n0.x, idx, -oodx), c0hix = __fmaf_rn(n0.y, idx, -oodx);
+        const float c0loy = __fmaf_rn(n0.z, idy, -oody), c0hiy = __fmaf_rn(n0.w, idy, -oody);
+        const float c0loz = __fmaf_rn(nz.x, idz, -oodz), c0hiz = __fmaf_rn(nz.y, idz, -oodz);
+        const float c1loz = __fmaf_rn(nz.z, idz, -oodz), c1hiz = __fmaf_rn(nz.w, idz, -oodz);
+        const float c0min = span_begin(c0lox, c0hix, c0loy, c0hiy, c0loz, c0hiz, tmin);
+        const float c0max = span_end(c0lox, c0hix, c0loy, c0hiy, c0loz, c0hiz, hitT);
+        const float c1lox = __fmaf_rn(n1.x, idx, -oodx), c1hix = __fmaf_rn(n1.y, idx, -oodx);
+        const float c1loy = __fmaf_rn(n1.z, idy, -oody), c1hiy = __fmaf_rn(n1.w, idy, -oody);
+        const float c1min = span_begin(c1lox, c1hix, c1loy, c1hiy, c1loz, c1hiz, tmin);
+        const float c1max = span_end(c1lox, c1hix, c1loy, c1hiy, c1loz, c1hiz, hitT);
+        const bool swp = c1min < c0min;
+        const bool t0 = c0max >= c0min, t1 = c1max >= c1min;
+        if (!t0 && !t1) {
+            pop();
+        } else {
+            nodeAddr = t0 ? c0 : c1;
+            if (t0 && t1) {
+                if (swp) { const int tmp = nodeAddr; nodeAddr = c1; c1 = tmp; }
+                if (sp + 1 >= kStack) {  // deeper than the stack: give the ray up
+                    overflow = true;
+                    nodeAddr = kSentinel;
+                    leafAddr = 0;
+                    return;
                 }
-                const uint32_t mesh = __ldg(map.group_mesh + lo);
-                const uint32_t s0 = __ldg(map.tri_off + mesh);
-                nodes = nodes_all + 4 * ((size_t)s0 - mesh);
-                woop = woop_all + 4 * (size_t)s0;
-                tri_index = tri_all + 4 * (size_t)s0;
+                if (sp < kSharedStack) s_stack[sp][threadIdx.x] = top;
+                else stack[max(sp - kSharedStack, 0)] = top;
+                ++sp;
+                top = c1;
             }
-            const float4 o = __ldg(rays + 2 * rayidx), d = __ldg(rays + 2 * rayidx + 1);
-            ox = o.x; oy = o.y; oz = o.z; tmin = o.w;
-            dx = d.x; dy = d.y; dz = d.z; hitT = d.w;
-            const float ooeps = 8.271806125530277e-25f;  // 2^-80
-            idx = __fdiv_rn(1.0f, fabsf(dx) > ooeps ? dx : copysignf(ooeps, dx));
-            idy = __fdiv_rn(1.0f, fabsf(dy) > ooeps ? dy : copysignf(ooeps, dy));
-            idz = __fdiv_rn(1.0f, fabsf(dz) > ooeps ? dz : copysignf(ooeps, dz));
-            oodx = __fmul_rn(ox, idx);
-            oody = __fmul_rn(oy, idy);
-            oodz = __fmul_rn(oz, idz);
-            stack[0] = kSentinel;
-            sp = 0;
-            leafAddr = 0;
-            nodeAddr = 0;
-            hitIndex = -1;
-            overflow = false;
         }
+        if (nodeAddr < 0 && leafAddr >= 0) {
+            leafAddr = nodeAddr;
+            pop();
+        }
+    };
+    // The next triangle of the leaf set aside, and whether it was the last: a
+    // triangle is always followed by another or by the terminator, so all of
+    // these loads lie in the list and can be in flight together.
+    auto leaf_step = [&]() {
+        const int tri = ~leafAddr;
+        const float4 v00 = __ldg(woop + tri);
+        const int next = __ldg(reinterpret_cast<const int*>(woop + tri + 3));
+        bool last = true;
+        if (__float_as_int(v00.x) != (int)0x80000000u) {
+            last = next == (int)0x80000000u;
+            const float Oz = __fmaf_rn(-oz, v00.z, __fmaf_rn(-oy, v00.y, __fmaf_rn(-ox, v00.x, v00.w)));
+            const float invDz = __frcp_rn(__fmaf_rn(dz, v00.z, __fmaf_rn(dy, v00.y, __fmul_rn(dx, v00.x))));
+            const float t = __fmul_rn(Oz, invDz);
+            if (t > tmin && t < hitT) {
+                const float4 v11 = __ldg(woop + tri + 1), v22 = __ldg(woop + tri + 2);
+                const float Ox = __fmaf_rn(oz, v11.z, __fmaf_rn(oy, v11.y, __fmaf_rn(ox, v11.x, v11.w)));
+                const float Dx = __fmaf_rn(dz, v11.z, __fmaf_rn(dy, v11.y, __fmul_rn(dx, v11.x)));
+                const float u = __fmaf_rn(t, Dx, Ox);
+                const float Oy = __fmaf_rn(oz, v22.z, __fmaf_rn(oy, v22.y, __fmaf_rn(ox, v22.x, v22.w)));
+                const float Dy = __fmaf_rn(dz, v22.z, __fmaf_rn(dy, v22.y, __fmul_rn(dx, v22.x)));
+                const float v = __fmaf_rn(t, Dy, Oy);
+                if (u >= 0.0f && v >= 0.0f && __fadd_rn(u, v) <= 1.0f) {
+                    hitT = t;
+                    hitIndex = tri;
+                    if (any_hit) {
+                        nodeAddr = kSentinel;
+                        last = true;
+                    }
+                }
+            }
+        }
+        if (!last) {
+            leafAddr -= 3;  // ~(tri + 3)
+        } else {
+            leafAddr = nodeAddr;
+            if (nodeAddr < 0) pop();
+        }
+    };
 
-        while (nodeAddr != kSentinel) {
-            while ((unsigned)nodeAddr < (unsigned)kSentinel) {
-                const float4 n0 = __ldg(nodes + nodeAddr), n1 = __ldg(nodes + nodeAddr + 1);
-                const float4 nz = __ldg(nodes + nodeAddr + 2), cn = __ldg(nodes + nodeAddr + 3);
-                int c0 = __float_as_int(cn.x), c1 = __float_as_int(cn.y);
-                const float c0lox = __fmaf_rn(n0.x, idx, -oodx), c0hix = __fmaf_rn(n0.y, idx, -oodx);
-                const float c0loy = __fmaf_rn(n0.z, idy, -oody), c0hiy = __fmaf_rn(n0.w, idy, -oody);
-                const float c0loz = __fmaf_rn(nz.x, idz, -oodz), c0hiz = __fmaf_rn(nz.y, idz, -oodz);
-                const float c1loz = __fmaf_rn(nz.z, idz, -oodz), c1hiz = __fmaf_rn(nz.w, idz, -oodz);
-                const float c0min = span_begin(c0lox, c0hix, c0loy, c0hiy, c0loz, c0hiz, tmin);
-                const float c0max = span_end(c0lox, c0hix, c0loy, c0hiy, c0loz, c0hiz, hitT);
-                const float c1lox = __fmaf_rn(n1.x, idx, -oodx), c1hix = __fmaf_rn(n1.y, idx, -oodx);
-                const float c1loy = __fmaf_rn(n1.z, idy, -oody), c1hiy = __fmaf_rn(n1.w, idy, -oody);
-                const float c1min = span_begin(c1lox, c1hix, c1loy, c1hiy, c1loz, c1hiz, tmin);
-                const float c1max = span_end(c1lox, c1hix, c1loy, c1hiy, c1loz, c1hiz, hitT);
-                const bool swp = c1min < c0min;
-                const bool t0 = c0max >= c0min, t1 = c1max >= c1min;
-                if (!t0 && !t1) {
-                    nodeAddr = stack[sp--];
-                } else {
-                    nodeAddr = t0 ? c0 : c1;
-                    if (t0 && t1) {
-                        if (swp) { const int tmp = nodeAddr; nodeAddr = c1; c1 = tmp; }
-                        if (sp + 1 >= kStack) {  // deeper than the stack: give the ray up
-                            overflow = true;
-                            nodeAddr = kSentinel;
-                            leafAddr = 0;
-                            break;
+    while (true) {
+        if (more) {
+            // Lanes without a ray take the next ones.
+            const unsigned idle = __ballot_sync(team, !has);
+            const int leader = __ffs(idle) - 1;
+            unsigned long long base = 0;
+            if (lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(idle));
+            base = __shfl_sync(team, base, leader);
+            more = (long long)base + __popc(idle) < nrays;
+            if (!has) {
+                rayidx = (long long)base + __popc(idle & lanemask_lt());
+                has = rayidx < nrays;
+                if (has) {
+                    if constexpr (kMapped) {
+                        uint32_t lo = 0, hi = map.groups;
+                        while (hi - lo > 1) {
+                            const uint32_t mid = (lo + hi) >> 1;
+                            if ((long long)__ldg(map.ray_off + mid) <= rayidx) lo = mid; else hi = mid;
                         }
-                        stack[++sp] = c1;
+                        const uint32_t mesh = __ldg(map.group_mesh + lo);
+                        const uint32_t s0 = __ldg(map.tri_off + mesh);
+                        nodes = nodes_all + 4 * ((size_t)s0 - mesh);
+                        woop = woop_all + 4 * (size_t)s0;
+                        tri_index = tri_all + 4 * (size_t)s0;
                     }
+                    const float4 o = __ldg(rays + 2 * rayidx), d = __ldg(rays + 2 * rayidx + 1);
+                    ox = o.x; oy = o.y; oz = o.z; tmin = o.w;
+                    dx = d.x; dy = d.y; dz = d.z; hitT = d.w;
+                    const float ooeps = 8.271806125530277e-25f;  // 2^-80
+                    idx = __frcp_rn(fabsf(dx) > ooeps ? dx : copysignf(ooeps, dx));
+                    idy = __frcp_rn(fabsf(dy) > ooeps ? dy : copysignf(ooeps, dy));
+                    idz = __frcp_rn(fabsf(dz) > ooeps ? dz : copysignf(ooeps, dz));
+                    oodx = __fmul_rn(ox, idx);
+                    oody = __fmul_rn(oy, idy);
+                    oodz = __fmul_rn(oz, idz);
+                    top = kSentinel;
+                    sp = 0;
+                    leafAddr = 0;
+                    nodeAddr = 0;
+                    hitIndex = -1;
+                    overflow = false;
                 }
-                if (nodeAddr < 0 && leafAddr >= 0) {
-                    leafAddr = nodeAddr;
-                    nodeAddr = stack[sp--];
-                }
-                if (leafAddr < 0) break;
             }
-            while (leafAddr < 0) {
-                for (int triAddr = ~leafAddr;; triAddr += 3) {
-                    const float4 v00 = __ldg(woop + triAddr);
-                    if (__float_as_int(v00.x) == (int)0x80000000u) break;
-                    const float4 v11 = __ldg(woop + triAddr + 1), v22 = __ldg(woop + triAddr + 2);
-                    const float Oz = __fmaf_rn(-oz, v00.z, __fmaf_rn(-oy, v00.y, __fmaf_rn(-ox, v00.x, v00.w)));
-                    const float invDz = __fdiv_rn(1.0f, __fmaf_rn(dz, v00.z, __fmaf_rn(dy, v00.y, __fmul_rn(dx, v00.x))));
-                    const float t = __fmul_rn(Oz, invDz);
-                    if (t > tmin && t < hitT) {
-                        const float Ox = __fmaf_rn(oz, v11.z, __fmaf_rn(oy, v11.y, __fmaf_rn(ox, v11.x, v11.w)));
-                        const float Dx = __fmaf_rn(dz, v11.z, __fmaf_rn(dy, v11.y, __fmul_rn(dx, v11.x)));
-                        const float u = __fmaf_rn(t, Dx, Ox);
-                        if (u >= 0.0f) {
-                            const float Oy = __fmaf_rn(oz, v22.z, __fmaf_rn(oy, v22.y, __fmaf_rn(ox, v22.x, v22.w)));
-                            const float Dy = __fmaf_rn(dz, v22.z, __fmaf_rn(dy, v22.y, __fmul_rn(dx, v22.x)));
-                            const float v = __fmaf_rn(t, Dy, Oy);
-                            if (v >= 0.0f && __fadd_rn(u, v) <= 1.0f) {
-                                hitT = t;
-                                hitIndex = triAddr;
-                                if (any_hit) { nodeAddr = kSentinel; break; }
-                            }
-                        }
-                    }
-                }
-                leafAddr = nodeAddr;
-                if (nodeAddr < 0) nodeAddr = stack[sp--];
-            }
-            if (__popc(__activemask()) < kDynamicFetch) break;
         }
-        if (nodeAddr == kSentinel) {
+        // Steps until fewer than `fetch` lanes have work (or none, once there
+        // are no rays to fetch).  A lane either descends or tests its leaf; each
+        // warp step is one of the two: descent unless the lanes at leaves are
+        // more than half as many (a leaf step is short and frees its lane).
+        const int enough = more ? fetch : 1;
+        while (true) {
+            const bool leaf = has && leafAddr < 0;
+            const bool inner = has && !leaf && nodeAddr != kSentinel;
+            const unsigned bi = __ballot_sync(team, inner), bl = __ballot_sync(team, leaf);
+            if (__popc(bi | bl) < enough) break;
+            if (__popc(bi) >= kLeafWeight * __popc(bl)) {
+                // Two steps a vote: most lanes that descend do so again.
+                if (inner) {
+                    node_step();
+                    if ((unsigned)nodeAddr < (unsigned)kSentinel && leafAddr >= 0) node_step();
+                }
+            } else {
+                if (leaf) leaf_step();
+            }
+        }
+        if (has && nodeAddr == kSentinel && leafAddr >= 0) {
             if (overflow) set_error_bits(err, kErrTraceStack);
             const int id = hitIndex == -1 ? -1 : __ldg(tri_index + hitIndex);
             results[rayidx] = make_int4(id, __float_as_int(hitT), 0, 0);
+            has = false;
         }
+        if (!more && !__any_sync(team, has)) break;
     }
+    // The last warp leaves both counters at zero for the next launch.
+    if (lane == 0 && atomicAdd(counter + 1, 1ull) == (unsigned long long)gridDim.x * (kTraceThreads / 32) - 1ull) {
+        counter[0] = 0ull;
+        counter[1] = 0ull;
+    }
+}
+
+template <int kStack, bool kMapped>
+void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
+                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter) {
+    static int blocks_per_sm = 0;
+    if (!blocks_per_sm) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_trace<kStack, kMapped>, kTraceThreads, 0);
+        if (blocks_per_sm < 1) blocks_per_sm = 1;
+    }
+    // Rays per warp: the paths of a warp's rays add up as far as they differ, so
+    // few rays are spread over as many warps as run at once (1,000 rays through
+    // 20,011 triangles: 57 us at one ray a warp, 93 at 32; 50,000 rays: 103 us at
+    // 32 or 16, 117 at 8).
+    constexpr int W = kTraceThreads / 32;
+    const int64_t warps = (int64_t)ctx->num_sms * blocks_per_sm * W;
+    int lanes = 32;
+    while (lanes > 1 && n <= warps * (lanes / 2)) lanes /= 2;
+    const int64_t need = (n + W * lanes - 1) / (W * lanes);
+    int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
+    if (need < grid) grid = need;
+    k_trace<kStack, kMapped><<<(unsigned)grid, kTraceThreads, 0, ctx->stream>>>(
+        reinterpret_cast<const float4*>(nodes), woop, tri, map, rays, n, any_hit, res, counter, lanes, ctx->d_error);
+    ctx->launches += 1;
 }
 
 template <int kStack>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
                   const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter) {
-    static int blocks_per_sm = 0;
-    if (!blocks_per_sm) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_trace<kStack>, 128, 0);
-        if (blocks_per_sm < 1) blocks_per_sm = 1;
-    }
-    const int64_t need = (n + 127) / 128;
-    int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
-    if (need < grid) grid = need;
-    k_trace<kStack><<<(unsigned)grid, 128, 0, ctx->stream>>>(reinterpret_cast<const float4*>(nodes), woop, tri, map,
-                                                             rays, n, any_hit, res, counter, ctx->d_error);
-    ctx->launches += 1;
+    if (map.groups) launch_trace<kStack, true>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter);
+    else launch_trace<kStack, false>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter);
 }
 
 // Cosine-weighted diffuse bounce per primary hit (the workload of
@@ -250,16 +344,25 @@ __global__ void __launch_bounds__(256) k_bounce(const float4* __restrict__ verts
 int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
               int max_depth, const float4* rays, int64_t n, int any_hit, int4* res) {
     if (n == 0) return ATR_OK;
-    unsigned long long* counter = nullptr;
-    ATR_TRY(ctx->alloc(reinterpret_cast<void**>(&counter), 8));
-    cudaMemsetAsync(counter, 0, 8, ctx->stream);
+    // The ray counter: the context's own, which every launch on its stream
+    // leaves at zero.  A captured trace gets one of its own, since its graph may
+    // run on any stream beside others.
+    unsigned long long* counter = ctx->d_trace;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    ATR_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+    unsigned long long* own = nullptr;
+    if (cap != cudaStreamCaptureStatusNone) {
+        ATR_TRY(ctx->alloc(reinterpret_cast<void**>(&own), 16));
+        cudaMemsetAsync(own, 0, 16, ctx->stream);
+        counter = own;
+    }
     int st = ATR_OK;
     ctx->phase_begin("trace");
     if (max_depth + 1 < 64) launch_trace<64>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter);
     else if (max_depth + 1 < 256) launch_trace<256>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter);
     else st = ATR_ERR_UNSUPPORTED;
     ctx->phase_end();
-    ctx->release(counter);
+    ctx->release(own);
     if (st == ATR_ERR_UNSUPPORTED) {
         set_error("trace: layout depth %d exceeds the traversal stack", max_depth);
         return st;
