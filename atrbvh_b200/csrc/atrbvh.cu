@@ -40,6 +40,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "levels.cuh"
 #include "treelet.cuh"
 
 namespace atr {
@@ -57,29 +58,6 @@ struct GroupLayout {
     static constexpr int kFloats = kDistPad + 12 * kLeaves;
 };
 
-// The optimiser's per-node record, node-indexed in the batch layout (one
-// 16-byte load gives a treelet leaf everything but its box):
-//   x  subtree triangle count;
-//   y  nodesSah of even iterations, z  nodesSah of odd iterations -- this
-//      iteration's in component 1 + par (par = iteration & 1), the next
-//      iteration's in the other;
-//   w  big-node level: this iteration's until the node is finished, the next
-//      iteration's after (only the level lists, built before any node is
-//      finished, read this iteration's).
-// The reference recomputes nodesSah bottom-up every iteration as
-// (ci*A + left) + right, while a rewritten node stores the merge cost
-// (left + right) + ci*A; the two can differ in the last bit, so the next
-// iteration's values are kept in the recomputation's order.
-__device__ __forceinline__ int rec_ns_cur(int par) { return 1 + par; }
-__device__ __forceinline__ int rec_ns_next(int par) { return 2 - par; }
-__device__ __forceinline__ float* rec_f(int4* r, int x, int c) { return reinterpret_cast<float*>(r + x) + c; }
-__device__ __forceinline__ int* rec_i(int4* r, int x, int c) { return reinterpret_cast<int*>(r + x) + c; }
-// A record from its fields, the nodesSah values placed by parity.
-__device__ __forceinline__ int4 make_rec(int cnt, float ns_cur, float ns_next, int lvl, int par) {
-    return par ? make_int4(cnt, __float_as_int(ns_next), __float_as_int(ns_cur), lvl)
-               : make_int4(cnt, __float_as_int(ns_cur), __float_as_int(ns_next), lvl);
-}
-
 // What the treelet code keeps up to date, per mesh (rec starts at the mesh's
 // first node): the records of the nodes it finishes or rewrites, the next
 // iteration's gamma for their levels.
@@ -96,55 +74,6 @@ constexpr int warp_floats() {
                ? GroupLayout<G>::kFloats * GroupLayout<G>::kGroups
                : GroupLayout<32>::kFloats;
 }
-
-// formTreelet's argmax tree (Treelet.cuh:23-39) over m lanes -- lane i takes
-// lane i + floor(c/2) when that value is strictly larger, c halving upward --
-// returns the largest value and, among equal largest values, the lane that
-// comes first in a fixed order that depends only on m.  tree_winner replays
-// the tree on a tie pattern; argmax_priority ranks the lanes by removing
-// winners one at a time.  The full-warp path then needs two warp reductions:
-// the maximum value, then the lowest rank among the lanes holding it.
-struct ArgmaxPriority {
-    uint8_t rank[kMaxTreelet + 1][32];
-};
-
-constexpr int tree_winner(int m, uint32_t tied) {
-    int val[32] = {};
-    int idx[32] = {};
-    for (int i = 0; i < 32; ++i) {
-        val[i] = (i < m && ((tied >> i) & 1u)) ? 1 : 0;
-        idx[i] = i;
-    }
-    int c = m, sh = m / 2;
-    while (c > 1) {
-        for (int i = 0; i < c - sh; ++i)  // ascending: lane i + sh is read before it is updated
-            if (val[i + sh] > val[i]) {
-                val[i] = val[i + sh];
-                idx[i] = idx[i + sh];
-            }
-        c = (c + 1) / 2;
-        sh = c / 2;
-    }
-    return idx[0];
-}
-
-constexpr ArgmaxPriority argmax_priority() {
-    ArgmaxPriority t{};
-    for (int m = 0; m <= kMaxTreelet; ++m)
-        for (int i = 0; i < 32; ++i) t.rank[m][i] = 255;
-    for (int m = 1; m <= kMaxTreelet; ++m) {
-        uint32_t rem = m == 32 ? 0xffffffffu : ((1u << m) - 1u);
-        int k = 0;
-        while (rem) {
-            const int w = tree_winner(m, rem);
-            t.rank[m][w] = (uint8_t)k++;
-            rem &= ~(1u << w);
-        }
-    }
-    return t;
-}
-
-__device__ const ArgmaxPriority g_argmax_priority = argmax_priority();
 
 __device__ __forceinline__ float union_area3(float ax0, float ay0, float az0, float ax1, float ay1, float az1,
                                              float bx0, float by0, float bz0, float bx1, float by1, float bz1) {
@@ -818,134 +747,6 @@ cudaError_t launch_atrbvh_g(int warps, uint32_t blocks, cudaStream_t s, const Tr
     return cudaGetLastError();
 }
 
-// ---- level passes ---------------------------------------------------------------
-// A node whose subtree holds at least gamma triangles ("big") is a treelet
-// root; its results depend only on its subtree, so any order that finishes a
-// node's big descendants first gives the reference's result.  The level of a
-// big node is 1 + the largest level of its big children (0 for the others).
-// Phase A finishes every node that is not big (subtree count, nodesSah, child
-// record) and levels the big ones: k_levels climbs once from every leaf;
-// k_levels_pp and k_levels_pp_hist take counts, nodesSah (and levels) from
-// the LBVH build.  Phase B files big nodes of levels 1..L into per-level
-// lists (in the same pass as the level counts: k_levels_pp_hist for the first
-// iteration, k_level_hist for the others); phase C restructures each level's
-// treelets in one launch, several per warp in lane groups; the dataflow kernel
-// then climbs from the frontier below the levels above L.
-
-constexpr int kMaxLevels = 64;  // largest L (ATR_TUNE_ATR_LEVELS)
-constexpr int kListPer = 8;                  // nodes per thread of the level-list kernels
-constexpr int kListBlock = 256 * kListPer;  // nodes per block of those kernels
-
-struct LevelRefs {
-    int4* rec;             // per node (node-indexed): count, nodesSah x 2, level (see NextRefs)
-    int par;               // iteration & 1
-    float ct;              // the leaf cost constant (triangle leaves' records)
-    uint32_t* counters;
-    int4* kids;
-    uint32_t* cursor;      // [L + 2]: entries filed per level (the level's count)
-    uint2* order;          // (mesh, local node) of big nodes: level l's list at (l - 1) * cap
-    uint32_t cap;          // entries per level list (at most n / gamma nodes share a level)
-    uint2* frontier;       // climb starts of the dataflow pass
-    uint32_t* n_frontier;
-    uint32_t* err;
-};
-
-constexpr int kLvBlock = 512;  // threads (leaves) per block of the phase-A climb
-
-// Phase A of the first iteration: one climb from every leaf (sorted order)
-// that finishes the nodes that are not treelet roots and levels the roots.
-// With the radix tree's leaf ranges (a tree straight from the LBVH build), a
-// node whose range lies inside the block's leaves is reached only by threads
-// of the block, so its arrival counter and the first child's summary live in
-// shared memory under block-scope ordering; only nodes whose range crosses a
-// block boundary use a device-scope acquire-release atomic in global memory.
-// Without ranges every node takes the global path.
-__global__ void __launch_bounds__(kLvBlock) k_levels(TreeRefs g, Segs segs, LevelRefs lv, int tsize_all,
-                                                     const uint8_t* __restrict__ seg_tsize,
-                                                     const uint8_t* __restrict__ seg_iters, int iteration, float ci,
-                                                     float ct, int L, const int2* __restrict__ ranges) {
-    __shared__ uint32_t s_ctr[kLvBlock];
-    __shared__ int4 s_rec[kLvBlock][2];  // per local node and side: (count, level, nodesSah, area)
-    for (int k = threadIdx.x; k < kLvBlock; k += blockDim.x) s_ctr[k] = 0;
-    __syncthreads();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= segs.n) return;
-    const uint32_t m = segs.seg_of_tri(i);
-    if (seg_iters && iteration >= (int)seg_iters[m]) return;
-    const uint32_t s0 = segs.tri_begin(m);
-    const uint32_t n = segs.tri_end(m) - s0;
-    const int base = segs.node_base(m), cb = segs.inner_base(m);
-    const int gamma = (seg_tsize ? (int)seg_tsize[m] : tsize_all) << iteration;
-    const int64_t blo = (int64_t)blockIdx.x * blockDim.x, bhi = blo + blockDim.x - 1;
-    const int li = (int)(i - s0);
-    const int leaf = base + li + (int)n - 1;
-    // Summary of the subtree this thread has just finished (the leaf first).
-    const float la = g.area[leaf];
-    int my_cnt = 1, my_lvl = 0, my_first = li, child = li + (int)n - 1;
-    float my_nsah = __fmul_rn(ct, la), my_area = la;
-    lv.rec[leaf] = make_int4(1, __float_as_int(my_nsah), __float_as_int(my_nsah), 0);
-    const int cur_c = rec_ns_cur(lv.par);
-    int cur = g.parent[leaf];
-    while (cur >= 0) {
-        const int x = base + cur;
-        int sib_cnt, sib_lvl;
-        float sib_nsah, sib_area;
-        bool local = false;
-        if (ranges) {
-            const int2 rg = ranges[cb + cur];
-            local = (int64_t)s0 + rg.x >= blo && (int64_t)s0 + rg.y <= bhi;
-            if (local) {
-                // Internal node cur covers [rg.x, rg.y] and is numbered by one
-                // of its ends, so its slot lies inside the block.
-                const int slot = (int)((int64_t)s0 + cur - blo);
-                const int side = my_first == rg.x ? 0 : 1;
-                s_rec[slot][side] = make_int4(my_cnt, my_lvl, __float_as_int(my_nsah), __float_as_int(my_area));
-                __threadfence_block();
-                if (atomicAdd(&s_ctr[slot], 1u) == 0u) return;
-                __threadfence_block();
-                const int4 r = s_rec[slot][side ^ 1];
-                sib_cnt = r.x;
-                sib_lvl = r.y;
-                sib_nsah = __int_as_float(r.z);
-                sib_area = __int_as_float(r.w);
-                my_first = rg.x;
-            }
-        }
-        const int lc = ld_cg(g.left + x), rc = ld_cg(g.right + x);
-        const int sib = lc == child ? rc : lc;
-        if (!local) {
-            if (atomic_add_acq_rel_gpu(&lv.counters[cb + cur], 1u) == 0u) return;
-            const int4 sr = __ldcg(lv.rec + base + sib);
-            sib_cnt = sr.x;
-            sib_lvl = is_internal(sib, n) ? sr.w : 0;
-            sib_nsah = __int_as_float(cur_c == 1 ? sr.y : sr.z);
-            sib_area = ld_cg(g.area + base + sib);
-            if (ranges) my_first = min(my_first, ranges[cb + cur].x);
-        }
-        const bool mine_left = lc == child;
-        const int cnt = my_cnt + sib_cnt;
-        const float a = ld_cg(g.area + x);
-        lv.kids[cb + cur] = make_int4(lc, rc, __float_as_int(mine_left ? my_area : sib_area),
-                                      __float_as_int(mine_left ? sib_area : my_area));
-        int lvl = 0;
-        float ns = 0.0f;
-        if (cnt < gamma) {
-            ns = __fadd_rn(__fadd_rn(__fmul_rn(ci, a), mine_left ? my_nsah : sib_nsah), mine_left ? sib_nsah : my_nsah);
-            lv.rec[x] = make_int4(cnt, __float_as_int(ns), __float_as_int(ns), 0);
-        } else {
-            lvl = 1 + max(my_lvl, sib_lvl);
-            *rec_i(lv.rec, x, 0) = cnt;
-            *rec_i(lv.rec, x, 3) = lvl;
-        }
-        my_cnt = cnt;
-        my_lvl = lvl;
-        my_nsah = ns;  // only read while the climb stays below the treelet roots (cnt < gamma)
-        my_area = a;
-        child = cur;
-        cur = g.parent[x];
-    }
-}
-
 // Phase A of the first iteration on a tree straight from the LBVH build,
 // which left every node's nodesSah for the default constants: subtree counts
 // come from the radix tree's leaf ranges, so a streaming pass (one thread per
@@ -1005,41 +806,6 @@ __global__ void __launch_bounds__(256) k_levels_pp(TreeRefs g, Segs segs, LevelR
 // one streaming pass writes the counts, child records and next-iteration
 // values of the nodes that are not big, counts the levels 1..L and lists
 // the frontier below the levels above L (k_level_hist's work as well).
-// Files a block's nodes of levels 1..L into the level lists: thread-held
-// levels me[q] (0: none) and entries ent[q].  Ranks within the block come from
-// one shared atomic per level present in a warp (__match_any_sync), then one
-// global reservation per level per block on lv.cursor (which ends as the
-// level's count).  Nodes of one level have disjoint subtrees of at least gamma
-// triangles each, so a list holds at most lv.cap of them; a reservation past
-// that sets kErrLevelList and writes nothing.  Every thread of the block calls
-// it; s_cnt holds L + 2 zeroed counters.
-__device__ __forceinline__ void file_levels(const LevelRefs& lv, int L, const int (&me)[kListPer],
-                                            const uint2 (&ent)[kListPer], uint32_t* s_cnt, uint32_t* s_base) {
-    const int lane = threadIdx.x & 31;
-    uint32_t key[kListPer];
-#pragma unroll
-    for (int q = 0; q < kListPer; ++q) {
-        const uint32_t peers = __match_any_sync(kFull, me[q]);
-        const int leader = __ffs(peers) - 1;
-        uint32_t b = 0;
-        if (lane == leader && me[q] > 0) b = atomicAdd(&s_cnt[me[q]], (uint32_t)__popc(peers));
-        b = __shfl_sync(kFull, b, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-        key[q] = me[q] > 0 ? ((uint32_t)me[q] << 16) | b : 0u;  // rank < kListBlock
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < L + 2; k += blockDim.x)
-        s_base[k] = s_cnt[k] ? atomicAdd(&lv.cursor[k], s_cnt[k]) : 0u;
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < kListPer; ++q)
-        if (key[q]) {
-            const uint32_t l = key[q] >> 16;
-            const uint32_t at = s_base[l] + (key[q] & 0xffffu);
-            if (at < lv.cap) lv.order[(size_t)(l - 1) * lv.cap + at] = ent[q];
-            else set_error_bits(lv.err, kErrLevelList);
-        }
-}
-
 __global__ void __launch_bounds__(256) k_levels_pp_hist(TreeRefs g, Segs segs, LevelRefs lv,
                                                         const int2* __restrict__ ranges, int tsize_all,
                                                         const uint8_t* __restrict__ seg_tsize,
@@ -1054,6 +820,7 @@ __global__ void __launch_bounds__(256) k_levels_pp_hist(TreeRefs g, Segs segs, L
     for (int q = 0; q < kListPer; ++q) {
         const uint32_t i = blockIdx.x * kListBlock + q * 256 + threadIdx.x;
         int push = 0;
+        bool above = false;
         uint2 ent[2];
         lvl[q] = 0;
         lent[q] = make_uint2(0u, 0u);
@@ -1076,10 +843,11 @@ __global__ void __launch_bounds__(256) k_levels_pp_hist(TreeRefs g, Segs segs, L
                         make_int4(lc, rc, __float_as_int(g.area[base + lc]), __float_as_int(g.area[base + rc]));
                     if (cnt >= gamma) {
                         const int me = *rec_i(lv.rec, base + x, 3);
+                        lent[q] = make_uint2(m, (uint32_t)x);
                         if (me <= L) {
                             lvl[q] = me;
-                            lent[q] = make_uint2(m, (uint32_t)x);
                         } else {
+                            above = true;
                             if ((is_internal(lc, n) ? *rec_i(lv.rec, base + lc, 3) : 0) <= L)
                                 ent[push++] = make_uint2(m, (uint32_t)lc);
                             if ((is_internal(rc, n) ? *rec_i(lv.rec, base + rc, 3) : 0) <= L)
@@ -1089,67 +857,7 @@ __global__ void __launch_bounds__(256) k_levels_pp_hist(TreeRefs g, Segs segs, L
                 }
             }
         }
-        // Frontier entries: one atomic per warp.
-        uint32_t incl = push;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, o);
-            if ((threadIdx.x & 31) >= o) incl += y;
-        }
-        const uint32_t total = __shfl_sync(kFull, incl, 31);
-        uint32_t at = 0;
-        if ((threadIdx.x & 31) == 31 && total) at = atomicAdd(lv.n_frontier, total);
-        at = __shfl_sync(kFull, at, 31) + incl - push;
-        for (int k = 0; k < push; ++k) lv.frontier[at + k] = ent[k];
-    }
-    file_levels(lv, L, lvl, lent, s_cnt, s_base);
-}
-
-// Phase A of iterations after the first: the previous iteration left every
-// internal node's level for this one (next levels of the nodes it finished,
-// kept current by treelet rewrites), and subtree counts, nodesSah and child
-// records that are already final for nodes that are not treelet roots now.
-// Count the levels, mark this iteration's non-roots as non-roots for the next
-// one too, and list the frontier below the levels above L.
-__global__ void __launch_bounds__(256) k_level_hist(Segs segs, LevelRefs lv, const uint8_t* __restrict__ seg_iters,
-                                                    int iteration, int L) {
-    __shared__ uint32_t s_cnt[kMaxLevels + 2];
-    __shared__ uint32_t s_base[kMaxLevels + 2];
-    for (int k = threadIdx.x; k < L + 2; k += blockDim.x) s_cnt[k] = 0;
-    __syncthreads();
-    int lvl[kListPer];
-    uint2 lent[kListPer];
-#pragma unroll
-    for (int q = 0; q < kListPer; ++q) {
-        const uint32_t i = blockIdx.x * kListBlock + q * 256 + threadIdx.x;
-        int push = 0;
-        uint32_t m = 0;
-        uint2 ent[2];
-        lvl[q] = 0;
-        lent[q] = make_uint2(0u, 0u);
-        if (i < segs.n) {
-            m = segs.seg_of_tri(i);
-            const uint32_t s0 = segs.tri_begin(m);
-            const uint32_t n = segs.tri_end(m) - s0;
-            const uint32_t li = i - s0;
-            if ((!seg_iters || iteration < (int)seg_iters[m]) && li < n - 1) {
-                const int cb = segs.inner_base(m), nb = segs.node_base(m);
-                const int me = *rec_i(lv.rec, nb + (int)li, 3);
-                if (me == 0) {
-                    // Not a treelet root: its next nodesSah is this one (the level
-                    // stays 0).
-                    *rec_f(lv.rec, nb + (int)li, rec_ns_next(lv.par)) = *rec_f(lv.rec, nb + (int)li, rec_ns_cur(lv.par));
-                } else if (me <= L) {
-                    lvl[q] = me;
-                    lent[q] = make_uint2(m, li);
-                } else {
-                    const int4 kd = lv.kids[cb + (int)li];
-                    if ((is_internal(kd.x, n) ? *rec_i(lv.rec, nb + kd.x, 3) : 0) <= L)
-                        ent[push++] = make_uint2(m, (uint32_t)kd.x);
-                    if ((is_internal(kd.y, n) ? *rec_i(lv.rec, nb + kd.y, 3) : 0) <= L)
-                        ent[push++] = make_uint2(m, (uint32_t)kd.y);
-                }
-            }
-        }
+        list_top(lv, above, lent[q]);
         // Frontier entries: one atomic per warp.
         uint32_t incl = push;
         for (int o = 1; o < 32; o <<= 1) {
@@ -1517,6 +1225,41 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
     __syncwarp();
 }
 
+// The treelets of the calling warp's lane groups (QUADS: of four lanes, else of
+// G): `has` and the root `q` are a group's own, `leader` is one lane of it.
+template <int G, bool QUADS>
+__device__ __forceinline__ void restructure_roots(const TreeRefs& g, const Segs& segs, const LevelRefs& lv, bool has,
+                                                  uint2 q, bool leader, int tsize_all,
+                                                  const uint8_t* __restrict__ seg_tsize, int iteration, float ci,
+                                                  float* sm, const uint16_t* __restrict__ s_rc,
+                                                  const uint8_t* __restrict__ s_prio, uint32_t* err) {
+    int nb = 0, x = 0, tsize = 0;
+    uint32_t n = 2;
+    int4* kd = lv.kids;
+    float root_sah = 0.0f;
+    int4 rk = make_int4(-1, -1, 0, 0);
+    const int cur_c = rec_ns_cur(lv.par);
+    if (has) {
+        const uint32_t s0 = segs.tri_begin(q.x);
+        n = segs.tri_end(q.x) - s0;
+        nb = segs.node_base(q.x);
+        kd = lv.kids + segs.inner_base(q.x);
+        x = (int)q.y;
+        tsize = seg_tsize ? (int)seg_tsize[q.x] : tsize_all;
+        rk = __ldcg(kd + x);
+        root_sah = __fadd_rn(__fadd_rn(__fmul_rn(ci, __ldcg(g.area + nb + x)), ld_cg(rec_f(lv.rec, nb + rk.x, cur_c))),
+                             ld_cg(rec_f(lv.rec, nb + rk.y, cur_c)));
+        if (leader) *rec_f(lv.rec, nb + x, cur_c) = root_sah;
+    }
+    const int maxts = (int)__reduce_max_sync(kFull, has ? (unsigned)tsize : 0u);
+    __syncwarp();
+    const NextRefs nx{lv.rec + nb, lv.par, tsize << (iteration + 1), lv.ct};
+    if constexpr (QUADS)
+        process_quad<kQuadLeaves>(g, has, nb, n, x, rk, kd, nx, root_sah, tsize, maxts, ci, sm, s_rc, s_prio, err);
+    else
+        process_group<G>(g, has, nb, n, x, rk, kd, nx, root_sah, tsize, maxts, ci, sm, s_rc, s_prio, err);
+}
+
 // Phase C: every treelet root of level `lev`.  Each warp takes `per` roots
 // at a time: 32/G in lane groups of G, or (QUADS) eight in four-lane groups.
 template <int G, int W, bool QUADS>
@@ -1546,35 +1289,33 @@ __global__ void __launch_bounds__(W * 32, (G == 32 ? 16 : 32) / W) k_level_group
     for (uint32_t e0 = beg + warp * per; e0 < end; e0 += nwarps * per) {
         const uint32_t e = e0 + (uint32_t)grp;
         const bool has = grp < per && e < end;
-        int nb = 0, x = 0, tsize = 0;
-        uint32_t n = 2;
-        int4* kd = lv.kids;
-        float root_sah = 0.0f;
-        int4 rk = make_int4(-1, -1, 0, 0);
-        const int cur_c = rec_ns_cur(lv.par);
-        if (has) {
-            const uint2 q = lv.order[e];
-            const uint32_t s0 = segs.tri_begin(q.x);
-            n = segs.tri_end(q.x) - s0;
-            nb = segs.node_base(q.x);
-            kd = lv.kids + segs.inner_base(q.x);
-            x = (int)q.y;
-            tsize = seg_tsize ? (int)seg_tsize[q.x] : tsize_all;
-            rk = __ldcg(kd + x);
-            root_sah = __fadd_rn(__fadd_rn(__fmul_rn(ci, __ldcg(g.area + nb + x)), ld_cg(rec_f(lv.rec, nb + rk.x, cur_c))),
-                                 ld_cg(rec_f(lv.rec, nb + rk.y, cur_c)));
-            if (lane == grp * gw) *rec_f(lv.rec, nb + x, cur_c) = root_sah;
-        }
-        const int maxts = (int)__reduce_max_sync(kFull, has ? (unsigned)tsize : 0u);
-        __syncwarp();
-        const NextRefs nx{lv.rec + nb, lv.par, tsize << (iteration + 1), lv.ct};
         float* const sm = &s_mem[w][0] + (grp < per ? grp : per - 1) * kGroupFloats;
-        if constexpr (QUADS)
-            process_quad<kQuadLeaves>(g, has, nb, n, x, rk, kd, nx, root_sah, tsize, maxts, ci, sm, s_rc, s_prio,
-                                      err);
-        else
-            process_group<G>(g, has, nb, n, x, rk, kd, nx, root_sah, tsize, maxts, ci, sm, s_rc, s_prio, err);
+        restructure_roots<G, QUADS>(g, segs, lv, has, has ? lv.order[e] : make_uint2(0u, 0u), lane == grp * gw,
+                                    tsize_all, seg_tsize, iteration, ci, sm, s_rc, s_prio, err);
     }
+}
+
+__global__ void __launch_bounds__(kTopWarps * 32, 1) k_atr_top(TreeRefs g, Segs segs, LevelRefs lv, TopRefs tr,
+                                                               int L, int tsize_all,
+                                                               const uint8_t* __restrict__ seg_tsize, int iteration,
+                                                               float ci, uint32_t* err) {
+    __shared__ __align__(16) float s_mem[kTopWarps][GroupLayout<32>::kFloats];
+    __shared__ uint16_t s_rc[kMaxDist];
+    __shared__ __align__(4) uint8_t s_prio[(kMaxTreelet + 1) * 32];
+    __shared__ uint32_t s_off[kTopLevels + 1];
+    __shared__ uint32_t s_max;
+    for (int k = threadIdx.x; k < kMaxDist; k += blockDim.x) {
+        int r, c;
+        trm_rc(k, r, c);
+        s_rc[k] = (uint16_t)((r << 8) | c);
+    }
+    for (int k = threadIdx.x; k < (kMaxTreelet + 1) * 8; k += blockDim.x)
+        reinterpret_cast<uint32_t*>(s_prio)[k] = reinterpret_cast<const uint32_t*>(&g_argmax_priority.rank[0][0])[k];
+    __syncthreads();
+    top_levels(segs, lv, tr, L, s_off, &s_max, [&](uint2 q) {
+        restructure_roots<32, false>(g, segs, lv, true, q, (threadIdx.x & 31) == 0, tsize_all, seg_tsize, iteration,
+                                     ci, &s_mem[threadIdx.x >> 5][0], s_rc, s_prio, err);
+    });
 }
 
 template <int G, bool QUADS>
@@ -1587,6 +1328,11 @@ void launch_level_g(int warps, unsigned blocks, cudaStream_t s, const TreeRefs& 
         default: k_level_groups<G, 4, QUADS><<<blocks, 128, 0, s>>>(g, segs, lv, lev, tsize, seg_tsize, it, ci, err); break;
     }
 }
+
+constexpr int kDefaultLevels = 12;  // atr_ctx::atr_levels unless tuned
+// ATRBVH(9, 2) with the cluster and with the dataflow pass: 1,003 triangles 151
+// and 177 us, 65,536 311 and 321, 1,000,003 921 and 890.
+constexpr uint32_t kClusterTriangles = 131072;
 
 }  // namespace
 
@@ -1604,27 +1350,27 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
     if (iterations <= 0) return ATR_OK;
     const size_t inner = segs.n - segs.count;
     const int max_ts = seg_tsize ? max_tsize : tsize;
-    const int L = ctx->atr_levels;
+    // Level passes of iteration it, and what takes the levels above them.  Up to
+    // kClusterTriangles triangles the passes follow the size and a cluster of CTAs
+    // takes the rest; above, and with a number the context asks for, the dataflow
+    // pass does, whose climbs advance without waiting for the slowest treelet of a
+    // level.
+    const bool cluster = ctx->atr_levels == kDefaultLevels && segs.n <= kClusterTriangles;
+    auto levels_of = [&](int it) { return cluster ? auto_levels(segs.n, tsize << it) : ctx->atr_levels; };
+    const int L0 = levels_of(0);
     void* scratch = nullptr;
     const size_t b_rec = align256(total_nodes * 16), b_ctr = align256(inner * 4);
     const size_t b_kid = align256(inner * 16);
-    // Big nodes of one level root disjoint subtrees of at least gamma
-    // triangles (the first iteration's gamma, the smallest; 3 bounds per-mesh
-    // sizes), so each level's list holds at most n / gamma; frontier nodes
-    // root disjoint subtrees too, so they number at most the triangles.
-    const uint32_t gamma0 = seg_tsize ? 3u : (uint32_t)tsize;
-    const uint32_t cap = (segs.n + gamma0 - 1) / gamma0;
-    const size_t b_ord = L ? align256((size_t)L * cap * 8) : 0;
-    const size_t b_front = L ? align256((size_t)segs.n * 8) : 0;
-    const size_t b_small = L ? align256((size_t)((L + 2) + 1) * 4) : 0;
+    // Per-mesh sizes bound the first iteration's gamma by 3.
+    const LevelScratch ls(segs.n, seg_tsize ? 3u : (uint32_t)tsize, L0);
     // The build's prepass records (counts, first nodesSah, levels) serve as
     // the optimiser's records when its constants are this pass's.
-    const bool use_pp = prepass && prepass->rec && karras_ranges && L > 0 && ci == kPrepassCi && ct == kPrepassCt;
+    const bool use_pp = prepass && prepass->rec && karras_ranges && L0 > 0 && ci == kPrepassCi && ct == kPrepassCt;
     // ... and its levels serve as the first iteration's when its gamma is this
     // pass's treelet size (per mesh, when the sizes are per mesh).
     const bool use_pp_levels = use_pp && (seg_tsize ? prepass->seg_gamma == seg_tsize
                                                     : !prepass->seg_gamma && tsize == prepass->gamma);
-    ATR_TRY(ctx->alloc(&scratch, (use_pp ? 0 : b_rec) + b_kid + b_ctr + b_ord + b_front + b_small));
+    ATR_TRY(ctx->alloc(&scratch, (use_pp ? 0 : b_rec) + b_kid + b_ctr + ls.bytes()));
     char* p = static_cast<char*>(scratch);
     TreeRefs g = g_in;
     int4* rec;
@@ -1637,17 +1383,11 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
     int4* kids = reinterpret_cast<int4*>(p); p += b_kid;
     uint32_t* counters = reinterpret_cast<uint32_t*>(p); p += b_ctr;
     LevelRefs lv{};
+    TopRefs tr{};
     lv.rec = rec;
     lv.counters = counters;
     lv.kids = kids;
-    if (L) {
-        lv.order = reinterpret_cast<uint2*>(p); p += b_ord;
-        lv.cap = cap;
-        lv.err = ctx->d_error;
-        lv.frontier = reinterpret_cast<uint2*>(p); p += b_front;
-        lv.cursor = reinterpret_cast<uint32_t*>(p);
-        lv.n_frontier = lv.cursor + (L + 2);
-    }
+    if (L0) ls.bind(p, inner, ctx->d_error, lv, tr);
     const int warps = ctx->atr_warps == 2 || ctx->atr_warps == 4 ? ctx->atr_warps : 8;
     const int threads = warps * 32;
     const uint32_t leaf_blocks = (segs.n + threads - 1) / threads;
@@ -1658,17 +1398,19 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
     cudaError_t e = cudaSuccess;
     ctx->phase_begin("atrbvh");
     for (int it = 0; it < iterations && e == cudaSuccess; ++it) {
+        const int L = levels_of(it);
         lv.par = it & 1;
         lv.ct = ct;
         const bool hist_done = L && it == 0 && use_pp_levels;
-        // Arrival counters: for the first iteration's climbs, else only for
-        // the dataflow pass (cleared again below).
+        // Arrival counters: for the first iteration's climbs, or the dataflow
+        // pass without level passes (with them, cleared again below, or by k_atr_top
+        // when it leaves that pass work).
         if (!L || (it == 0 && !hist_done)) e = cudaMemsetAsync(counters, 0, inner * 4, st);
         const uint2* start = nullptr;
         const uint32_t* start_count = nullptr;
         uint32_t blocks = leaf_blocks;
         if (L && e == cudaSuccess) {
-            if (zero_words_async(ctx, lv.cursor, b_small / 4) != ATR_OK) e = cudaErrorLaunchFailure;
+            if (zero_words_async(ctx, lv.cursor, ls.b_small / 4) != ATR_OK) e = cudaErrorLaunchFailure;
             const unsigned gb = (segs.n + 255) / 256;
             const unsigned gbl = (segs.n + kListBlock - 1) / kListBlock;
             if (hist_done)
@@ -1689,13 +1431,11 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
                 ++ctx->launches;
             }
             const unsigned lg = (unsigned)ctx->num_sms * (256 / threads) * 4;
-            // Roots per level fall by about 0.62 per level from n / (1.5 gamma)
-            // at level 1 (gamma = tsize << it); levels expected to hold at
-            // least atr_quad_min roots run in four-lane groups, levels expected
-            // to hold at most atr_warp_max one treelet per warp (the shortest
-            // latency per treelet, for levels too narrow to fill the GPU).
-            const double gamma = (double)(tsize << it);
-            double expect = (double)segs.n / (1.5 * gamma);
+            // Levels expected to hold at least atr_quad_min roots run in four-lane
+            // groups, levels expected to hold at most atr_warp_max one treelet per
+            // warp (the shortest latency per treelet, for levels too narrow to
+            // fill the GPU).
+            double expect = level_roots(segs.n, tsize << it);
             for (int lev = 1; lev <= L; ++lev, expect *= 0.62) {
                 const bool quads = max_ts <= kQuadLeaves && ctx->atr_quad_min >= 0 && expect >= ctx->atr_quad_min;
                 const bool whole = !quads && max_ts <= kRegTreelet && expect <= (double)ctx->atr_warp_max;
@@ -1713,7 +1453,14 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
                 }
                 ++ctx->launches;
             }
-            if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, inner * 4, st);
+            if (e == cudaSuccess && cluster) {
+                cudaLaunchAttribute at{};
+                const cudaLaunchConfig_t cfg = top_config(ctx->top_ctas, &at, st);
+                e = cudaLaunchKernelEx(&cfg, k_atr_top, g, segs, lv, tr, L, tsize, seg_tsize, it, ci, ctx->d_error);
+                ++ctx->launches;
+            } else if (e == cudaSuccess) {
+                if (zero_words_async(ctx, counters, inner) != ATR_OK) e = cudaErrorLaunchFailure;
+            }
             start = lv.frontier;
             start_count = lv.n_frontier;
             blocks = front_blocks;
@@ -1733,8 +1480,8 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
     return ATR_OK;
 }
 
-// Kernel attributes (once per context); none are needed at present.
-int atrbvh_prepare() { return ATR_OK; }
+// Kernel attributes (once per context).
+int atrbvh_prepare(atr_ctx* ctx) { return top_cluster(k_atr_top, 0, &ctx->top_ctas); }
 
 }  // namespace atr
 
