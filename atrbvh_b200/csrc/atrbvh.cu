@@ -1494,7 +1494,7 @@ extern "C" int atr_optimize_atrbvh(atr_ctx* ctx, atr_tree* tree, int tsize, int 
     ATR_REQUIRE(iterations >= 0 && iterations <= 24, ATR_ERR_INVALID_ARG, "atr_optimize_atrbvh: iterations %d",
                 iterations);
     const uint32_t n = tree->n;
-    TreeRefs g{n, tree->parent, tree->left, tree->right, tree->bmin, tree->bmax, tree->area, nullptr};
+    TreeRefs g{n, tree->parent, tree->left, tree->right, tree->bmin, tree->bmax, tree->area};
     Segs segs{nullptr, nullptr, 1u, n};
     const int2* ranges = tree->karras ? tree->range : nullptr;
     const BuildPrepass* pp = tree->prepass_block ? &tree->prepass : nullptr;

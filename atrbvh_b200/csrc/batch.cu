@@ -125,7 +125,7 @@ int batch_run(atr_ctx* ctx, atr_batch* b, int optimizer, int tsize, int iteratio
     int st = lbvh_build_segs(ctx, segs, b->tiles, b->verts, b->d_bounds, 30, b->tree, nullptr, nullptr,
                              want_pp ? &pp : nullptr);
     if (st != ATR_OK) { ctx->release(ppb); return st; }
-    TreeRefs g{b->n, b->tree.parent, b->tree.left, b->tree.right, b->tree.bmin, b->tree.bmax, b->tree.area, nullptr};
+    TreeRefs g{b->n, b->tree.parent, b->tree.left, b->tree.right, b->tree.bmin, b->tree.bmax, b->tree.area};
     const uint8_t* ts = b->per_mesh_params ? b->d_tsize : nullptr;
     const uint8_t* it = b->per_mesh_params ? b->d_iters : nullptr;
     const int iters = b->per_mesh_params ? b->max_iters : iterations;
@@ -136,7 +136,7 @@ int batch_run(atr_ctx* ctx, atr_batch* b, int optimizer, int tsize, int iteratio
         return st;
     }
     ctx->release(ppb);
-    if (optimizer == 2) return trbvh_run(ctx, g, segs, b->total_nodes, iters, it, ci, ct);
+    if (optimizer == 2) return trbvh_run(ctx, g, segs, b->total_nodes, iters, it, ci, ct, b->tree.range);
     return ATR_OK;
 }
 

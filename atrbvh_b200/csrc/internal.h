@@ -106,7 +106,7 @@ struct atr_ctx {
     // four-lane groups (eight per warp); -1 = never.
     int atr_quad_min = 20000;
     int atr_warp_max = 4096;
-    int top_ctas = 8;  // cluster size of the ATRBVH top kernel (atrbvh_prepare)
+    int top_ctas = 8, tr_top_ctas = 8;  // cluster sizes of the ATRBVH and TRBVH top kernels
     struct Phase {
         std::string name;
         cudaEvent_t a, b;
@@ -285,7 +285,8 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_n
 int atrbvh_group_width(int max_tsize);
 int atrbvh_prepare(atr_ctx* ctx);  // kernel attributes; once per context
 int trbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_nodes, int iterations,
-              const uint8_t* seg_iters, float ci, float ct);
+              const uint8_t* seg_iters, float ci, float ct, const int2* karras_ranges = nullptr);
+int trbvh_prepare(atr_ctx* ctx);  // kernel attributes; once per context
 
 constexpr uint32_t kSortTileSize = 3072;  // triangles per sort tile (lbvh.cu)
 int lbvh_prepare();                       // kernel attributes; once per context
