@@ -70,6 +70,13 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
+// Digits (bit k: 8-bit digit k, 0..23) of six-word keys in which some key differs
+// from the first, from the words' difference bits.  Called by whole warps.
+__device__ __forceinline__ uint32_t active_digits(const uint32_t* __restrict__ diff) {
+    const uint32_t lane = threadIdx.x & 31;
+    return __ballot_sync(kFull, lane < 24 && ((__ldg(diff + (lane < 24 ? lane >> 2 : 0)) >> (8 * (lane & 3))) & 255u));
+}
+
 __device__ __forceinline__ void set_error_bits(uint32_t* err, uint32_t bits) {
     if (err) atomicOr(err, bits);
 }

@@ -288,6 +288,9 @@ int trbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_no
               const uint8_t* seg_iters, float ci, float ct, const int2* karras_ranges = nullptr);
 int trbvh_prepare(atr_ctx* ctx);  // kernel attributes; once per context
 
+int sort_ray_words(atr_ctx* ctx, const uint32_t* words, const uint32_t* diff, uint32_t n, uint32_t* keys_a,
+                   uint32_t* keys_b, uint32_t* perm_a, uint32_t* perm_b);
+
 constexpr uint32_t kSortTileSize = 3072;  // triangles per sort tile (lbvh.cu)
 int lbvh_prepare();                       // kernel attributes; once per context
 

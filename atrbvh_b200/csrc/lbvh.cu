@@ -240,6 +240,18 @@ __device__ __forceinline__ void block_exclusive_scan(const uint32_t (&x)[R], uin
 // (the decoupled look-back this replaces spent a third of every pass walking
 // over the aggregates of the tiles running beside it).
 
+// A pass over one 8-bit digit (0..23, least significant first) of 192-bit ray
+// keys kept as six words of n keys each (word w of key i at words[w n + i]).
+// The keys travel as one word at a time with their permutation, in two buffers;
+// a digit that all keys share is skipped, so the device decides which buffer a
+// pass reads: `diff` holds the bits in which some key differs from the first
+// (see active_digits in common.cuh).
+struct WordPass {
+    const uint32_t* diff = nullptr;  // nullptr: not a word pass
+    const uint32_t* words = nullptr;
+    int digit = 0;
+};
+
 // Tile counts of digit `pass` (D per tile, tile-major).  A thread loads its
 // kSortItems keys at once and counts them with shared atomics into its warp's
 // own histogram (no ranks are needed here); the warps' histograms are summed
@@ -275,6 +287,56 @@ __global__ void __launch_bounds__(kSortThreads) k_tile_counts(Segs segs, const K
     }
 }
 
+// Tile counts of a word pass.  The first pass over a word fetches it through the
+// permutation and leaves it beside it.
+__global__ void __launch_bounds__(kSortThreads) k_word_counts(uint32_t n, WordPass wp, uint32_t* __restrict__ keys_a,
+                                                               uint32_t* __restrict__ keys_b,
+                                                               const uint32_t* __restrict__ perm_a,
+                                                               const uint32_t* __restrict__ perm_b,
+                                                               uint32_t* __restrict__ counts) {
+    __shared__ uint32_t sh[kSortWarps][256];
+    const uint32_t active = active_digits(wp.diff);
+    const int in_word = wp.digit & 3;
+    const bool fetch = in_word == 0 && ((active >> wp.digit) & 15u) != 0u;
+    const bool mine = (active >> wp.digit) & 1u;
+    if (!fetch && !mine) return;
+    const bool odd = __popc(active & ((1u << wp.digit) - 1u)) & 1;
+    uint32_t* const keys = odd ? keys_b : keys_a;
+    const uint32_t* const perm = odd ? perm_b : perm_a;
+    const uint32_t* const word = wp.words + (size_t)(wp.digit >> 2) * n;
+    const uint32_t base = blockIdx.x * kSortTile;
+    for (int j = threadIdx.x; j < kSortWarps * 256; j += kSortThreads) (&sh[0][0])[j] = 0;
+    uint32_t key[kSortItems];
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const uint32_t i = base + r * kSortThreads + threadIdx.x;
+        key[r] = i < n ? (fetch ? perm[i] : keys[i]) : 0u;
+    }
+    if (fetch) {
+#pragma unroll
+        for (int r = 0; r < kSortItems; ++r)
+            if (base + r * kSortThreads + threadIdx.x < n) key[r] = __ldg(word + key[r]);
+#pragma unroll
+        for (int r = 0; r < kSortItems; ++r) {
+            const uint32_t i = base + r * kSortThreads + threadIdx.x;
+            if (i < n) keys[i] = key[r];
+        }
+    }
+    if (!mine) return;
+    __syncthreads();
+    uint32_t* const wh = sh[threadIdx.x >> 5];
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r)
+        if (base + r * kSortThreads + threadIdx.x < n) atomicAdd(&wh[(key[r] >> (8 * in_word)) & 255u], 1u);
+    __syncthreads();
+    for (int j = threadIdx.x; j < 256; j += kSortThreads) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int w = 0; w < kSortWarps; ++w) c += sh[w][j];
+        counts[(size_t)blockIdx.x * 256 + j] = c;
+    }
+}
+
 // In place: counts[t][d] -> the sum of counts[t'][d] over the earlier tiles
 // t' of t's mesh within t's chunk of kPrefixChunk tiles.  Block (x, y) takes
 // 32 digits (one per lane) and chunk y, split into 32 runs of 8 tiles (one
@@ -284,6 +346,12 @@ __global__ void __launch_bounds__(kSortThreads) k_tile_counts(Segs segs, const K
 // bit set when it holds one) goes to chunk_tot; k_chunk_carry turns those
 // into each chunk's carry from earlier chunks, which the scatter adds for a
 // tile whose mesh began before its chunk.
+//
+// FOLD: block x walks all the chunks of its 32 digits instead, carrying the
+// sums along, so the counts come out whole and no carry pass follows; used up to
+// kFoldChunks chunks (a chunk takes the walk about 1 us, k_chunk_carry and its
+// launch 4.5 us), and by the word passes, which take each digit's total from here.
+constexpr uint32_t kFoldChunks = 4;
 constexpr int kPrefixRuns = 32;
 constexpr int kPrefixRunTiles = 8;
 constexpr uint32_t kPrefixChunk = kPrefixRuns * kPrefixRunTiles;
@@ -294,63 +362,79 @@ __device__ __forceinline__ uint32_t next_mesh_tile(const Segs& segs, uint32_t m)
     return m + 1 < segs.count ? segs.tile_begin(m + 1) : 0xffffffffu;
 }
 
-template <int D>
+template <int D, bool FOLD>
 __global__ void __launch_bounds__(32 * kPrefixRuns) k_tile_prefix(Segs segs, uint32_t tiles,
                                                                    uint32_t* __restrict__ counts,
-                                                                   uint32_t* __restrict__ chunk_tot) {
+                                                                   uint32_t* __restrict__ chunk_tot, WordPass wp) {
     __shared__ uint32_t s_sum[kPrefixRuns][32];
     __shared__ uint8_t s_cut[kPrefixRuns][32];
+    __shared__ uint32_t s_in[32];  // FOLD: the carry into the chunk
+    if (FOLD && wp.diff && !((active_digits(wp.diff) >> wp.digit) & 1u)) return;
     const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
     const uint32_t d = blockIdx.x * 32 + lane;
-    const uint32_t c0 = blockIdx.y * kPrefixChunk;
-    const uint32_t t0 = min(tiles, c0 + run * kPrefixRunTiles), t1 = min(tiles, t0 + kPrefixRunTiles);
-    const uint32_t m0 = t0 < t1 ? segs.seg_of_tile(t0) : 0;
-    const bool starts = t0 < t1 && t0 == segs.tile_begin(m0);  // the run begins a mesh
-    const uint32_t next0 = t0 < t1 ? next_mesh_tile(segs, m0) : 0xffffffffu;
-    uint32_t v[kPrefixRunTiles];
+    if (FOLD && run == 0) s_in[lane] = 0u;
+    const uint32_t c_end = FOLD ? tiles : blockIdx.y * kPrefixChunk + 1;
+    for (uint32_t c0 = FOLD ? 0u : blockIdx.y * kPrefixChunk; c0 < c_end; c0 += kPrefixChunk) {
+        const uint32_t t0 = min(tiles, c0 + run * kPrefixRunTiles), t1 = min(tiles, t0 + kPrefixRunTiles);
+        const uint32_t m0 = t0 < t1 ? segs.seg_of_tile(t0) : 0;
+        const bool starts = t0 < t1 && t0 == segs.tile_begin(m0);  // the run begins a mesh
+        const uint32_t next0 = t0 < t1 ? next_mesh_tile(segs, m0) : 0xffffffffu;
+        uint32_t v[kPrefixRunTiles];
 #pragma unroll
-    for (int u = 0; u < kPrefixRunTiles; ++u) v[u] = t0 + u < t1 ? counts[(size_t)(t0 + u) * D + d] : 0u;
-    uint32_t sum = 0;
-    bool cut = starts;
-    {
+        for (int u = 0; u < kPrefixRunTiles; ++u) v[u] = t0 + u < t1 ? counts[(size_t)(t0 + u) * D + d] : 0u;
+        uint32_t sum = 0;
+        bool cut = starts;
+        {
+            uint32_t m = m0, next = next0;
+#pragma unroll
+            for (int u = 0; u < kPrefixRunTiles; ++u) {
+                if (t0 + u < t1 && t0 + u == next) {  // a mesh starts here: the run's sum restarts
+                    sum = 0;
+                    cut = true;
+                    next = next_mesh_tile(segs, ++m);
+                }
+                sum += v[u];
+            }
+        }
+        s_sum[run][lane] = sum;
+        s_cut[run][lane] = cut;
+        __syncthreads();
+        // Carry into this run from the chunk's earlier runs, back to the last cut.
+        uint32_t carry = 0;
+        if (!starts) {
+            int r = run - 1;
+            for (; r >= 0; --r) {
+                carry += s_sum[r][lane];
+                if (s_cut[r][lane]) break;
+            }
+            if (FOLD && r < 0) carry += s_in[lane];
+        }
+        const uint32_t out = cut ? sum : carry + sum;
+        if (!FOLD && run == kPrefixRuns - 1) {
+            bool any = false;
+            for (int r = 0; r < kPrefixRuns; ++r) any |= s_cut[r][lane] != 0;
+            chunk_tot[(size_t)blockIdx.y * D + d] = out | (any ? kCutBit : 0u);
+        }
+        uint32_t acc = carry;
         uint32_t m = m0, next = next0;
 #pragma unroll
         for (int u = 0; u < kPrefixRunTiles; ++u) {
-            if (t0 + u < t1 && t0 + u == next) {  // a mesh starts here: the run's sum restarts
-                sum = 0;
-                cut = true;
+            if (t0 + u >= t1) break;
+            if (t0 + u == next) {
+                acc = 0;
                 next = next_mesh_tile(segs, ++m);
             }
-            sum += v[u];
+            counts[(size_t)(t0 + u) * D + d] = acc;
+            acc += v[u];
+        }
+        if (FOLD) {
+            __syncthreads();  // every run has read s_in
+            if (run == kPrefixRuns - 1) s_in[lane] = out;
+            __syncthreads();
         }
     }
-    s_sum[run][lane] = sum;
-    s_cut[run][lane] = cut;
-    __syncthreads();
-    // Carry into this run from the chunk's earlier runs, back to the last cut.
-    uint32_t carry = 0;
-    if (!starts)
-        for (int r = run - 1; r >= 0; --r) {
-            carry += s_sum[r][lane];
-            if (s_cut[r][lane]) break;
-        }
-    if (run == kPrefixRuns - 1) {
-        bool any = false;
-        for (int r = 0; r < kPrefixRuns; ++r) any |= s_cut[r][lane] != 0;
-        chunk_tot[(size_t)blockIdx.y * D + d] = (cut ? sum : carry + sum) | (any ? kCutBit : 0u);
-    }
-    uint32_t acc = carry;
-    uint32_t m = m0, next = next0;
-#pragma unroll
-    for (int u = 0; u < kPrefixRunTiles; ++u) {
-        if (t0 + u >= t1) break;
-        if (t0 + u == next) {
-            acc = 0;
-            next = next_mesh_tile(segs, ++m);
-        }
-        counts[(size_t)(t0 + u) * D + d] = acc;
-        acc += v[u];
-    }
+    // A word pass has one mesh: what the last chunk carries out is the total.
+    if (FOLD && wp.diff && run == kPrefixRuns - 1) chunk_tot[d] = s_in[lane];
 }
 
 // In place over the chunk totals: chunk_tot[y][d] -> the segmented sum of the
@@ -380,14 +464,15 @@ __global__ void __launch_bounds__(256) k_chunk_carry(uint32_t chunks, uint32_t* 
 // mesh, prefix the tile's offsets within its chunk from k_tile_prefix,
 // chunk_carry the chunk's carry for tiles whose mesh began before the chunk).  Each
 // thread owns R = D / 256 consecutive digits in the tile-wide steps.
+// chunk_carry is nullptr when the prefixes are whole; hist is the pass's row of D.
 template <typename K, bool kIota, int BITS>
-__global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 ? 4 : 3) k_scatter(
-        Segs segs, const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
-        uint32_t* __restrict__ vout, int pass, const uint32_t* __restrict__ hist,
-        const uint32_t* __restrict__ prefix, const uint32_t* __restrict__ chunk_carry) {
+__device__ __forceinline__ void scatter_tile(const Segs& segs, const K* __restrict__ kin,
+                                             const uint32_t* __restrict__ vin, K* __restrict__ kout,
+                                             uint32_t* __restrict__ vout, int shift, const uint32_t* __restrict__ hist,
+                                             size_t hist_stride, const uint32_t* __restrict__ prefix,
+                                             const uint32_t* __restrict__ chunk_carry) {
     using Plan = SortPlan<K, BITS>;
-    constexpr int P = Plan::kPasses, D = Plan::kDigits, R = Plan::kPerThread;
-    const int shift = BITS * pass;
+    constexpr int D = Plan::kDigits, R = Plan::kPerThread;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     K* s_keys = reinterpret_cast<K*>(smem_raw);
     uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + kSortTile);
@@ -446,7 +531,7 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 ? 4 : 3) k_scatte
             run += c;
         }
         count[r] = run;
-        hv[r] = hist[((size_t)m * P + pass) * D + d];
+        hv[r] = hist[m * hist_stride + d];
     }
     block_exclusive_scan<R>(count, dstart, s_scan);
     block_exclusive_scan<R>(hv, gdig, s_scan);
@@ -455,7 +540,7 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 ? 4 : 3) k_scatte
     for (int r = 0; r < R; ++r) {
         const int d = threadIdx.x * R + r;
         s_dstart[d] = dstart[r];
-        const uint32_t carry = segs.tile_begin(m) < chunk0 ? chunk_carry[(size_t)chunk * D + d] : 0u;
+        const uint32_t carry = chunk_carry && segs.tile_begin(m) < chunk0 ? chunk_carry[(size_t)chunk * D + d] : 0u;
         s_gbase[d] = seg_start + gdig[r] + prefix[(size_t)tile * D + d] + carry - dstart[r];
     }
     __syncthreads();
@@ -479,6 +564,29 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 ? 4 : 3) k_scatte
             vout[dst] = s_vals[i];
         }
     }
+}
+
+template <typename K, bool kIota, int BITS>
+__global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 ? 4 : 3) k_scatter(
+        Segs segs, const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
+        uint32_t* __restrict__ vout, int pass, const uint32_t* __restrict__ hist,
+        const uint32_t* __restrict__ prefix, const uint32_t* __restrict__ chunk_carry) {
+    constexpr int P = SortPlan<K, BITS>::kPasses, D = SortPlan<K, BITS>::kDigits;
+    scatter_tile<K, kIota, BITS>(segs, kin, vin, kout, vout, BITS * pass, hist + pass * D, (size_t)P * D, prefix,
+                                 chunk_carry);
+}
+
+// A word pass: from one pair of buffers to the other, by the number of passes
+// that ran before it.
+__global__ void __launch_bounds__(kSortThreads, 4) k_word_scatter(Segs segs, WordPass wp, uint32_t* keys_a,
+                                                                  uint32_t* keys_b, uint32_t* perm_a, uint32_t* perm_b,
+                                                                  const uint32_t* __restrict__ total,
+                                                                  const uint32_t* __restrict__ prefix) {
+    const uint32_t active = active_digits(wp.diff);
+    if (!((active >> wp.digit) & 1u)) return;
+    const bool odd = __popc(active & ((1u << wp.digit) - 1u)) & 1;
+    scatter_tile<uint32_t, false, 8>(segs, odd ? keys_b : keys_a, odd ? perm_b : perm_a, odd ? keys_a : keys_b,
+                                     odd ? perm_a : perm_b, 8 * (wp.digit & 3), total, 0, prefix, nullptr);
 }
 
 // ---- fused Karras build + refit ------------------------------------------------
@@ -853,22 +961,27 @@ int sort_pairs(atr_ctx* ctx, const Segs& segs, uint32_t tiles, K** keys, uint32_
     K* ka = *keys; K* kb2 = k2;
     uint32_t* va = *vals; uint32_t* vb2 = v2;
     const dim3 prefix_grid((unsigned)(D / 32), chunks);
+    const uint32_t* const carry = chunks > kFoldChunks ? chunk_tot : nullptr;
     for (int pass = 0; pass < P && e == cudaSuccess; ++pass) {
         if (pass > 0 || !tile_counts0) {
             k_tile_counts<K, BITS><<<tiles, kSortThreads, 0, s>>>(segs, ka, pass, counts);
             ctx->launches += 1;
         }
-        k_tile_prefix<D><<<prefix_grid, 32 * kPrefixRuns, 0, s>>>(segs, tiles, counts, chunk_tot);
-        if (chunks > 1) {
+        if (chunks <= kFoldChunks)
+            k_tile_prefix<D, true><<<D / 32, 32 * kPrefixRuns, 0, s>>>(segs, tiles, counts, chunk_tot, WordPass{});
+        else
+            k_tile_prefix<D, false><<<prefix_grid, 32 * kPrefixRuns, 0, s>>>(segs, tiles, counts, chunk_tot,
+                                                                             WordPass{});
+        if (chunks > kFoldChunks) {
             k_chunk_carry<D><<<(D + 255) / 256, 256, 0, s>>>(chunks, chunk_tot);
             ctx->launches += 1;
         }
         if (pass == 0 && iota)
             k_scatter<K, true, BITS><<<tiles, kSortThreads, Plan::kSmem, s>>>(segs, ka, va, kb2, vb2, pass, hist,
-                                                                              counts, chunk_tot);
+                                                                              counts, carry);
         else
             k_scatter<K, false, BITS><<<tiles, kSortThreads, Plan::kSmem, s>>>(segs, ka, va, kb2, vb2, pass, hist,
-                                                                               counts, chunk_tot);
+                                                                               counts, carry);
         ctx->launches += 2;
         std::swap(ka, kb2);
         std::swap(va, vb2);
@@ -967,6 +1080,8 @@ int lbvh_prepare() {
     ATR_CUDA((scatter_attrs<uint32_t, 10>()));
     ATR_CUDA((scatter_attrs<uint64_t, 8>()));
     ATR_CUDA((scatter_attrs<uint64_t, 10>()));
+    ATR_CUDA(cudaFuncSetAttribute(k_word_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)SortPlan<uint32_t, 8>::kSmem));
     return ATR_OK;
 }
 
@@ -1012,6 +1127,34 @@ int lbvh_build_into(atr_ctx* ctx, const float4* verts, uint32_t n, const float* 
     t->sorted_keys = keys;
     t->sorted_idx = idx;
     t->karras = true;
+    return ATR_OK;
+}
+
+// Sorts the permutation of n ray keys (six words each, WordPass) that perm_a
+// holds; keys_a / keys_b and perm_b are scratch.  The result is in perm_a or,
+// after an odd number of active digits, in perm_b.
+int sort_ray_words(atr_ctx* ctx, const uint32_t* words, const uint32_t* diff, uint32_t n, uint32_t* keys_a,
+                   uint32_t* keys_b, uint32_t* perm_a, uint32_t* perm_b) {
+    using Plan = SortPlan<uint32_t, 8>;
+    const Segs segs{nullptr, nullptr, 1u, n};
+    const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
+    void* tmp = nullptr;
+    const size_t cbytes = align256((size_t)tiles * 256 * 4);
+    ATR_TRY(ctx->alloc(&tmp, cbytes + 256 * 4));
+    uint32_t* counts = static_cast<uint32_t*>(tmp);
+    uint32_t* total = reinterpret_cast<uint32_t*>(static_cast<char*>(tmp) + cbytes);
+    cudaStream_t s = ctx->stream;
+    for (int digit = 0; digit < 24; ++digit) {
+        const WordPass wp{diff, words, digit};
+        k_word_counts<<<tiles, kSortThreads, 0, s>>>(n, wp, keys_a, keys_b, perm_a, perm_b, counts);
+        k_tile_prefix<256, true><<<8, 32 * kPrefixRuns, 0, s>>>(segs, tiles, counts, total, wp);
+        k_word_scatter<<<tiles, kSortThreads, Plan::kSmem, s>>>(segs, wp, keys_a, keys_b, perm_a, perm_b, total,
+                                                                counts);
+    }
+    ctx->launches += 72;
+    ctx->release(tmp);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "ray key sort", __FILE__, __LINE__);
     return ATR_OK;
 }
 
