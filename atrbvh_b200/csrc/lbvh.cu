@@ -12,6 +12,7 @@
 
 #include <climits>
 #include <cstdio>
+#include <type_traits>
 #include <utility>
 
 #include "common.cuh"
@@ -21,8 +22,22 @@ namespace atr {
 namespace {
 
 constexpr int kSortThreads = 256;
+// Keys per thread, hence per tile.  Batches use kSortItems; a single sort of up
+// to kTilesWanted tiles of 3 or 6 keys a thread uses those (sort_items): with
+// fewer tiles than the GPU holds at once, a pass costs one block's chain of
+// ranking rounds, which is shorter in smaller tiles.
 constexpr int kSortItems = 12;
 constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr uint32_t kTilesWanted = 256;
+inline int sort_items(uint32_t n) {
+    return n <= kTilesWanted * kSortThreads * 3 ? 3 : n <= kTilesWanted * kSortThreads * 6 ? 6 : kSortItems;
+}
+template <class F>
+auto with_items(int items, F f) {
+    if (items == 3) return f(std::integral_constant<int, 3>{});
+    if (items == 6) return f(std::integral_constant<int, 6>{});
+    return f(std::integral_constant<int, kSortItems>{});
+}
 constexpr int kSortWarps = kSortThreads / 32;
 
 // Digit plan of an LSD sort of K keys with BITS-bit digits.  8-bit digits
@@ -37,7 +52,9 @@ struct SortPlan {
     static constexpr int kPerThread = kDigits / kSortThreads;  // digits per thread in tile-wide steps
     // Dynamic shared memory of one scatter block: the tile's keys and
     // values, per-warp digit counters, digit starts and global bases.
-    static constexpr size_t kSmem = (size_t)kSortTile * (sizeof(K) + 4) + (size_t)(kSortWarps + 2) * kDigits * 4;
+    static constexpr size_t smem(int items) {
+        return (size_t)kSortThreads * items * (sizeof(K) + 4) + (size_t)(kSortWarps + 2) * kDigits * 4;
+    }
 };
 
 // ---- scene bounds (SceneConverter.cpp:28-60 on the device) -----------------
@@ -126,13 +143,33 @@ __device__ __forceinline__ uint64_t morton_code<uint64_t>(float cx, float cy, fl
     return q[0] * 4u + q[1] * 2u + q[2];
 }
 
+// The code of triangle (or primitive) t in the box b.
+template <typename K>
+__device__ __forceinline__ K prim_code(const float4* __restrict__ v, const PrimBoxes& pr, uint32_t t, const float* b) {
+    float cx, cy, cz;
+    if (pr.bmin) {
+        // A primitive box's centroid, (min + max) / 2 (LBVH.cu:41-49; the
+        // halving is exact, so it equals the product by 0.5).
+        const float4 lo = __ldg(pr.bmin + t), hi = __ldg(pr.bmax + t);
+        cx = __fmul_rn(__fadd_rn(lo.x, hi.x), 0.5f);
+        cy = __fmul_rn(__fadd_rn(lo.y, hi.y), 0.5f);
+        cz = __fmul_rn(__fadd_rn(lo.z, hi.z), 0.5f);
+    } else {
+        const float4 a = __ldg(v + 3 * (size_t)t), p = __ldg(v + 3 * (size_t)t + 1), c = __ldg(v + 3 * (size_t)t + 2);
+        cx = __fmul_rn(__fadd_rn(fmaxf(fmaxf(a.x, p.x), c.x), fminf(fminf(a.x, p.x), c.x)), 0.5f);
+        cy = __fmul_rn(__fadd_rn(fmaxf(fmaxf(a.y, p.y), c.y), fminf(fminf(a.y, p.y), c.y)), 0.5f);
+        cz = __fmul_rn(__fadd_rn(fmaxf(fmaxf(a.z, p.z), c.z), fminf(fminf(a.z, p.z), c.z)), 0.5f);
+    }
+    return morton_code<K>(cx, cy, cz, b);
+}
+
 // One block per sort tile (kSortTile triangles of one mesh); histograms of
 // every digit of every pass are accumulated in shared memory and added to the
 // mesh's histograms (P x D per mesh) once per block; the block's own counts
 // of the first pass's digits are the sort's first tile counts (D per tile in
 // tile_counts).  Each mesh is normalised to its own box (6 floats per mesh
 // in `bounds`).
-template <typename K, int BITS>
+template <typename K, int BITS, int ITEMS>
 __global__ void __launch_bounds__(256) k_morton(Segs segs, const float4* __restrict__ v,
                                                  const float* __restrict__ bounds, K* __restrict__ keys,
                                                  uint32_t* __restrict__ hist, uint32_t* __restrict__ tile_counts,
@@ -140,6 +177,7 @@ __global__ void __launch_bounds__(256) k_morton(Segs segs, const float4* __restr
     constexpr int P = SortPlan<K, BITS>::kPasses, D = SortPlan<K, BITS>::kDigits;
     __shared__ uint32_t sh[P * D];
     __shared__ float sb[6];
+    constexpr uint32_t kSortTile = kSortThreads * ITEMS;
     const uint32_t m = segs.seg_of_tile(blockIdx.x);
     const uint32_t t0 = segs.tri_begin(m) + (blockIdx.x - segs.tile_begin(m)) * kSortTile;
     const uint32_t t1 = min(t0 + kSortTile, segs.tri_end(m));
@@ -147,21 +185,7 @@ __global__ void __launch_bounds__(256) k_morton(Segs segs, const float4* __restr
     if (threadIdx.x < 6) sb[threadIdx.x] = bounds[6 * m + threadIdx.x];
     __syncthreads();
     for (uint32_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
-        float cx, cy, cz;
-        if (pr.bmin) {
-            // A primitive box's centroid, (min + max) / 2 (LBVH.cu:41-49; the
-            // halving is exact, so it equals the product by 0.5).
-            const float4 lo = __ldg(pr.bmin + t), hi = __ldg(pr.bmax + t);
-            cx = __fmul_rn(__fadd_rn(lo.x, hi.x), 0.5f);
-            cy = __fmul_rn(__fadd_rn(lo.y, hi.y), 0.5f);
-            cz = __fmul_rn(__fadd_rn(lo.z, hi.z), 0.5f);
-        } else {
-            const float4 a = __ldg(v + 3 * (size_t)t), b = __ldg(v + 3 * (size_t)t + 1), c = __ldg(v + 3 * (size_t)t + 2);
-            cx = __fmul_rn(__fadd_rn(fmaxf(fmaxf(a.x, b.x), c.x), fminf(fminf(a.x, b.x), c.x)), 0.5f);
-            cy = __fmul_rn(__fadd_rn(fmaxf(fmaxf(a.y, b.y), c.y), fminf(fminf(a.y, b.y), c.y)), 0.5f);
-            cz = __fmul_rn(__fadd_rn(fmaxf(fmaxf(a.z, b.z), c.z), fminf(fminf(a.z, b.z), c.z)), 0.5f);
-        }
-        const K code = morton_code<K>(cx, cy, cz, sb);
+        const K code = prim_code<K>(v, pr, t, sb);
         keys[t] = code;
         if (hist) {
 #pragma unroll
@@ -256,10 +280,10 @@ struct WordPass {
 // kSortItems keys at once and counts them with shared atomics into its warp's
 // own histogram (no ranks are needed here); the warps' histograms are summed
 // at the end.
-template <typename K, int BITS>
+template <typename K, int BITS, int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) k_tile_counts(Segs segs, const K* __restrict__ keys, int pass,
                                                                uint32_t* __restrict__ counts) {
-    constexpr int D = SortPlan<K, BITS>::kDigits;
+    constexpr int D = SortPlan<K, BITS>::kDigits, kSortTile = kSortThreads * ITEMS;
     __shared__ uint32_t sh[kSortWarps][D];
     const int shift = BITS * pass;
     const uint32_t tile = blockIdx.x;
@@ -267,16 +291,16 @@ __global__ void __launch_bounds__(kSortThreads) k_tile_counts(Segs segs, const K
     const uint32_t base = segs.tri_begin(m) + (tile - segs.tile_begin(m)) * kSortTile;
     const uint32_t end = min(base + (uint32_t)kSortTile, segs.tri_end(m));
     for (int j = threadIdx.x; j < kSortWarps * D; j += kSortThreads) (&sh[0][0])[j] = 0;
-    uint32_t dg[kSortItems];
+    uint32_t dg[ITEMS];
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const uint32_t i = base + r * kSortThreads + threadIdx.x;
         dg[r] = i < end ? (uint32_t)((keys[i] >> shift) & (D - 1)) : (uint32_t)D;
     }
     __syncthreads();
     uint32_t* const wh = sh[threadIdx.x >> 5];
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r)
+    for (int r = 0; r < ITEMS; ++r)
         if (dg[r] < (uint32_t)D) atomicAdd(&wh[dg[r]], 1u);
     __syncthreads();
     for (int j = threadIdx.x; j < D; j += kSortThreads) {
@@ -289,11 +313,13 @@ __global__ void __launch_bounds__(kSortThreads) k_tile_counts(Segs segs, const K
 
 // Tile counts of a word pass.  The first pass over a word fetches it through the
 // permutation and leaves it beside it.
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) k_word_counts(uint32_t n, WordPass wp, uint32_t* __restrict__ keys_a,
                                                                uint32_t* __restrict__ keys_b,
                                                                const uint32_t* __restrict__ perm_a,
                                                                const uint32_t* __restrict__ perm_b,
                                                                uint32_t* __restrict__ counts) {
+    constexpr int kSortTile = kSortThreads * ITEMS;
     __shared__ uint32_t sh[kSortWarps][256];
     const uint32_t active = active_digits(wp.diff);
     const int in_word = wp.digit & 3;
@@ -306,18 +332,18 @@ __global__ void __launch_bounds__(kSortThreads) k_word_counts(uint32_t n, WordPa
     const uint32_t* const word = wp.words + (size_t)(wp.digit >> 2) * n;
     const uint32_t base = blockIdx.x * kSortTile;
     for (int j = threadIdx.x; j < kSortWarps * 256; j += kSortThreads) (&sh[0][0])[j] = 0;
-    uint32_t key[kSortItems];
+    uint32_t key[ITEMS];
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const uint32_t i = base + r * kSortThreads + threadIdx.x;
         key[r] = i < n ? (fetch ? perm[i] : keys[i]) : 0u;
     }
     if (fetch) {
 #pragma unroll
-        for (int r = 0; r < kSortItems; ++r)
+        for (int r = 0; r < ITEMS; ++r)
             if (base + r * kSortThreads + threadIdx.x < n) key[r] = __ldg(word + key[r]);
 #pragma unroll
-        for (int r = 0; r < kSortItems; ++r) {
+        for (int r = 0; r < ITEMS; ++r) {
             const uint32_t i = base + r * kSortThreads + threadIdx.x;
             if (i < n) keys[i] = key[r];
         }
@@ -326,7 +352,7 @@ __global__ void __launch_bounds__(kSortThreads) k_word_counts(uint32_t n, WordPa
     __syncthreads();
     uint32_t* const wh = sh[threadIdx.x >> 5];
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r)
+    for (int r = 0; r < ITEMS; ++r)
         if (base + r * kSortThreads + threadIdx.x < n) atomicAdd(&wh[(key[r] >> (8 * in_word)) & 255u], 1u);
     __syncthreads();
     for (int j = threadIdx.x; j < 256; j += kSortThreads) {
@@ -465,14 +491,14 @@ __global__ void __launch_bounds__(256) k_chunk_carry(uint32_t chunks, uint32_t* 
 // chunk_carry the chunk's carry for tiles whose mesh began before the chunk).  Each
 // thread owns R = D / 256 consecutive digits in the tile-wide steps.
 // chunk_carry is nullptr when the prefixes are whole; hist is the pass's row of D.
-template <typename K, bool kIota, int BITS>
+template <typename K, bool kIota, int BITS, int ITEMS>
 __device__ __forceinline__ void scatter_tile(const Segs& segs, const K* __restrict__ kin,
                                              const uint32_t* __restrict__ vin, K* __restrict__ kout,
                                              uint32_t* __restrict__ vout, int shift, const uint32_t* __restrict__ hist,
                                              size_t hist_stride, const uint32_t* __restrict__ prefix,
                                              const uint32_t* __restrict__ chunk_carry) {
     using Plan = SortPlan<K, BITS>;
-    constexpr int D = Plan::kDigits, R = Plan::kPerThread;
+    constexpr int D = Plan::kDigits, R = Plan::kPerThread, kSortTile = kSortThreads * ITEMS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     K* s_keys = reinterpret_cast<K*>(smem_raw);
     uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + kSortTile);
@@ -491,21 +517,21 @@ __device__ __forceinline__ void scatter_tile(const Segs& segs, const K* __restri
     const uint32_t valid_n = min((uint32_t)kSortTile, seg_end - base);
     const uint32_t end = base + valid_n;
 
-    K key[kSortItems];
-    uint32_t val[kSortItems];
-    uint32_t rank[kSortItems];
+    K key[ITEMS];
+    uint32_t val[ITEMS];
+    uint32_t rank[ITEMS];
     const uint32_t lt = lanemask_lt();
     uint32_t* const wh = s_wh + w * D;
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const uint32_t idx = base + (uint32_t)w * (kSortItems * 32) + r * 32 + lane;
+    for (int r = 0; r < ITEMS; ++r) {
+        const uint32_t idx = base + (uint32_t)w * (ITEMS * 32) + r * 32 + lane;
         const bool valid = idx < end;
         key[r] = valid ? kin[idx] : (K)0;
         val[r] = kIota ? (uint32_t)idx : (valid ? vin[idx] : 0u);
     }
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const bool valid = base + (uint32_t)w * (kSortItems * 32) + r * 32 + lane < end;
+    for (int r = 0; r < ITEMS; ++r) {
+        const bool valid = base + (uint32_t)w * (ITEMS * 32) + r * 32 + lane < end;
         const uint32_t d = valid ? (uint32_t)((key[r] >> shift) & (D - 1)) : (uint32_t)D;
         const uint32_t peers = __match_any_sync(kFull, d);
         const uint32_t before = __popc(peers & lt);
@@ -547,7 +573,7 @@ __device__ __forceinline__ void scatter_tile(const Segs& segs, const K* __restri
 
     // Scatter into shared memory in digit order, then write out coalesced.
 #pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         if (rank[r] == 0xffffffffu) continue;
         const uint32_t dd = (uint32_t)((key[r] >> shift) & (D - 1));
         const uint32_t p = s_dstart[dd] + wh[dd] + rank[r];
@@ -566,18 +592,19 @@ __device__ __forceinline__ void scatter_tile(const Segs& segs, const K* __restri
     }
 }
 
-template <typename K, bool kIota, int BITS>
+template <typename K, bool kIota, int BITS, int ITEMS>
 __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 ? 4 : 3) k_scatter(
         Segs segs, const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
         uint32_t* __restrict__ vout, int pass, const uint32_t* __restrict__ hist,
         const uint32_t* __restrict__ prefix, const uint32_t* __restrict__ chunk_carry) {
     constexpr int P = SortPlan<K, BITS>::kPasses, D = SortPlan<K, BITS>::kDigits;
-    scatter_tile<K, kIota, BITS>(segs, kin, vin, kout, vout, BITS * pass, hist + pass * D, (size_t)P * D, prefix,
+    scatter_tile<K, kIota, BITS, ITEMS>(segs, kin, vin, kout, vout, BITS * pass, hist + pass * D, (size_t)P * D, prefix,
                                  chunk_carry);
 }
 
 // A word pass: from one pair of buffers to the other, by the number of passes
 // that ran before it.
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads, 4) k_word_scatter(Segs segs, WordPass wp, uint32_t* keys_a,
                                                                   uint32_t* keys_b, uint32_t* perm_a, uint32_t* perm_b,
                                                                   const uint32_t* __restrict__ total,
@@ -585,8 +612,120 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_word_scatter(Segs segs, Wor
     const uint32_t active = active_digits(wp.diff);
     if (!((active >> wp.digit) & 1u)) return;
     const bool odd = __popc(active & ((1u << wp.digit) - 1u)) & 1;
-    scatter_tile<uint32_t, false, 8>(segs, odd ? keys_b : keys_a, odd ? perm_b : perm_a, odd ? keys_a : keys_b,
+    scatter_tile<uint32_t, false, 8, ITEMS>(segs, odd ? keys_b : keys_a, odd ? perm_b : perm_a, odd ? keys_a : keys_b,
                                      odd ? perm_a : perm_b, 8 * (wp.digit & 3), total, 0, prefix, nullptr);
+}
+
+// ---- meshes of one sort tile ------------------------------------------------------
+// Where every mesh fits one tile (at most kSortTile triangles), a block sorts a
+// whole mesh: codes into registers, then every pass within the block -- rank,
+// scan, through shared memory in digit order, back into registers -- and one
+// write of keys and order.  One launch in place of the codes' and three per
+// digit, whose latency is all that such meshes cost (1,003 triangles: codes and
+// sort 54 -> @@ us).  Ranks as scatter_tile does, so equal keys keep their order.
+constexpr int kTileThreads = 512;
+constexpr int kTileItems = kSortTile / kTileThreads;
+constexpr int kTileWarps = kTileThreads / 32;
+
+template <typename K>
+__global__ void __launch_bounds__(kTileThreads) k_sort_tile(Segs segs, const float4* __restrict__ v,
+                                                             const float* __restrict__ bounds, PrimBoxes pr,
+                                                             K* __restrict__ keys, uint32_t* __restrict__ idx) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    K* const s_keys = reinterpret_cast<K*>(smem_raw);
+    uint32_t* const s_vals = reinterpret_cast<uint32_t*>(s_keys + kSortTile);
+    uint32_t* const s_wh = s_vals + kSortTile;  // [kTileWarps][256] per-warp digit counters
+    __shared__ uint32_t s_start[256], s_scan[8];
+    __shared__ float sb[6];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const uint32_t m = blockIdx.x;
+    const uint32_t base = segs.tri_begin(m), n = segs.tri_end(m) - base;
+    if (tid < 6) sb[tid] = bounds[6 * m + tid];
+    __syncthreads();
+    const uint32_t lt = lanemask_lt();
+    uint32_t* const wh = s_wh + w * 256;
+    const uint32_t first = (uint32_t)w * (kTileItems * 32) + lane;  // this lane's items: first + 32 r
+    K key[kTileItems];
+    uint32_t val[kTileItems];
+#pragma unroll
+    for (int r = 0; r < kTileItems; ++r) {
+        const uint32_t i = first + 32 * r;
+        val[r] = base + i;
+        key[r] = i < n ? prim_code<K>(v, pr, base + i, sb) : (K)0;
+    }
+    for (int shift = 0; shift < (sizeof(K) == 4 ? 32 : 64); shift += 8) {
+        for (int j = tid; j < kTileWarps * 256; j += kTileThreads) s_wh[j] = 0;
+        __syncthreads();
+        uint32_t rank[kTileItems];
+#pragma unroll
+        for (int r = 0; r < kTileItems; ++r) {
+            const bool valid = first + 32 * r < n;
+            const uint32_t d = valid ? (uint32_t)((key[r] >> shift) & 255u) : 256u;
+            const uint32_t peers = __match_any_sync(kFull, d);
+            const uint32_t before = __popc(peers & lt);
+            uint32_t cnt = 0;
+            if (valid) cnt = wh[d];
+            __syncwarp();
+            if (valid && before == 0) wh[d] = cnt + __popc(peers);
+            __syncwarp();
+            rank[r] = cnt + before;
+        }
+        __syncthreads();
+        // Digit starts: offsets across the warps, then over the digits.
+        uint32_t total = 0;
+        if (tid < 256) {
+#pragma unroll
+            for (int j = 0; j < kTileWarps; ++j) {
+                const uint32_t c = s_wh[j * 256 + tid];
+                s_wh[j * 256 + tid] = total;
+                total += c;
+            }
+        }
+        uint32_t inc = total;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (tid < 256 && lane == 31) s_scan[w] = inc;
+        __syncthreads();
+        if (tid < 256) {
+            uint32_t run = inc - total;
+            for (int j = 0; j < w; ++j) run += s_scan[j];
+            s_start[tid] = run;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kTileItems; ++r)
+            if (first + 32 * r < n) {
+                const uint32_t d = (uint32_t)((key[r] >> shift) & 255u);
+                const uint32_t p = s_start[d] + wh[d] + rank[r];
+                s_keys[p] = key[r];
+                s_vals[p] = val[r];
+            }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kTileItems; ++r) {
+            const uint32_t i = first + 32 * r;
+            if (i < n) {
+                key[r] = s_keys[i];
+                val[r] = s_vals[i];
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < kTileItems; ++r) {
+        const uint32_t i = first + 32 * r;
+        if (i < n) {
+            keys[base + i] = key[r];
+            idx[base + i] = val[r];
+        }
+    }
+}
+template <typename K>
+constexpr size_t tile_smem() {
+    return (size_t)kSortTile * (sizeof(K) + 4) + (size_t)kTileWarps * 256 * 4;
 }
 
 // ---- fused Karras build + refit ------------------------------------------------
@@ -924,7 +1063,7 @@ int grid_for(atr_ctx* ctx, uint64_t work, int per_sm_blocks, int threads) {
 // k_morton; tiles x D) and is consumed.  With iota the first pass generates
 // the values (global element indices).
 template <typename K, int BITS>
-int sort_pairs(atr_ctx* ctx, const Segs& segs, uint32_t tiles, K** keys, uint32_t** vals, uint32_t* hist,
+int sort_pairs(atr_ctx* ctx, const Segs& segs, uint32_t tiles, int items, K** keys, uint32_t** vals, uint32_t* hist,
                bool hist_ready, bool iota, bool owned, uint32_t* tile_counts0 = nullptr) {
     using Plan = SortPlan<K, BITS>;
     constexpr int P = Plan::kPasses, D = Plan::kDigits;
@@ -964,7 +1103,9 @@ int sort_pairs(atr_ctx* ctx, const Segs& segs, uint32_t tiles, K** keys, uint32_
     const uint32_t* const carry = chunks > kFoldChunks ? chunk_tot : nullptr;
     for (int pass = 0; pass < P && e == cudaSuccess; ++pass) {
         if (pass > 0 || !tile_counts0) {
-            k_tile_counts<K, BITS><<<tiles, kSortThreads, 0, s>>>(segs, ka, pass, counts);
+            with_items(items, [&](auto I) {
+                k_tile_counts<K, BITS, I.value><<<tiles, kSortThreads, 0, s>>>(segs, ka, pass, counts);
+            });
             ctx->launches += 1;
         }
         if (chunks <= kFoldChunks)
@@ -976,12 +1117,15 @@ int sort_pairs(atr_ctx* ctx, const Segs& segs, uint32_t tiles, K** keys, uint32_
             k_chunk_carry<D><<<(D + 255) / 256, 256, 0, s>>>(chunks, chunk_tot);
             ctx->launches += 1;
         }
-        if (pass == 0 && iota)
-            k_scatter<K, true, BITS><<<tiles, kSortThreads, Plan::kSmem, s>>>(segs, ka, va, kb2, vb2, pass, hist,
-                                                                              counts, carry);
-        else
-            k_scatter<K, false, BITS><<<tiles, kSortThreads, Plan::kSmem, s>>>(segs, ka, va, kb2, vb2, pass, hist,
-                                                                               counts, carry);
+        with_items(items, [&](auto I) {
+            const size_t smem = Plan::smem(I.value);
+            if (pass == 0 && iota)
+                k_scatter<K, true, BITS, I.value>
+                    <<<tiles, kSortThreads, smem, s>>>(segs, ka, va, kb2, vb2, pass, hist, counts, carry);
+            else
+                k_scatter<K, false, BITS, I.value>
+                    <<<tiles, kSortThreads, smem, s>>>(segs, ka, va, kb2, vb2, pass, hist, counts, carry);
+        });
         ctx->launches += 2;
         std::swap(ka, kb2);
         std::swap(va, vb2);
@@ -1003,7 +1147,7 @@ int sort_pairs(atr_ctx* ctx, const Segs& segs, uint32_t tiles, K** keys, uint32_
 }
 
 template <typename K, int BITS>
-int build_typed(atr_ctx* ctx, const Segs& segs, uint32_t tiles, const float4* verts, const float* d_bounds,
+int build_typed(atr_ctx* ctx, const Segs& segs, uint32_t mesh_tiles, const float4* verts, const float* d_bounds,
                 const TreeOut& t, void** keep_keys, uint32_t** keep_idx, const BuildPrepass* prepass,
                 const PrimBoxes& pr) {
     constexpr int P = SortPlan<K, BITS>::kPasses, D = SortPlan<K, BITS>::kDigits;
@@ -1012,8 +1156,14 @@ int build_typed(atr_ctx* ctx, const Segs& segs, uint32_t tiles, const float4* ve
     void* kv = nullptr;
     void* iv = nullptr;
     void* aux = nullptr;
-    const size_t hbytes = (size_t)segs.count * P * D * 4;
-    const size_t cbytes = (size_t)tiles * D * 4;
+    const bool one_tile = mesh_tiles == segs.count;  // every mesh fits a sort tile of a batch
+    // A batch's tiles are the caller's; a single mesh is cut to the GPU's size.
+    const int items = segs.count == 1 ? sort_items(segs.n) : kSortItems;
+    const uint32_t tiles = segs.count == 1 && !one_tile
+                               ? (segs.n + (uint32_t)(kSortThreads * items) - 1) / (uint32_t)(kSortThreads * items)
+                               : mesh_tiles;
+    const size_t hbytes = one_tile ? 0 : (size_t)segs.count * P * D * 4;
+    const size_t cbytes = one_tile ? 0 : (size_t)tiles * D * 4;
     const size_t inner = n - segs.count;
     ATR_TRY(ctx->alloc(&kv, (size_t)n * sizeof(K)));
     int st = ctx->alloc(&iv, (size_t)n * 4);
@@ -1029,19 +1179,25 @@ int build_typed(atr_ctx* ctx, const Segs& segs, uint32_t tiles, const float4* ve
     uint32_t* tile_counts = reinterpret_cast<uint32_t*>(ap); ap += align256(cbytes);
     int32_t* slot = reinterpret_cast<int32_t*>(ap); ap += align256(inner * 4);
     BuildEdge* edges = reinterpret_cast<BuildEdge*>(ap);
-    const int zs = zero_words_async(ctx, hist, hbytes / 4);
-    if (zs != ATR_OK) {
-        ctx->release(aux); ctx->release(kv); ctx->release(iv);
-        return zs;
+    if (one_tile) {
+        ctx->phase_begin("sort");
+        k_sort_tile<K><<<tiles, kTileThreads, tile_smem<K>(), s>>>(segs, verts, d_bounds, pr, keys, idx);
+        ctx->phase_end();
+        ctx->launches += 1;
+    } else {
+        st = zero_words_async(ctx, hist, hbytes / 4);
+        if (st == ATR_OK) {
+            ctx->phase_begin("morton");
+            with_items(items, [&](auto I) {
+                k_morton<K, BITS, I.value><<<tiles, 256, 0, s>>>(segs, verts, d_bounds, keys, hist, tile_counts, pr);
+            });
+            ctx->phase_end();
+            ctx->launches += 1;
+            ctx->phase_begin("sort");
+            st = sort_pairs<K, BITS>(ctx, segs, tiles, items, &keys, &idx, hist, true, true, true, tile_counts);
+            ctx->phase_end();
+        }
     }
-
-    ctx->phase_begin("morton");
-    k_morton<K, BITS><<<tiles, 256, 0, s>>>(segs, verts, d_bounds, keys, hist, tile_counts, pr);
-    ctx->phase_end();
-    ctx->launches += 1;
-    ctx->phase_begin("sort");
-    st = sort_pairs<K, BITS>(ctx, segs, tiles, &keys, &idx, hist, true, true, true, tile_counts);
-    ctx->phase_end();
     if (st == ATR_OK) {
         ctx->phase_begin("build");
         const BuildOut<K> o{t.parent, t.left,  t.right, t.data,
@@ -1067,10 +1223,18 @@ static_assert(kSortTile == (int)kSortTileSize, "sort tile size");
 
 template <typename K, int BITS>
 cudaError_t scatter_attrs() {
-    const int smem = (int)SortPlan<K, BITS>::kSmem;
-    cudaError_t e = cudaFuncSetAttribute(k_scatter<K, true, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_scatter<K, false, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    auto of = [](auto I) {
+        const int smem = (int)SortPlan<K, BITS>::smem(I.value);
+        cudaError_t e = cudaFuncSetAttribute(k_scatter<K, true, BITS, I.value>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_scatter<K, false, BITS, I.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     smem);
+        return e;
+    };
+    cudaError_t e = with_items(3, of);
+    if (e == cudaSuccess) e = with_items(6, of);
+    if (e == cudaSuccess) e = with_items(kSortItems, of);
     return e;
 }
 
@@ -1080,8 +1244,15 @@ int lbvh_prepare() {
     ATR_CUDA((scatter_attrs<uint32_t, 10>()));
     ATR_CUDA((scatter_attrs<uint64_t, 8>()));
     ATR_CUDA((scatter_attrs<uint64_t, 10>()));
-    ATR_CUDA(cudaFuncSetAttribute(k_word_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)SortPlan<uint32_t, 8>::kSmem));
+    ATR_CUDA(cudaFuncSetAttribute(k_sort_tile<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)tile_smem<uint32_t>()));
+    ATR_CUDA(cudaFuncSetAttribute(k_sort_tile<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)tile_smem<uint64_t>()));
+    for (int items : {3, 6, kSortItems})
+        ATR_CUDA(with_items(items, [](auto I) {
+            return cudaFuncSetAttribute(k_word_scatter<I.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)SortPlan<uint32_t, 8>::smem(I.value));
+        }));
     return ATR_OK;
 }
 
@@ -1137,7 +1308,8 @@ int sort_ray_words(atr_ctx* ctx, const uint32_t* words, const uint32_t* diff, ui
                    uint32_t* keys_b, uint32_t* perm_a, uint32_t* perm_b) {
     using Plan = SortPlan<uint32_t, 8>;
     const Segs segs{nullptr, nullptr, 1u, n};
-    const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
+    const int items = sort_items(n);
+    const uint32_t tile = (uint32_t)(kSortThreads * items), tiles = (n + tile - 1) / tile;
     void* tmp = nullptr;
     const size_t cbytes = align256((size_t)tiles * 256 * 4);
     ATR_TRY(ctx->alloc(&tmp, cbytes + 256 * 4));
@@ -1146,10 +1318,12 @@ int sort_ray_words(atr_ctx* ctx, const uint32_t* words, const uint32_t* diff, ui
     cudaStream_t s = ctx->stream;
     for (int digit = 0; digit < 24; ++digit) {
         const WordPass wp{diff, words, digit};
-        k_word_counts<<<tiles, kSortThreads, 0, s>>>(n, wp, keys_a, keys_b, perm_a, perm_b, counts);
-        k_tile_prefix<256, true><<<8, 32 * kPrefixRuns, 0, s>>>(segs, tiles, counts, total, wp);
-        k_word_scatter<<<tiles, kSortThreads, Plan::kSmem, s>>>(segs, wp, keys_a, keys_b, perm_a, perm_b, total,
-                                                                counts);
+        with_items(items, [&](auto I) {
+            k_word_counts<I.value><<<tiles, kSortThreads, 0, s>>>(n, wp, keys_a, keys_b, perm_a, perm_b, counts);
+            k_tile_prefix<256, true><<<8, 32 * kPrefixRuns, 0, s>>>(segs, tiles, counts, total, wp);
+            k_word_scatter<I.value><<<tiles, kSortThreads, Plan::smem(I.value), s>>>(segs, wp, keys_a, keys_b, perm_a,
+                                                                                    perm_b, total, counts);
+        });
     }
     ctx->launches += 72;
     ctx->release(tmp);
@@ -1314,11 +1488,11 @@ int atr_device_morton(atr_ctx* ctx, const float* vertices, uint32_t n, const flo
     Segs segs{nullptr, nullptr, 1u, n};
     const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
     if (morton_bits == 30)
-        k_morton<uint32_t, 8><<<tiles, 256, 0, ctx->stream>>>(segs, v, static_cast<float*>(b),
+        k_morton<uint32_t, 8, kSortItems><<<tiles, 256, 0, ctx->stream>>>(segs, v, static_cast<float*>(b),
                                                               static_cast<uint32_t*>(keys), nullptr, nullptr,
                                                               PrimBoxes{});
     else
-        k_morton<uint64_t, 8><<<tiles, 256, 0, ctx->stream>>>(segs, v, static_cast<float*>(b),
+        k_morton<uint64_t, 8, kSortItems><<<tiles, 256, 0, ctx->stream>>>(segs, v, static_cast<float*>(b),
                                                               static_cast<uint64_t*>(keys), nullptr, nullptr,
                                                               PrimBoxes{});
     ctx->launches += 1;
@@ -1333,13 +1507,14 @@ int atr_device_sort_pairs(atr_ctx* ctx, void* keys, uint32_t* values, uint32_t c
     ATR_REQUIRE(count < (1u << 30), ATR_ERR_INVALID_ARG, "atr_device_sort_pairs: count %u >= 2^30", count);
     if (count == 0) return ATR_OK;
     Segs segs{nullptr, nullptr, 1u, count};
-    const uint32_t tiles = (count + kSortTile - 1) / kSortTile;
+    const int items = sort_items(count);
+    const uint32_t tile = (uint32_t)(kSortThreads * items), tiles = (count + tile - 1) / tile;
     if (key_bits <= 32) {
         uint32_t* k = static_cast<uint32_t*>(keys);
-        return sort_pairs<uint32_t, 8>(ctx, segs, tiles, &k, &values, nullptr, false, false, false);
+        return sort_pairs<uint32_t, 8>(ctx, segs, tiles, items, &k, &values, nullptr, false, false, false);
     }
     uint64_t* k = static_cast<uint64_t*>(keys);
-    return sort_pairs<uint64_t, 8>(ctx, segs, tiles, &k, &values, nullptr, false, false, false);
+    return sort_pairs<uint64_t, 8>(ctx, segs, tiles, items, &k, &values, nullptr, false, false, false);
 }
 
 }  // extern "C"
