@@ -17,6 +17,8 @@
 // number of leaves in right subtrees hanging off its path below the emitted
 // node.
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -45,6 +47,8 @@ struct CollapseRefs {
     // Per node: (SAH cost bits, triangle count << 1 | pass flag), one 8-byte
     // record so a climbing thread reads each child with one load.
     int2* rec;
+    // Per inner node: triangles of the leaf list it emits (0: none; a list has at
+    // least two triangles, so triangle leaves need no entry).
     uint32_t* emit_cnt;
     // False when the collapsed tree shares the source tree's links and boxes
     // (a collapse leaves them as they are): only data and counts are written.
@@ -68,14 +72,15 @@ __device__ __forceinline__ unsigned long long pack_rec(int2 v) {
 
 __global__ void __launch_bounds__(256) k_collapse_cost(CollapseRefs g, Segs segs,
                                                         unsigned long long* __restrict__ slots, float ci, float ct,
-                                                        int max_leaf) {
+                                                        int max_leaf, float* __restrict__ sah_parts) {
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     if (gi >= segs.n) return;
     const uint32_t m = segs.seg_of_tri(gi);
     const uint32_t s0 = segs.tri_begin(m);
     const uint32_t n = segs.tri_end(m) - s0;
     const int nb = segs.node_base(m);
-    unsigned long long* const slot = slots + segs.inner_base(m);
+    const int cb = segs.inner_base(m);
+    unsigned long long* const slot = slots + cb;
     int ch = (int)(gi - s0) + (int)n - 1;
     int cur = g.parent[nb + ch];
     int2 mine = make_int2(__float_as_int(__fmul_rn(ct, g.area[nb + ch])), (1 << 1) | 1);
@@ -130,13 +135,19 @@ __global__ void __launch_bounds__(256) k_collapse_cost(CollapseRefs g, Segs segs
         const bool reached = pl && pr;
         const int x = nb + cur;
         if (reached && !col) {
-            if (cl > 1) g.emit_cnt[nb + l] = (uint32_t)cl;
-            if (cr > 1) g.emit_cnt[nb + r] = (uint32_t)cr;
+            if (cl > 1) g.emit_cnt[cb + l] = (uint32_t)cl;
+            if (cr > 1) g.emit_cnt[cb + r] = (uint32_t)cr;
         }
         mine = make_int2(__float_as_int(c), (cnt << 1) | (reached && col ? 1 : 0));
         g.c_count[x] = cnt;
         g.rec[x] = mine;
-        if (up < 0) return;
+        if (up < 0) {
+            if (sah_parts) {  // the root's cost and area
+                sah_parts[2 * m] = c;
+                sah_parts[2 * m + 1] = a;
+            }
+            return;
+        }
         ch = cur;
         cur = up;
         l = nl;
@@ -153,7 +164,7 @@ __global__ void __launch_bounds__(256) k_collapse_emit(CollapseRefs g, Segs segs
     const uint32_t m = segs.seg_of_tri(gi);
     const uint32_t s0 = segs.tri_begin(m);
     const uint32_t n = segs.tri_end(m) - s0;
-    const int nb = segs.node_base(m);
+    const int nb = segs.node_base(m), cb = segs.inner_base(m);
     const int leaf = (int)(gi - s0) + (int)n - 1;
     int ch = leaf, a = g.parent[nb + leaf], top = -1;
     uint32_t rank = 0;
@@ -163,19 +174,21 @@ __global__ void __launch_bounds__(256) k_collapse_emit(CollapseRefs g, Segs segs
         ch = a;
         a = g.parent[nb + a];
     }
-    if (top < 0 || g.emit_cnt[nb + top] == 0) return;
-    const uint32_t off = offsets[nb + top] - offsets[nb];  // local to the mesh's list slice
+    if (top < 0 || g.emit_cnt[cb + top] == 0) return;
+    const uint32_t off = offsets[cb + top] - offsets[cb];  // local to the mesh's list slice
     tri_indices[s0 + off + rank] = g.data[nb + leaf];
     if (rank == 0) g.c_data[nb + top] = (int32_t)off;
 }
 
-__global__ void k_sah_parts(Segs segs, const int2* __restrict__ rec, const float* __restrict__ area,
-                            float* __restrict__ out) {
-    const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= segs.count) return;
-    const int nb = segs.node_base(m);
-    out[2 * m] = __int_as_float(rec[nb].x);
-    out[2 * m + 1] = area[nb];
+// What the cost climb starts from: zeroed exchange slots and list counts, list
+// entries of -1.  One kernel: each memset node of a captured collapse left the
+// device idle for several microseconds (collapse of 1,003 triangles in all 28 ->
+// 20 us, of 4,194,304 284 -> 266).
+__global__ void __launch_bounds__(256) k_collapse_clear(uint4* __restrict__ zero, size_t quads, int* __restrict__ list,
+                                                        uint32_t n) {
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = t; i < quads; i += stride) zero[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (size_t i = t; i < n; i += stride) list[i] = -1;
 }
 
 }  // namespace
@@ -235,41 +248,32 @@ int collapse_segs(atr_ctx* ctx, const Segs& segs, size_t total_nodes, const Tree
     const uint32_t n = segs.n;
     const size_t nn = total_nodes;
     void* scratch = nullptr;
-    const size_t b4 = align256(nn * 4);
     const size_t inner = n - segs.count;
-    ATR_TRY(ctx->alloc(&scratch, align256(nn * 8) + 2 * b4 + align256(inner * 4)));
+    const size_t b8 = align256(inner * 8), b4 = align256(inner * 4);
+    ATR_TRY(ctx->alloc(&scratch, align256(nn * 8) + b8 + b4));
     char* p = static_cast<char*>(scratch);
     int2* rec = reinterpret_cast<int2*>(p); p += align256(nn * 8);
-    uint32_t* emit = reinterpret_cast<uint32_t*>(p); p += b4;
-    uint32_t* offs = reinterpret_cast<uint32_t*>(p); p += b4;
-    // The exchange slots (8 B per inner node, at most 4 B per node) are dead
-    // once the cost pass ends, before the scan writes the list offsets.
-    unsigned long long* slots = reinterpret_cast<unsigned long long*>(offs);
+    unsigned long long* slots = reinterpret_cast<unsigned long long*>(p); p += b8;
+    uint32_t* emit = reinterpret_cast<uint32_t*>(p);
+    // The slots are dead once the cost pass ends, before the scan writes the
+    // list offsets.
+    uint32_t* offs = reinterpret_cast<uint32_t*>(slots);
     cudaStream_t s = ctx->stream;
-    // The climb reads a zero slot as "no sibling yet": a failed clear must stop here.
-    cudaError_t me = cudaMemsetAsync(slots, 0, inner * 8, s);
-    if (me == cudaSuccess) me = cudaMemsetAsync(emit, 0, nn * 4, s);
-    if (me == cudaSuccess) me = cudaMemsetAsync(dst.tri_indices, 0xff, (size_t)n * 4, s);
-    if (me != cudaSuccess) {
-        ctx->release(scratch);
-        return cuda_fail(me, "collapse scratch clear", __FILE__, __LINE__);
-    }
+    const size_t quads = (b8 + b4) / 16;
+    const unsigned clear_blocks = (unsigned)std::min<size_t>((quads + 255) / 256, (size_t)ctx->num_sms * 16);
+    k_collapse_clear<<<clear_blocks, 256, 0, s>>>(reinterpret_cast<uint4*>(slots), quads, dst.tri_indices, n);
     const bool shared = dst.parent == src.parent && dst.left == src.left && dst.right == src.right &&
                         dst.bmin == src.bmin && dst.bmax == src.bmax;
     CollapseRefs r{n,        src.area,  src.parent, src.left,  src.right, src.data, src.bmin, src.bmax,
                    dst.parent, dst.left, dst.right, dst.data, dst.count, dst.bmin, dst.bmax, rec,
                    emit,     !shared};
     const unsigned blocks = (n + 255) / 256;
-    k_collapse_cost<<<blocks, 256, 0, s>>>(r, segs, slots, ci, ct, max_leaf);
-    ctx->launches += 1;
-    int st = exclusive_scan_u32(ctx, emit, offs, nn, nullptr);
+    k_collapse_cost<<<blocks, 256, 0, s>>>(r, segs, slots, ci, ct, max_leaf, d_sah_parts);
+    ctx->launches += 2;
+    int st = exclusive_scan_u32(ctx, emit, offs, inner, nullptr);
     if (st == ATR_OK) {
         k_collapse_emit<<<blocks, 256, 0, s>>>(r, segs, offs, dst.tri_indices);
         ctx->launches += 1;
-        if (d_sah_parts) {
-            k_sah_parts<<<(segs.count + 255) / 256, 256, 0, s>>>(segs, rec, src.area, d_sah_parts);
-            ctx->launches += 1;
-        }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) st = cuda_fail(e, "collapse kernels", __FILE__, __LINE__);
     }
@@ -307,7 +311,7 @@ int atr_collapse(atr_ctx* ctx, const atr_tree* tree, float ci, float ct, int max
     c->split = tree->split;
     if (st == ATR_OK && sah) {
         float h[2];
-        cudaError_t e = cudaMemcpyAsync(h, parts, 8, cudaMemcpyDeviceToHost, ctx->stream);
+        const cudaError_t e = cudaMemcpyAsync(h, parts, 8, cudaMemcpyDeviceToHost, ctx->stream);
         if (e != cudaSuccess) st = cuda_fail(e, "cudaMemcpyAsync(sah)", __FILE__, __LINE__);
         if (st == ATR_OK) st = atr_ctx_synchronize(ctx);
         if (st == ATR_OK) *sah = h[0] / h[1];

@@ -1,7 +1,8 @@
 // Exclusive prefix sum of uint32 values (reduce, scan the tile sums, scan the
 // tiles), used for deterministic output offsets.  Three short launches with no
 // inter-block waiting: every tile's sum is read once, scanned by one block,
-// and added back while the tiles are scanned.  Sums wrap modulo 2^32.
+// and added back while the tiles are scanned; up to 16,384 values take one
+// block and one launch.  Sums wrap modulo 2^32.
 
 #include "common.cuh"
 #include "internal.h"
@@ -129,9 +130,34 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t* __restric
     }
 }
 
+// Up to kScanOne values in one block, one launch in place of three.
+constexpr uint64_t kScanOne = (uint64_t)kSumThreads * kScanItems;
+__global__ void __launch_bounds__(kSumThreads) k_scan_one(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                          uint32_t n, uint32_t* __restrict__ total) {
+    __shared__ uint32_t s_warp[kSumThreads / 32];
+    const uint32_t base = threadIdx.x * kScanItems;
+    uint32_t v[kScanItems], sum = 0, tot;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        v[k] = base + k < n ? in[base + k] : 0u;
+        sum += v[k];
+    }
+    uint32_t run = block_exclusive<kSumThreads>(sum, s_warp, &tot);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        if (base + k < n) out[base + k] = run;
+        run += v[k];
+    }
+    if (total && threadIdx.x == 0) *total = tot;
+}
+
 __global__ void __launch_bounds__(256) k_zero_words(uint32_t* __restrict__ p, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        p[i] = 0u;
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    // Callers pass starts of allocations or of their 256-byte aligned parts.
+    uint4* const q = reinterpret_cast<uint4*>(p);
+    const size_t quads = (reinterpret_cast<uintptr_t>(p) & 15u) ? 0 : n / 4;
+    for (size_t i = t; i < quads; i += stride) q[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (size_t i = 4 * quads + t; i < n; i += stride) p[i] = 0u;
 }
 
 }  // namespace
@@ -142,7 +168,7 @@ __global__ void __launch_bounds__(256) k_zero_words(uint32_t* __restrict__ p, si
 // follows its neighbours without that hand-off.
 int zero_words_async(atr_ctx* ctx, uint32_t* p, size_t words) {
     if (words == 0) return ATR_OK;
-    const size_t want = (words + 255) / 256, cap = (size_t)ctx->num_sms * 8;
+    const size_t want = (words + 1023) / 1024, cap = (size_t)ctx->num_sms * 8;
     k_zero_words<<<(unsigned)(want < cap ? want : cap), 256, 0, ctx->stream>>>(p, words);
     ctx->launches += 1;
     const cudaError_t e = cudaGetLastError();
@@ -153,6 +179,13 @@ int zero_words_async(atr_ctx* ctx, uint32_t* p, size_t words) {
 // out may equal in: every thread reads its own values before it writes them.
 int exclusive_scan_u32(atr_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* d_total) {
     if (n == 0) return ATR_OK;
+    if (n <= kScanOne) {
+        k_scan_one<<<1, kSumThreads, 0, ctx->stream>>>(in, out, (uint32_t)n, d_total);
+        ctx->launches += 1;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return cuda_fail(e, "k_scan_one launch", __FILE__, __LINE__);
+        return ATR_OK;
+    }
     const uint64_t tiles = (n + kScanTile - 1) / kScanTile;
     ATR_REQUIRE(tiles <= (1ull << 31), ATR_ERR_INVALID_ARG, "exclusive_scan_u32: %llu values",
                 (unsigned long long)n);
