@@ -26,6 +26,14 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
     return ATR_ERR_CUDA;
 }
 
+int read_back(atr_ctx* ctx, void* dst, const void* src, size_t bytes, bool check) {
+    ATR_CUDA(cudaMemcpyAsync(ctx->h_stage, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    if (check) ATR_TRY(atr_ctx_synchronize(ctx));
+    else ATR_CUDA(cudaStreamSynchronize(ctx->stream));
+    std::memcpy(dst, ctx->h_stage, bytes);
+    return ATR_OK;
+}
+
 int tree_alloc(atr_ctx* ctx, uint32_t n, atr_tree** out) {
     const size_t nn = 2 * (size_t)n - 1;
     const size_t b4 = align256(nn * 4), b16 = align256(nn * 16), b8 = align256((size_t)(n - 1) * 8);
@@ -127,11 +135,14 @@ int atr_ctx_create(int device, void* stream, atr_ctx** out) {
     }
     e = cudaMalloc(&c->d_error, 128);
     if (e == cudaSuccess) e = cudaMemset(c->d_error, 0, 128);
+    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&c->h_stage), atr_ctx::kStage, cudaHostAllocDefault);
     if (e == cudaSuccess) c->d_trace = reinterpret_cast<unsigned long long*>(c->d_error + 16);
     if (e == cudaSuccess && atr::lbvh_prepare() != ATR_OK) e = cudaErrorInvalidValue;
     if (e == cudaSuccess && atr::atrbvh_prepare(c) != ATR_OK) e = cudaErrorInvalidValue;
     if (e == cudaSuccess && atr::trbvh_prepare(c) != ATR_OK) e = cudaErrorInvalidValue;
     if (e != cudaSuccess) {
+        cudaFree(c->d_error);
+        cudaFreeHost(c->h_stage);
         cudaMemPoolDestroy(c->pool);
         if (c->own_stream) cudaStreamDestroy(c->stream);
         delete c;
@@ -146,6 +157,7 @@ int atr_ctx_destroy(atr_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     for (auto& p : ctx->phases) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     cudaFree(ctx->d_error);
+    cudaFreeHost(ctx->h_stage);
     // Memory still allocated from the pool (objects the caller has not yet
     // destroyed) stays valid; the pool goes once the last of it is freed.
     cudaMemPoolDestroy(ctx->pool);
@@ -156,9 +168,11 @@ int atr_ctx_destroy(atr_ctx* ctx) {
 
 int atr_ctx_synchronize(atr_ctx* ctx) {
     ATR_REQUIRE(ctx, ATR_ERR_INVALID_ARG, "atr_ctx_synchronize: ctx is NULL");
+    // The error word lands in pinned memory behind the stream's work.
+    uint32_t* const word = reinterpret_cast<uint32_t*>(ctx->h_stage + atr_ctx::kStage - 16);
+    ATR_CUDA(cudaMemcpyAsync(word, ctx->d_error, sizeof(*word), cudaMemcpyDeviceToHost, ctx->stream));
     ATR_CUDA(cudaStreamSynchronize(ctx->stream));
-    uint32_t err = 0;
-    ATR_CUDA(cudaMemcpy(&err, ctx->d_error, sizeof(err), cudaMemcpyDeviceToHost));
+    const uint32_t err = *word;
     if (err) {
         cudaMemset(ctx->d_error, 0, sizeof(uint32_t));
         atr::set_error("device-side bounded wait gave up (error bits 0x%x)", err);

@@ -311,9 +311,7 @@ int atr_collapse(atr_ctx* ctx, const atr_tree* tree, float ci, float ct, int max
     c->split = tree->split;
     if (st == ATR_OK && sah) {
         float h[2];
-        const cudaError_t e = cudaMemcpyAsync(h, parts, 8, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e != cudaSuccess) st = cuda_fail(e, "cudaMemcpyAsync(sah)", __FILE__, __LINE__);
-        if (st == ATR_OK) st = atr_ctx_synchronize(ctx);
+        st = read_back(ctx, h, parts, sizeof(h), true);
         if (st == ATR_OK) *sah = h[0] / h[1];
     }
     ctx->release(parts);

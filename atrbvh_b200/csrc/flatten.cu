@@ -431,10 +431,8 @@ int atr_flatten_compact2(atr_ctx* ctx, const atr_collapsed* c, const atr_scene* 
     st = flatten_segs(ctx, segs, co, scene->verts, cp->nodes, cp->woop, cp->tri_index, sizes);
     ctx->phase_end();
     if (st == ATR_OK) {
-        int64_t h[3];
-        cudaError_t e = cudaMemcpyAsync(h, sizes, 24, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) st = cuda_fail(e, "flatten kernels", __FILE__, __LINE__);
+        int64_t h[3] = {0, 0, 0};
+        st = read_back(ctx, h, sizes, sizeof(h), false);
         cp->num_nodes = h[0];
         cp->num_woop = h[1];
         cp->max_depth = (int32_t)h[2];

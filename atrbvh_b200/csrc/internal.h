@@ -89,6 +89,10 @@ struct atr_ctx {
     // Traversal's ray counter and finished-warp counter, zero between launches
     // (in d_error's allocation).
     unsigned long long* d_trace = nullptr;
+    // Pinned words that small read-backs and the error word are copied to, so
+    // that one stream synchronisation covers them.
+    static constexpr size_t kStage = 256;
+    char* h_stage = nullptr;
     uint64_t launches = 0;        // kernels enqueued by this context
     bool timing = false;
     // Launch tuning (atr_ctx_set_tuning): ATRBVH warps per block (2, 4, 8);
@@ -210,6 +214,11 @@ struct atr_compact {
 };
 
 namespace atr {
+
+// Copies `bytes` (at most atr_ctx::kStage - 16) from the device to dst through the
+// pinned words: waits for the stream, and with `check` reports device-side
+// errors as atr_ctx_synchronize does.
+int read_back(atr_ctx* ctx, void* dst, const void* src, size_t bytes, bool check);
 
 struct Segs;       // common.cuh: meshes of a batch laid end to end
 struct TreeRefs;   // treelet.cuh

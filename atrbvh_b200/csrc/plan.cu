@@ -276,8 +276,7 @@ int atr_plan_compact(atr_ctx* ctx, atr_plan* P, const atr_compact** compact) {
     ATR_REQUIRE(P->ran, ATR_ERR_INVALID_ARG, "atr_plan_compact: the plan has not run");
     if (!P->sizes_read) {
         int64_t h[3];
-        ATR_CUDA(cudaMemcpyAsync(h, P->d_sizes, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-        ATR_TRY(atr_ctx_synchronize(ctx));
+        ATR_TRY(read_back(ctx, h, P->d_sizes, sizeof(h), true));
         P->cp->num_nodes = h[0];
         P->cp->num_woop = h[1];
         P->cp->max_depth = (int32_t)h[2];
@@ -291,8 +290,7 @@ int atr_plan_sah(atr_ctx* ctx, atr_plan* P, float* sah) {
     ATR_REQUIRE(ctx && P && sah, ATR_ERR_INVALID_ARG, "atr_plan_sah: NULL argument");
     ATR_REQUIRE(P->ran, ATR_ERR_INVALID_ARG, "atr_plan_sah: the plan has not run");
     float h[2];
-    ATR_CUDA(cudaMemcpyAsync(h, P->d_sah, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    ATR_TRY(atr_ctx_synchronize(ctx));
+    ATR_TRY(read_back(ctx, h, P->d_sah, sizeof(h), true));
     *sah = h[0] / h[1];
     return ATR_OK;
 }
