@@ -892,13 +892,24 @@ struct QuadLayout {
 };
 constexpr int kQuadLeaves = 10;  // largest treelet the quad path takes
 
-template <int KL>
+// TS > 0: every treelet has TS leaves, a constant, and the searches are unrolled,
+// so a lane's reads of areas and distances are in flight together.  The passes
+// are bound by shared-memory wavefronts (71 % of peak on the first level of
+// 4,194,304 triangles), their latency and issue: ATRBVH(9, 2) of 4,194,304
+// triangles 1,889 -> 1,819 us, of 16,777,216 5,464 -> 5,253 against TS = 0.
+// Measured and not kept: the merge steps unrolled too (5,535 at 16,777,216:
+// instruction fetch), the groups' slots interleaved over the banks (5,750 and
+// more: lanes of a group then share four banks), distances read ahead of their
+// comparisons (the same).
+template <int KL, int TS>
 __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int nb, uint32_t n, int root,
-                                             int4 rk, int4* KD, const NextRefs& nx, float root_sah, int tsize,
-                                             int maxts,
+                                             int4 rk, int4* KD, const NextRefs& nx, float root_sah, int tsize_v,
+                                             int maxts_v,
                                              float ci, float* sm, const uint16_t* __restrict__ s_rc,
                                              const uint8_t* __restrict__ s_prio, uint32_t* err) {
     using Lay = QuadLayout<KL>;
+    constexpr int kUnroll = TS > 0 ? 16 : 1;
+    const int tsize = TS > 0 ? TS : tsize_v, maxts = TS > 0 ? TS : maxts_v;
     const int lane = threadIdx.x & 31;
     const int gb = lane & ~3;
     const int gl = lane & 3;
@@ -935,6 +946,7 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
     }
     __syncwarp();
     bool ok = true;
+#pragma unroll kUnroll
     for (int it = 0; it < maxts - 2; ++it) {
         const bool act = active && ok && it < tsize - 2;
         const int m = 2 + it;
@@ -942,7 +954,10 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
         // lowest rank of the reference's reduction tree over m lanes.
         float bv = -FLT_MAX;
         int bk = gl < m ? gl : 0, brk = 255;
-        for (int k = gl; k < m; k += 4) {
+#pragma unroll kUnroll
+        for (int u = 0; u < (m + 3) / 4; ++u) {
+            const int k = gl + 4 * u;
+            if (k >= m) break;
             const float v = is_internal(__float_as_int(lmx[k].w), n) ? lmn[k].w : -FLT_MAX;
             const int rk = s_prio[m * 32 + k];
             if (brk == 255 || v > bv || (v == bv && rk < brk)) {
@@ -1033,7 +1048,10 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
     __syncwarp();
     if (run) {
         const int np = tsize * (tsize - 1) / 2;
-        for (int j = gl; j < np; j += 4) {
+#pragma unroll kUnroll
+        for (int u = 0; u < (np + 3) / 4; ++u) {
+            const int j = gl + 4 * u;
+            if (j >= np) break;
             const uint32_t rc = s_rc[j];
             const float4 a0 = lmn[rc >> 8], a1 = lmx[rc >> 8], b0 = lmn[rc & 255u], b1 = lmx[rc & 255u];
             dist[j] = union_area3(a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, b0.x, b0.y, b0.z, b1.x, b1.y, b1.z);
@@ -1045,13 +1063,16 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
     for (int step = 0; step < maxts - 1; ++step) {
         const int last = tsize - 1 - step;
         const bool act = run && last >= 1;
-        const int msize = act ? last * (last + 1) / 2 : 0;
+        const int msize = TS > 0 ? last * (last + 1) / 2 : act ? last * (last + 1) / 2 : 0;
         // findMinimumDistance as in process_group: distances alone unless the
         // group minimum is held twice; then the exact key.
         uint32_t bd = 0xffffffffu;
         int bj = 0;
         bool tie = false;
-        for (int j = gl; j < msize; j += 4) {
+#pragma unroll kUnroll
+        for (int u = 0; u < (msize + 3) / 4; ++u) {
+            const int j = gl + 4 * u;
+            if (j >= msize) break;
             uint32_t d = __float_as_uint(dist[j]);
             d = d < 0x7f7fffffu ? d : 0xffffffffu;
             if (d < bd) {
@@ -1061,6 +1082,10 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
             } else if (d == bd) {
                 tie = true;
             }
+        }
+        if (TS > 0 && !act) {  // the matrix of a group without a treelet holds nothing
+            bd = 0xffffffffu;
+            tie = false;
         }
         uint32_t dmin = min(bd, __shfl_xor_sync(kFull, bd, 1));
         dmin = min(dmin, __shfl_xor_sync(kFull, dmin, 2));
@@ -1139,6 +1164,7 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             const int c = gl + 4 * q;
+            if (TS > 0 && 4 * q >= last) break;
             if (du && c < last && c != jr) mv[q] = dist[trm_idx(last, c)];
         }
         __syncwarp();
@@ -1151,12 +1177,14 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             const int c = gl + 4 * q;
+            if (TS > 0 && 4 * q >= last) break;
             if (du && c < last && c != jr) dist[trm_idx(max(jr, c), min(jr, c))] = mv[q];
         }
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             const int c = gl + 4 * q;
+            if (TS > 0 && 4 * q >= last) break;
             if (du && c < last && c != jc) {
                 const float4 b0 = lmn[c], b1 = lmx[c];
                 dist[trm_idx(max(jc, c), min(jc, c))] =
@@ -1227,7 +1255,7 @@ __device__ __forceinline__ void process_quad(const TreeRefs& g, bool active, int
 
 // The treelets of the calling warp's lane groups (QUADS: of four lanes, else of
 // G): `has` and the root `q` are a group's own, `leader` is one lane of it.
-template <int G, bool QUADS>
+template <int G, bool QUADS, int TS = 0>
 __device__ __forceinline__ void restructure_roots(const TreeRefs& g, const Segs& segs, const LevelRefs& lv, bool has,
                                                   uint2 q, bool leader, int tsize_all,
                                                   const uint8_t* __restrict__ seg_tsize, int iteration, float ci,
@@ -1255,14 +1283,14 @@ __device__ __forceinline__ void restructure_roots(const TreeRefs& g, const Segs&
     __syncwarp();
     const NextRefs nx{lv.rec + nb, lv.par, tsize << (iteration + 1), lv.ct};
     if constexpr (QUADS)
-        process_quad<kQuadLeaves>(g, has, nb, n, x, rk, kd, nx, root_sah, tsize, maxts, ci, sm, s_rc, s_prio, err);
+        process_quad<kQuadLeaves, TS>(g, has, nb, n, x, rk, kd, nx, root_sah, tsize, maxts, ci, sm, s_rc, s_prio, err);
     else
         process_group<G>(g, has, nb, n, x, rk, kd, nx, root_sah, tsize, maxts, ci, sm, s_rc, s_prio, err);
 }
 
 // Phase C: every treelet root of level `lev`.  Each warp takes `per` roots
 // at a time: 32/G in lane groups of G, or (QUADS) eight in four-lane groups.
-template <int G, int W, bool QUADS>
+template <int G, int W, bool QUADS, int TS = 0>
 __global__ void __launch_bounds__(W * 32, (G == 32 ? 16 : 32) / W) k_level_groups(TreeRefs g, Segs segs, LevelRefs lv, int lev,
                                                                  int tsize_all, const uint8_t* __restrict__ seg_tsize,
                                                                  int iteration, float ci, uint32_t* err) {
@@ -1290,7 +1318,7 @@ __global__ void __launch_bounds__(W * 32, (G == 32 ? 16 : 32) / W) k_level_group
         const uint32_t e = e0 + (uint32_t)grp;
         const bool has = grp < per && e < end;
         float* const sm = &s_mem[w][0] + (grp < per ? grp : per - 1) * kGroupFloats;
-        restructure_roots<G, QUADS>(g, segs, lv, has, has ? lv.order[e] : make_uint2(0u, 0u), lane == grp * gw,
+        restructure_roots<G, QUADS, TS>(g, segs, lv, has, has ? lv.order[e] : make_uint2(0u, 0u), lane == grp * gw,
                                     tsize_all, seg_tsize, iteration, ci, sm, s_rc, s_prio, err);
     }
 }
@@ -1440,7 +1468,14 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
                 const bool quads = max_ts <= kQuadLeaves && ctx->atr_quad_min >= 0 && expect >= ctx->atr_quad_min;
                 const bool whole = !quads && max_ts <= kRegTreelet && expect <= (double)ctx->atr_warp_max;
                 if (quads) {
-                    launch_level_g<8, true>(warps, lg, st, g, segs, lv, lev, tsize, seg_tsize, it, ci, ctx->d_error);
+                    // Sizes of the autotuner's range that have a kernel of their own.
+                    const int ts = seg_tsize || warps != 8 ? 0 : tsize;
+                    switch (ts) {
+                        case 5: k_level_groups<8, 8, true, 5><<<lg, 256, 0, st>>>(g, segs, lv, lev, tsize, nullptr, it, ci, ctx->d_error); break;
+                        case 7: k_level_groups<8, 8, true, 7><<<lg, 256, 0, st>>>(g, segs, lv, lev, tsize, nullptr, it, ci, ctx->d_error); break;
+                        case 9: k_level_groups<8, 8, true, 9><<<lg, 256, 0, st>>>(g, segs, lv, lev, tsize, nullptr, it, ci, ctx->d_error); break;
+                        default: launch_level_g<8, true>(warps, lg, st, g, segs, lv, lev, tsize, seg_tsize, it, ci, ctx->d_error); break;
+                    }
                 } else if (whole) {
                     launch_level_g<32, false>(warps, lg, st, g, segs, lv, lev, tsize, seg_tsize, it, ci, ctx->d_error);
                 } else {
