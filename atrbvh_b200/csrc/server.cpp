@@ -93,6 +93,8 @@ struct Lane {
     size_t h_res_cap = 0;
     void* h_rverts = nullptr;  // refit vertices
     size_t h_rverts_cap = 0;
+    void* h_late = nullptr;  // vertices, rays and results of refits that join a batch
+    size_t h_late_cap = 0;
 };
 
 struct CopyJob {
@@ -310,7 +312,38 @@ struct atr_server {
         return out;
     }
 
+    // Waiting refits of the meshes that `lane` has just built in `builds` (kept
+    // resident, no other build of them in flight), with the mesh's index: they
+    // join the batch that built them.  Takes the lock.
+    std::vector<Request*> join_refits(int lane, const std::vector<Request*>& builds, size_t taken) {
+        std::vector<Request*> out;
+        std::lock_guard<std::mutex> lock(mu);
+        for (auto it = pending.begin(); it != pending.end();) {
+            Request* r = *it;
+            size_t m = builds.size();
+            if (r->req.kind == ATR_REQ_REFIT)
+                for (m = 0; m < builds.size(); ++m)
+                    if (builds[m]->req.mesh_id == r->req.mesh_id && builds[m]->req.keep_resident) break;
+            auto bld = building.find(r->req.mesh_id);
+            if (m == builds.size() || bld == building.end() || bld->second != 1) { ++it; continue; }
+            const uint64_t need = kRayBytes * r->req.num_rays + 64ull * builds[m]->req.num_triangles;
+            if (taken + out.size() >= cfg.max_batch_requests || !make_room(need)) break;
+            r->refit_index = (uint32_t)m;
+            r->refit_n = builds[m]->req.num_triangles;
+            r->bytes = need;
+            inflight_bytes += need;
+            st.peak_bytes = std::max(st.peak_bytes, inflight_bytes + resident_bytes);
+            r->t_taken = Clock::now();
+            r->lane = (uint32_t)lane;
+            out.push_back(r);
+            it = pending.erase(it);
+        }
+        return out;
+    }
+
     int run_batch(Lane& L, std::vector<Request*>& work, std::shared_ptr<BatchRec>* new_rec, std::vector<uint32_t>* build_index);
+    int run_late(Lane& L, const std::vector<Request*>& late, atr_batch* batch, void** d_late,
+                 std::vector<CopyJob>* results);
     void lane_loop(Lane* L);
 };
 
@@ -321,6 +354,56 @@ void set_msg(Request* r, int st) {
 }
 
 }  // namespace
+
+// Enqueues the refits that joined a batch, behind its builds and their rays:
+// staging and device buffers of their own (*d_late, the caller releases it), the
+// copies of their results, and what is left to copy once the stream is done.
+int atr_server::run_late(Lane& L, const std::vector<Request*>& late, atr_batch* batch, void** d_late,
+                         std::vector<CopyJob>* results) {
+    atr_ctx* ctx = L.ctx;
+    uint64_t verts = 0, rays = 0;
+    for (const Request* r : late) {
+        verts += (uint64_t)r->refit_n * 48;
+        rays += r->req.num_rays;
+    }
+    ATR_TRY(grow_pinned(&L.h_late, &L.h_late_cap, verts + rays * 48));
+    if (rays) ATR_TRY(ctx->alloc(d_late, rays * 48));
+    char* const h_rays = static_cast<char*>(L.h_late) + verts;
+    char* const h_res = h_rays + rays * 32;
+    char* const d_rays = static_cast<char*>(*d_late);
+    char* const d_res = d_rays + rays * 32;
+    std::vector<CopyJob> jobs;
+    uint64_t va = 0, ra = 0;
+    for (const Request* r : late) {
+        jobs.push_back({static_cast<char*>(L.h_late) + va, r->req.vertices, (size_t)r->refit_n * 48});
+        if (r->req.num_rays) jobs.push_back({h_rays + ra * 32, r->req.rays, (size_t)r->req.num_rays * 32});
+        va += (uint64_t)r->refit_n * 48;
+        ra += r->req.num_rays;
+    }
+    par_copy(jobs);
+    if (rays) ATR_CUDA(cudaMemcpyAsync(d_rays, h_rays, rays * 32, cudaMemcpyHostToDevice, ctx->stream));
+    va = ra = 0;
+    for (Request* r : late) {
+        int s = atr::batch_refit_mesh(ctx, batch, r->refit_index,
+                                      reinterpret_cast<const float*>(static_cast<char*>(L.h_late) + va), 0, &r->sah);
+        if (s == ATR_OK && r->req.num_rays) {
+            const uint32_t roff[2] = {0, r->req.num_rays};
+            const uint32_t gm[1] = {r->refit_index};
+            s = atr_batch_trace(ctx, batch, reinterpret_cast<const float*>(d_rays + ra * 32), r->req.num_rays, roff,
+                                gm, 1, 0, reinterpret_cast<int32_t*>(d_res + ra * 16));
+        }
+        if (s != ATR_OK) {
+            r->status = s;
+            set_msg(r, s);
+        } else if (r->req.num_rays) {
+            results->push_back({r->req.results, h_res + ra * 16, (size_t)r->req.num_rays * 16});
+        }
+        va += (uint64_t)r->refit_n * 48;
+        ra += r->req.num_rays;
+    }
+    if (rays) ATR_CUDA(cudaMemcpyAsync(h_res, d_res, rays * 16, cudaMemcpyDeviceToHost, ctx->stream));
+    return ATR_OK;
+}
 
 int atr_server::run_batch(Lane& L, std::vector<Request*>& work, std::shared_ptr<BatchRec>* new_rec,
                           std::vector<uint32_t>* build_index) {
@@ -530,12 +613,30 @@ int atr_server::run_batch(Lane& L, std::vector<Request*>& work, std::shared_ptr<
                                         (size_t)work[i]->req.num_rays * 16, cudaMemcpyDeviceToHost, ctx->stream);
         if (e != cudaSuccess) { release_rays(); return atr::cuda_fail(e, "cudaMemcpyAsync(results)", __FILE__, __LINE__); }
     }
+    // 4. Refits that were waiting for this batch's builds join it: their copies
+    // and kernels follow on the stream while the batch's own rays are traced, in
+    // place of a batch of their own once this one has been taken apart.
+    std::vector<CopyJob> out;
+    void* d_late = nullptr;
+    const size_t own = work.size();
+    if (*new_rec) {
+        const std::vector<Request*> late = join_refits(L.id, builds, work.size());
+        if (!late.empty()) {
+            work.insert(work.end(), late.begin(), late.end());
+            const int st_late = run_late(L, late, (*new_rec)->batch, &d_late, &out);
+            for (Request* r : late)
+                if (st_late != ATR_OK && r->status == ATR_OK) {
+                    r->status = st_late;
+                    set_msg(r, st_late);
+                }
+        }
+    }
     const int s = atr_ctx_synchronize(ctx);
     release_rays();
+    ctx->release(d_late);
     const Clock::time_point t_done = Clock::now();
     ATR_TRY(s);
-    std::vector<CopyJob> out;
-    for (size_t i = 0; i < work.size(); ++i)
+    for (size_t i = 0; i < own; ++i)
         if (work[i]->req.num_rays && work[i]->status == ATR_OK && !res_pinned[i])
             out.push_back({work[i]->req.results, static_cast<char*>(L.h_res) + stage_at[i] * 16,
                            (size_t)work[i]->req.num_rays * 16});
@@ -579,6 +680,9 @@ void atr_server::lane_loop(Lane* L) {
         lock.lock();
         account_busy(-1);
         ++use_clock;
+        // Refits may have joined.
+        st.max_batch_requests_seen = std::max(st.max_batch_requests_seen, (uint32_t)work.size());
+        for (Request* r : work) r->batch_requests = (uint32_t)work.size();
         // Resident bookkeeping for new meshes.
         if (rec && s != ATR_OK) {
             atr_batch_destroy(rec->batch);
@@ -810,6 +914,7 @@ int atr_server_destroy(atr_server* s) {
         if (L->h_rays) cudaFreeHost(L->h_rays);
         if (L->h_res) cudaFreeHost(L->h_res);
         if (L->h_rverts) cudaFreeHost(L->h_rverts);
+        if (L->h_late) cudaFreeHost(L->h_late);
         atr_ctx_destroy(L->ctx);
     }
     delete s;
