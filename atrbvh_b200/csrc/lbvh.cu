@@ -733,13 +733,15 @@ constexpr size_t tile_smem() {
 // ---- fused Karras build + refit ------------------------------------------------
 // Common prefix of the adjacent sorted pairs (k, k+1) with the reference's
 // index tie-break (LBVH.cu:163-201).
-__device__ __forceinline__ int delta_adj(const uint32_t* keys, int k) {
-    const uint32_t a = keys[k], b = keys[k + 1];
+__device__ __forceinline__ int delta_of(uint32_t a, uint32_t b, int k) {
     return a == b ? 32 + __clz(k ^ (k + 1)) : __clz(a ^ b);
 }
-__device__ __forceinline__ int delta_adj(const uint64_t* keys, int k) {
-    const uint64_t a = keys[k], b = keys[k + 1];
+__device__ __forceinline__ int delta_of(uint64_t a, uint64_t b, int k) {
     return a == b ? 64 + __clzll((long long)(k ^ (k + 1))) : __clzll((long long)(a ^ b));
+}
+template <typename K>
+__device__ __forceinline__ int delta_adj(const K* keys, int k) {
+    return delta_of(keys[k], keys[k + 1], k);
 }
 
 // One thread per sorted leaf climbs while it is the second of two siblings to
@@ -983,19 +985,23 @@ __global__ void __launch_bounds__(256) k_build_top(Segs segs, const K* __restric
         const int lc = split == pl ? split + last : split;
         const int rc = split + 1 == pr ? split + 1 + last : split + 1;
         const int sib = is_left ? rc : lc;
+        // Everything the step reads is requested at once: the sibling's box and
+        // record, and the keys beyond the end that the sibling adds (the prefix
+        // at the other end is known from below).
         const float4 smn = ld_cg(o.bmin + nb + sib), smx = ld_cg(o.bmax + nb + sib);
+        const int4 sr = o.pp.rec ? __ldcg(o.pp.rec + nb + sib) : make_int4(0, 0, 0, 0);
+        const int beyond = is_left ? pr : pl - 1;  // the adjacent pair there
+        const bool inside = is_left ? pr < last : pl > 0;
+        const K ka = inside ? keys[beyond] : (K)0, kb = inside ? keys[beyond + 1] : (K)0;
         mn = make_float4(fminf(mn.x, smn.x), fminf(mn.y, smn.y), fminf(mn.z, smn.z), 0.0f);
         mx = make_float4(fmaxf(mx.x, smx.x), fmaxf(mx.y, smx.y), fmaxf(mx.z, smx.z), 0.0f);
+        const int d = inside ? delta_of(ka, kb, beyond) : -1;
+        if (is_left) dr = d;
+        else dl = d;
         const bool root = pl == 0 && pr == last;
-        int p = 0;
-        if (!root) {
-            dl = pl > 0 ? delta_adj(keys, pl - 1) : -1;
-            dr = pr < last ? delta_adj(keys, pr) : -1;
-            p = dr > dl ? pr : pl;
-        }
+        const int p = root ? 0 : dr > dl ? pr : pl;
         const float pa = box_area(mn, mx);
         if (o.pp.rec) {
-            const int4 sr = __ldcg(o.pp.rec + nb + sib);
             const float sns = __int_as_float(sr.y);
             my_ns = __fadd_rn(__fadd_rn(__fmul_rn(kPrepassCi, pa), is_left ? my_ns : sns), is_left ? sns : my_ns);
             my_lv = pr - pl + 1 >= (o.pp.seg_gamma ? (int)o.pp.seg_gamma[m] : o.pp.gamma) ? 1 + max(my_lv, sr.w)
