@@ -260,24 +260,48 @@ __global__ void __launch_bounds__(kRefitThreads) k_refit_level(int level, const 
         s_kids[j] = it_kids[j0 + j];
         s_par[j] = it_par[j0 + j];
     }
-    for (int i = threadIdx.x; i < nin; i += kRefitThreads) {
-        float mn[3], mx[3];
-        if (level == 0) {
-            const uint32_t tri = (uint32_t)in_src[i0 + i];
-            const float4 a = __ldg(verts + 3 * (size_t)tri), b = __ldg(verts + 3 * (size_t)tri + 1),
-                         c = __ldg(verts + 3 * (size_t)tri + 2);
-            mn[0] = fminf(fminf(a.x, b.x), c.x); mn[1] = fminf(fminf(a.y, b.y), c.y); mn[2] = fminf(fminf(a.z, b.z), c.z);
-            mx[0] = fmaxf(fmaxf(a.x, b.x), c.x); mx[1] = fmaxf(fmaxf(a.y, b.y), c.y); mx[2] = fmaxf(fmaxf(a.z, b.z), c.z);
-        } else {
-            const int node = in_src[i0 + i];
-            const float4 a = bmin[node], b = bmax[node];
-            mn[0] = a.x; mn[1] = a.y; mn[2] = a.z;
-            mx[0] = b.x; mx[1] = b.y; mx[2] = b.z;
+    // A thread's inputs are loaded together: their indices, then the vertices or
+    // boxes these name (1,000,003 triangles with new vertices: 112.4 -> 109.6 us,
+    // bound by the gather's latency and its 128 bytes of sectors a triangle).
+    constexpr int kPer = kCtaInputs / kRefitThreads;
+    int src[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int i = threadIdx.x + q * kRefitThreads;
+        src[q] = i < nin ? in_src[i0 + i] : -1;
+    }
+    if (level == 0) {
+        float4 v[kPer][3];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q)
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                v[q][k] = src[q] >= 0 ? __ldg(verts + 3 * (size_t)src[q] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int i = threadIdx.x + q * kRefitThreads;
+            const float4 a = v[q][0], b = v[q][1], c = v[q][2];
+            if (src[q] < 0) continue;
+            s_mn[i][0] = fminf(fminf(a.x, b.x), c.x);
+            s_mn[i][1] = fminf(fminf(a.y, b.y), c.y);
+            s_mn[i][2] = fminf(fminf(a.z, b.z), c.z);
+            s_mx[i][0] = fmaxf(fmaxf(a.x, b.x), c.x);
+            s_mx[i][1] = fmaxf(fmaxf(a.y, b.y), c.y);
+            s_mx[i][2] = fmaxf(fmaxf(a.z, b.z), c.z);
+        }
+    } else {
+        float4 lo[kPer], hi[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            lo[q] = src[q] >= 0 ? bmin[src[q]] : make_float4(0.f, 0.f, 0.f, 0.f);
+            hi[q] = src[q] >= 0 ? bmax[src[q]] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            s_mn[i][k] = mn[k];
-            s_mx[i][k] = mx[k];
+        for (int q = 0; q < kPer; ++q) {
+            const int i = threadIdx.x + q * kRefitThreads;
+            if (src[q] < 0) continue;
+            s_mn[i][0] = lo[q].x; s_mn[i][1] = lo[q].y; s_mn[i][2] = lo[q].z;
+            s_mx[i][0] = hi[q].x; s_mx[i][1] = hi[q].y; s_mx[i][2] = hi[q].z;
         }
     }
     __syncthreads();
