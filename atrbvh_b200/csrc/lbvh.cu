@@ -751,8 +751,8 @@ __device__ __forceinline__ int delta_adj(const K* keys, int k) {
 // addressed from the mesh's first entry, so every mesh gets exactly the tree
 // a build of that mesh alone produces (local node and triangle indices).
 //
-// Two passes.  k_build_block: a block owns 256 consecutive sorted leaves and
-// finishes every node whose split position and the one after it lie in its
+// Two passes.  k_build_block: a block owns 256 or 512 consecutive sorted leaves
+// and finishes every node whose split position and the one after it lie in its
 // range, with the arrival slots, the adjacent-key deltas and the finished
 // boxes in shared memory.  Such a node's children lie in the block, so the
 // climb meets no other block.  A climb that reaches a split on the block's
@@ -794,31 +794,42 @@ __device__ __forceinline__ void write_inner(const BuildOut<K>& o, const Segs& se
     }
 }
 
-constexpr int kBuildBlock = 256;
+// Leaves a block of k_build_block owns.  The kernel is bound by instruction
+// issue (0.62 of the cycles at 4,194,304 triangles) next to its gathers and
+// writes, so a climb step keeps its shared-memory accesses few: an internal
+// node's record is one packed word, the prepass terms ride in the boxes' w and
+// the prefix at a step's near end is carried (build phase 394 -> 360 us at
+// 4,194,304 triangles; with 40 registers a thread, six blocks of 256 to an SM,
+// 1,308 -> 1,289 at 16.8M; with 32 they spill: 1,572).  Wider blocks leave
+// fewer climbs to k_build_top's global exchanges but wait longer at their
+// barriers.  Build phase, 256 | 512 leaves a block: 1,048,576 triangles 134 |
+// 137 us, 2,097,152 204 | 207, 3,145,728 279 | 278, 4,194,304 360 | 354,
+// 16,777,216 1,291 | 1,197; 128 leaves are within 2 us of 256 up to 1M and
+// slower above.
+int build_block(uint32_t n) { return n > (1u << 21) ? 512 : 256; }
 
-template <typename K>
-__global__ void __launch_bounds__(kBuildBlock) k_build_block(Segs segs, const K* __restrict__ keys_all,
-                                                             const uint32_t* __restrict__ sidx,
-                                                             const float4* __restrict__ verts, BuildOut<K> o,
-                                                             BuildEdge* __restrict__ edges, PrimBoxes pr) {
+template <typename K, int kBuildBlock>
+__global__ void __launch_bounds__(kBuildBlock, 1536 / kBuildBlock)
+    k_build_block(Segs segs, const K* __restrict__ keys_all, const uint32_t* __restrict__ sidx,
+                  const float4* __restrict__ verts, BuildOut<K> o, BuildEdge* __restrict__ edges, PrimBoxes pr) {
+    // Boxes of the block's leaves and finished internal nodes; mn.w carries the
+    // prepass's nodesSah, mx.w its level (0 at a leaf).
     __shared__ float4 s_lmn[kBuildBlock], s_lmx[kBuildBlock], s_imn[kBuildBlock], s_imx[kBuildBlock];
-    __shared__ float s_lns[kBuildBlock], s_ins[kBuildBlock];
-    __shared__ int s_ilv[kBuildBlock];  // prepass levels of the block's finished internal nodes
     __shared__ int s_slot[kBuildBlock];
     __shared__ int s_delta[kBuildBlock + 1];  // delta at sorted position B0 - 1 + k
     // Records of the internal nodes the block finishes, by block position
     // (internal node p of a mesh sits at its sorted position p), and the
     // parents it assigns: written out coalesced once the block's climbs end.
-    __shared__ int s_left[kBuildBlock], s_right[kBuildBlock];  // kUnset: not finished here
-    __shared__ int2 s_rng[kBuildBlock];
-    __shared__ int s_ipar[kBuildBlock], s_lpar[kBuildBlock];   // parents of internal node / leaf
+    // A record packs block positions: first | last << 10 | split << 20; kUnset: not finished here.
+    __shared__ uint32_t s_rec[kBuildBlock];
+    __shared__ int s_ipar[kBuildBlock], s_lpar[kBuildBlock];  // parents of internal node / leaf
     constexpr int kUnset = INT_MIN;
     const int tid = threadIdx.x;
     const uint32_t B0 = blockIdx.x * kBuildBlock;
     const uint32_t gi = B0 + tid;
     const bool live = gi < segs.n;
     s_slot[tid] = -1;
-    s_left[tid] = kUnset;
+    s_rec[tid] = (uint32_t)kUnset;
     s_ipar[tid] = kUnset;
     s_lpar[tid] = kUnset;
     if (tid < 2) edges[2 * blockIdx.x + tid] = BuildEdge{-1, -1, -1, -1};
@@ -826,7 +837,6 @@ __global__ void __launch_bounds__(kBuildBlock) k_build_block(Segs segs, const K*
     int nb = 0, last = 0;
     const K* keys = keys_all;
     float4 mn = make_float4(0.f, 0.f, 0.f, 0.f), mx = mn;
-    float my_ns = 0.0f;
     s_delta[tid] = -1;
     if (tid == kBuildBlock - 1) s_delta[kBuildBlock] = -1;
     if (live) {
@@ -865,11 +875,11 @@ __global__ void __launch_bounds__(kBuildBlock) k_build_block(Segs segs, const K*
         o.area[nb + leaf] = my_area;
         // Prepass for the first ATRBVH iteration: this subtree's nodesSah under
         // the default constants, (ci*A + left) + right bottom-up from ct*A at leaves.
-        my_ns = __fmul_rn(kPrepassCt, my_area);
+        const float my_ns = __fmul_rn(kPrepassCt, my_area);
         if (o.pp.rec) o.pp.rec[nb + leaf] = make_int4(1, __float_as_int(my_ns), __float_as_int(my_ns), 0);
+        mn.w = my_ns;
         s_lmn[tid] = mn;
         s_lmx[tid] = mx;
-        s_lns[tid] = my_ns;
         // Deltas within the mesh only: the climb never reads one across meshes.
         if (i > 0) s_delta[tid] = delta_adj(keys, (int)i - 1);
         if (tid == kBuildBlock - 1 && (int)i < last) s_delta[kBuildBlock] = delta_adj(keys, (int)i);
@@ -879,7 +889,6 @@ __global__ void __launch_bounds__(kBuildBlock) k_build_block(Segs segs, const K*
         const int off = (int)s0 - (int)B0;  // block position of mesh-local sorted index 0
         auto sd = [&](int x) { return s_delta[off + x + 1]; };
         int l = (int)i, r = (int)i, node = (int)i + last;
-        int my_lv = 0;
         int dl = l > 0 ? sd(l - 1) : -1;
         int dr = r < last ? sd(r) : -1;
         while (true) {
@@ -896,39 +905,30 @@ __global__ void __launch_bounds__(kBuildBlock) k_build_block(Segs segs, const K*
             __threadfence_block();
             const int pl = is_left ? l : other;
             const int pr = is_left ? other : r;
-            const int lc = split == pl ? split + last : split;
-            const int rc = split + 1 == pr ? split + 1 + last : split + 1;
             const bool sib_leaf = is_left ? split + 1 == pr : split == pl;
-            const int sib = is_left ? rc : lc;
-            const int sp = off + (sib_leaf ? sib - last : sib);
-            const float4 smn = sib_leaf ? s_lmn[sp] : s_imn[sp];
-            const float4 smx = sib_leaf ? s_lmx[sp] : s_imx[sp];
+            const int sp = is_left ? bs + 1 : bs;  // the left child sits at split, the right at split + 1
+            const float4 smn = *(sib_leaf ? s_lmn + sp : s_imn + sp);
+            const float4 smx = *(sib_leaf ? s_lmx + sp : s_imx + sp);
+            // The prefix at the end that the sibling adds; the other is known from below.
+            if (is_left) dr = pr < last ? sd(pr) : -1;
+            else dl = pl > 0 ? sd(pl - 1) : -1;
+            const float ns = mn.w;
+            const int lv = __float_as_int(mx.w);
             mn = make_float4(fminf(mn.x, smn.x), fminf(mn.y, smn.y), fminf(mn.z, smn.z), 0.0f);
             mx = make_float4(fmaxf(mx.x, smx.x), fmaxf(mx.y, smx.y), fmaxf(mx.z, smx.z), 0.0f);
             const bool root = pl == 0 && pr == last;
-            int p = 0;
-            if (!root) {
-                dl = pl > 0 ? sd(pl - 1) : -1;
-                dr = pr < last ? sd(pr) : -1;
-                p = dr > dl ? pr : pl;
-            }
-            const float pa = box_area(mn, mx);
+            const int p = root ? 0 : dr > dl ? pr : pl;
             if (o.pp.rec) {
-                const float sns = sib_leaf ? s_lns[sp] : s_ins[sp];
-                my_ns = __fadd_rn(__fadd_rn(__fmul_rn(kPrepassCi, pa), is_left ? my_ns : sns), is_left ? sns : my_ns);
+                const float pa = box_area(mn, mx);
+                mn.w = __fadd_rn(__fadd_rn(__fmul_rn(kPrepassCi, pa), is_left ? ns : smn.w), is_left ? smn.w : ns);
                 const int gam = o.pp.seg_gamma ? (int)o.pp.seg_gamma[m] : o.pp.gamma;
-                my_lv = pr - pl + 1 >= gam ? 1 + max(my_lv, sib_leaf ? 0 : s_ilv[sp]) : 0;
+                mx.w = __int_as_float(pr - pl + 1 >= gam ? 1 + max(lv, __float_as_int(smx.w)) : 0);
             }
-            s_left[off + p] = lc;
-            s_right[off + p] = rc;
-            s_rng[off + p] = make_int2(pl, pr);
-            // The left child sits at position split, the right at split + 1.
-            (split == pl ? s_lpar : s_ipar)[off + split] = p;
-            (split + 1 == pr ? s_lpar : s_ipar)[off + split + 1] = p;
+            s_rec[off + p] = (uint32_t)(off + pl) | (uint32_t)(off + pr) << 10 | (uint32_t)bs << 20;
+            (split == pl ? s_lpar : s_ipar)[bs] = p;
+            (split + 1 == pr ? s_lpar : s_ipar)[bs + 1] = p;
             s_imn[off + p] = mn;
             s_imx[off + p] = mx;
-            s_ins[off + p] = my_ns;
-            s_ilv[off + p] = my_lv;
             if (root) {
                 s_ipar[off] = -1;
                 break;
@@ -940,10 +940,15 @@ __global__ void __launch_bounds__(kBuildBlock) k_build_block(Segs segs, const K*
     }
     __syncthreads();
     if (live) {
-        if (s_left[tid] != kUnset) {  // internal node i, finished by this block
-            const int2 rg = s_rng[tid];
-            write_inner(o, segs, m, nb, (int)i, rg.x, rg.y, s_left[tid], s_right[tid], s_imn[tid], s_imx[tid],
-                        box_area(s_imn[tid], s_imx[tid]), s_ins[tid], s_ilv[tid]);
+        if (const uint32_t rec = s_rec[tid]; rec != (uint32_t)kUnset) {  // internal node i, finished by this block
+            const int off = (int)s0 - (int)B0;
+            const int pl = (int)(rec & 1023) - off, pr = (int)(rec >> 10 & 1023) - off, split = (int)(rec >> 20) - off;
+            float4 imn = s_imn[tid], imx = s_imx[tid];
+            const float ns = imn.w;
+            const int lv = __float_as_int(imx.w);
+            imn.w = imx.w = 0.0f;
+            write_inner(o, segs, m, nb, (int)i, pl, pr, split == pl ? split + last : split,
+                        split + 1 == pr ? split + 1 + last : split + 1, imn, imx, box_area(imn, imx), ns, lv);
         }
         if (s_ipar[tid] != kUnset) o.parent[nb + (int)i] = s_ipar[tid];
         if (s_lpar[tid] != kUnset) o.parent[nb + (int)i + last] = s_lpar[tid];
@@ -1175,7 +1180,8 @@ int build_typed(atr_ctx* ctx, const Segs& segs, uint32_t mesh_tiles, const float
     const size_t inner = n - segs.count;
     ATR_TRY(ctx->alloc(&kv, (size_t)n * sizeof(K)));
     int st = ctx->alloc(&iv, (size_t)n * 4);
-    const uint32_t bblocks = (n + kBuildBlock - 1) / kBuildBlock;
+    const int bb = build_block(n);
+    const uint32_t bblocks = (n + bb - 1) / bb;
     const size_t ebytes = (size_t)bblocks * 2 * sizeof(BuildEdge);
     if (st == ATR_OK)
         st = ctx->alloc(&aux, align256(hbytes) + align256(cbytes) + align256(inner * 4) + align256(ebytes));
@@ -1211,7 +1217,8 @@ int build_typed(atr_ctx* ctx, const Segs& segs, uint32_t mesh_tiles, const float
         const BuildOut<K> o{t.parent, t.left,  t.right, t.data,
                             t.bmin,   t.bmax,  t.area,  slot,
                             t.range,  prepass ? *prepass : BuildPrepass{}};
-        k_build_block<K><<<bblocks, kBuildBlock, 0, s>>>(segs, keys, idx, verts, o, edges, pr);
+        (bb == 512 ? k_build_block<K, 512> : k_build_block<K, 256>)<<<bblocks, bb, 0, s>>>(segs, keys, idx, verts, o,
+                                                                                           edges, pr);
         k_build_top<K><<<(2 * bblocks + 255) / 256, 256, 0, s>>>(segs, keys, o, edges, 2 * bblocks);
         ctx->phase_end();
         ctx->launches += 2;
