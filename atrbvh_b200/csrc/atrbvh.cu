@@ -816,59 +816,52 @@ __global__ void __launch_bounds__(256) k_levels_pp_hist(TreeRefs g, Segs segs, L
     __syncthreads();
     int lvl[kListPer];
     uint2 lent[kListPer];
+    // The build's records are final for every node below gamma (count,
+    // both nodesSah, level 0) and hold the level of the others.
 #pragma unroll
-    for (int q = 0; q < kListPer; ++q) {
-        const uint32_t i = blockIdx.x * kListBlock + q * 256 + threadIdx.x;
-        int push = 0;
-        bool above = false;
-        uint2 ent[2];
-        lvl[q] = 0;
-        lent[q] = make_uint2(0u, 0u);
-        if (i < segs.n) {
-            const uint32_t m = segs.seg_of_tri(i);
-            const uint32_t s0 = segs.tri_begin(m);
-            const uint32_t n = segs.tri_end(m) - s0;
-            if (!seg_iters || 0 < (int)seg_iters[m]) {
-                const int base = segs.node_base(m), cb = segs.inner_base(m);
-                const int gamma = seg_tsize ? (int)seg_tsize[m] : tsize_all;
-                const int li = (int)(i - s0);
-                // The build's records are final for every node below gamma (count,
-                // both nodesSah, level 0) and hold the level of the others.
-                if (li < (int)n - 1) {
-                    const int x = li;
-                    const int lc = g.left[base + x], rc = g.right[base + x];
-                    const int2 r = ranges[cb + x];
-                    const int cnt = r.y - r.x + 1;
-                    lv.kids[cb + x] =
-                        make_int4(lc, rc, __float_as_int(g.area[base + lc]), __float_as_int(g.area[base + rc]));
-                    if (cnt >= gamma) {
-                        const int me = *rec_i(lv.rec, base + x, 3);
-                        lent[q] = make_uint2(m, (uint32_t)x);
-                        if (me <= L) {
-                            lvl[q] = me;
-                        } else {
-                            above = true;
-                            if ((is_internal(lc, n) ? *rec_i(lv.rec, base + lc, 3) : 0) <= L)
-                                ent[push++] = make_uint2(m, (uint32_t)lc);
-                            if ((is_internal(rc, n) ? *rec_i(lv.rec, base + rc, 3) : 0) <= L)
-                                ent[push++] = make_uint2(m, (uint32_t)rc);
-                        }
-                    }
+    for (int q0 = 0; q0 < kListPer; q0 += kListAhead) {
+        int lc[kListAhead], rc[kListAhead], cnt[kListAhead], me[kListAhead];
+        float al[kListAhead], ar[kListAhead];
+#pragma unroll
+        for (int u = 0; u < kListAhead; ++u) {
+            const uint32_t i = blockIdx.x * kListBlock + (q0 + u) * 256 + threadIdx.x;
+            lc[u] = rc[u] = cnt[u] = 0;  // no node
+            lent[q0 + u] = make_uint2(0u, 0u);
+            if (i < segs.n) {
+                const uint32_t m = segs.seg_of_tri(i);
+                const uint32_t s0 = segs.tri_begin(m);
+                if ((!seg_iters || 0 < (int)seg_iters[m]) && i - s0 < segs.tri_end(m) - s0 - 1) {
+                    const int x = (int)(i - s0), base = segs.node_base(m);
+                    lent[q0 + u] = make_uint2(m, (uint32_t)x);
+                    lc[u] = g.left[base + x];
+                    rc[u] = g.right[base + x];
+                    const int2 r = ranges[segs.inner_base(m) + x];
+                    cnt[u] = r.y - r.x + 1;
                 }
             }
         }
-        list_top(lv, above, lent[q]);
-        // Frontier entries: one atomic per warp.
-        uint32_t incl = push;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, o);
-            if ((threadIdx.x & 31) >= o) incl += y;
+#pragma unroll
+        for (int u = 0; u < kListAhead; ++u) {
+            const uint32_t m = lent[q0 + u].x;
+            const int x = (int)lent[q0 + u].y, base = segs.node_base(m);
+            al[u] = ar[u] = 0.0f;
+            me[u] = 0;
+            if (cnt[u]) {
+                al[u] = g.area[base + lc[u]];
+                ar[u] = g.area[base + rc[u]];
+                if (cnt[u] >= (seg_tsize ? (int)seg_tsize[m] : tsize_all)) me[u] = *rec_i(lv.rec, base + x, 3);
+            }
         }
-        const uint32_t total = __shfl_sync(kFull, incl, 31);
-        uint32_t at = 0;
-        if ((threadIdx.x & 31) == 31 && total) at = atomicAdd(lv.n_frontier, total);
-        at = __shfl_sync(kFull, at, 31) + incl - push;
-        for (int k = 0; k < push; ++k) lv.frontier[at + k] = ent[k];
+#pragma unroll
+        for (int u = 0; u < kListAhead; ++u) {
+            const int q = q0 + u;
+            const uint32_t m = lent[q].x, x = lent[q].y;
+            if (cnt[u])
+                lv.kids[segs.inner_base(m) + (int)x] =
+                    make_int4(lc[u], rc[u], __float_as_int(al[u]), __float_as_int(ar[u]));
+            lvl[q] = me[u] <= L ? me[u] : 0;
+            list_above(segs, lv, me[u] > L, m, x, lc[u], rc[u], L);
+        }
     }
     file_levels(lv, L, lvl, lent, s_cnt, s_base);
 }

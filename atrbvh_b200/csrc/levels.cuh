@@ -99,6 +99,14 @@ __device__ const ArgmaxPriority g_argmax_priority = argmax_priority();
 constexpr int kMaxLevels = 64;  // largest L (ATR_TUNE_ATR_LEVELS)
 constexpr int kListPer = 8;                  // nodes per thread of the level-list kernels
 constexpr int kListBlock = 256 * kListPer;  // nodes per block of those kernels
+// Nodes whose reads a thread of those kernels requests at once.  The passes are
+// bound by latency and by their warps in flight: one node after another, each
+// with its warp scan for the frontier, ATRBVH took 1,826 us at 4,194,304
+// triangles and 5,252 at 16.8M; two at once (48 registers) and the scan only in
+// warps that hold a node above the level passes 1,807 and 5,176, four (58) 1,814
+// and 5,181, eight (74) 1,828 and 5,223.
+constexpr int kListAhead = 2;
+static_assert(kListPer % kListAhead == 0, "whole batches of nodes");
 
 struct LevelRefs {
     int4* rec;             // per node (node-indexed): count, nodesSah x 2, level (see NextRefs)
@@ -258,6 +266,34 @@ __device__ __forceinline__ void file_levels(const LevelRefs& lv, int L, const in
         }
 }
 
+// A block's big nodes above level L (one per thread, m and x) go to the top
+// list, and their children at levels up to L to the dataflow pass's frontier.
+__device__ __forceinline__ void list_above(const Segs& segs, const LevelRefs& lv, bool above, uint32_t m, uint32_t x,
+                                           int lc, int rc, int L) {
+    if (!__any_sync(kFull, above)) return;  // nearly every warp: a few hundred nodes are above
+    list_top(lv, above, make_uint2(m, x));
+    bool pl = false, pr = false;
+    if (above) {
+        const uint32_t n = segs.tri_end(m) - segs.tri_begin(m);
+        const int nb = segs.node_base(m);
+        pl = (is_internal(lc, n) ? *rec_i(lv.rec, nb + lc, 3) : 0) <= L;
+        pr = (is_internal(rc, n) ? *rec_i(lv.rec, nb + rc, 3) : 0) <= L;
+    }
+    // Frontier entries: one atomic per warp.
+    const uint32_t push = pl + pr;
+    uint32_t incl = push;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, o);
+        if ((threadIdx.x & 31) >= o) incl += y;
+    }
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    uint32_t at = 0;
+    if ((threadIdx.x & 31) == 31 && total) at = atomicAdd(lv.n_frontier, total);
+    at = __shfl_sync(kFull, at, 31) + incl - push;
+    if (pl) lv.frontier[at++] = make_uint2(m, (uint32_t)lc);
+    if (pr) lv.frontier[at] = make_uint2(m, (uint32_t)rc);
+}
+
 // Phase A of iterations after the first: the previous iteration left every
 // internal node's level for this one (next levels of the nodes it finished,
 // kept current by treelet rewrites), and subtree counts, nodesSah and child
@@ -273,52 +309,35 @@ __global__ void __launch_bounds__(256) k_level_hist(Segs segs, LevelRefs lv, con
     int lvl[kListPer];
     uint2 lent[kListPer];
 #pragma unroll
-    for (int q = 0; q < kListPer; ++q) {
-        const uint32_t i = blockIdx.x * kListBlock + q * 256 + threadIdx.x;
-        int push = 0;
-        bool above = false;
-        uint32_t m = 0;
-        uint2 ent[2];
-        lvl[q] = 0;
-        lent[q] = make_uint2(0u, 0u);
-        if (i < segs.n) {
-            m = segs.seg_of_tri(i);
-            const uint32_t s0 = segs.tri_begin(m);
-            const uint32_t n = segs.tri_end(m) - s0;
-            const uint32_t li = i - s0;
-            if ((!seg_iters || iteration < (int)seg_iters[m]) && li < n - 1) {
-                const int cb = segs.inner_base(m), nb = segs.node_base(m);
-                const int me = *rec_i(lv.rec, nb + (int)li, 3);
-                if (me == 0) {
-                    // Not a treelet root: its next nodesSah is this one (the level
-                    // stays 0).
-                    *rec_f(lv.rec, nb + (int)li, rec_ns_next(lv.par)) = *rec_f(lv.rec, nb + (int)li, rec_ns_cur(lv.par));
-                } else if (me <= L) {
-                    lvl[q] = me;
-                    lent[q] = make_uint2(m, li);
-                } else {
-                    above = true;
-                    lent[q] = make_uint2(m, li);
-                    const int4 kd = lv.kids[cb + (int)li];
-                    if ((is_internal(kd.x, n) ? *rec_i(lv.rec, nb + kd.x, 3) : 0) <= L)
-                        ent[push++] = make_uint2(m, (uint32_t)kd.x);
-                    if ((is_internal(kd.y, n) ? *rec_i(lv.rec, nb + kd.y, 3) : 0) <= L)
-                        ent[push++] = make_uint2(m, (uint32_t)kd.y);
+    for (int q0 = 0; q0 < kListPer; q0 += kListAhead) {
+        int4 rec[kListAhead];
+#pragma unroll
+        for (int u = 0; u < kListAhead; ++u) {
+            const uint32_t i = blockIdx.x * kListBlock + (q0 + u) * 256 + threadIdx.x;
+            rec[u] = make_int4(0, 0, 0, -1);  // nothing to do
+            lent[q0 + u] = make_uint2(0u, 0u);
+            if (i < segs.n) {
+                const uint32_t m = segs.seg_of_tri(i);
+                const uint32_t s0 = segs.tri_begin(m);
+                if ((!seg_iters || iteration < (int)seg_iters[m]) && i - s0 < segs.tri_end(m) - s0 - 1) {
+                    lent[q0 + u] = make_uint2(m, i - s0);
+                    rec[u] = lv.rec[segs.node_base(m) + (int)(i - s0)];
                 }
             }
         }
-        list_top(lv, above, lent[q]);
-        // Frontier entries: one atomic per warp.
-        uint32_t incl = push;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, o);
-            if ((threadIdx.x & 31) >= o) incl += y;
+#pragma unroll
+        for (int u = 0; u < kListAhead; ++u) {
+            const int q = q0 + u, me = rec[u].w;
+            const uint32_t m = lent[q].x, x = lent[q].y;
+            // Not a treelet root: its next nodesSah is this one (the level stays 0).
+            if (me == 0)
+                *rec_i(lv.rec, segs.node_base(m) + (int)x, rec_ns_next(lv.par)) = lv.par ? rec[u].z : rec[u].y;
+            lvl[q] = me > 0 && me <= L ? me : 0;
+            const bool above = me > L;
+            int4 kd = make_int4(0, 0, 0, 0);
+            if (above) kd = lv.kids[segs.inner_base(m) + (int)x];
+            list_above(segs, lv, above, m, x, kd.x, kd.y, L);
         }
-        const uint32_t total = __shfl_sync(kFull, incl, 31);
-        uint32_t at = 0;
-        if ((threadIdx.x & 31) == 31 && total) at = atomicAdd(lv.n_frontier, total);
-        at = __shfl_sync(kFull, at, 31) + incl - push;
-        for (int k = 0; k < push; ++k) lv.frontier[at + k] = ent[k];
     }
     file_levels(lv, L, lvl, lent, s_cnt, s_base);
 }
