@@ -361,32 +361,46 @@ void set_msg(Request* r, int st) {
 int atr_server::run_late(Lane& L, const std::vector<Request*>& late, atr_batch* batch, void** d_late,
                          std::vector<CopyJob>* results) {
     atr_ctx* ctx = L.ctx;
-    uint64_t verts = 0, rays = 0;
-    for (const Request* r : late) {
-        verts += (uint64_t)r->refit_n * 48;
-        rays += r->req.num_rays;
+    // Page-locked buffers are copied from and to directly; staging holds the
+    // pageable ones only, packed (pinning more of it while lanes run stalls them).
+    uint64_t rays = 0, stage = 0;
+    std::vector<int64_t> v_at(late.size(), -1), r_at(late.size(), -1), s_at(late.size(), -1);  // -1: direct
+    for (size_t i = 0; i < late.size(); ++i) {
+        const Request* r = late[i];
+        const uint64_t n = r->req.num_rays;
+        auto place = [&](int64_t& at, const void* p, uint64_t bytes) {
+            if (!bytes || is_pinned(p)) return;
+            at = (int64_t)stage;
+            stage += bytes;
+        };
+        place(v_at[i], r->req.vertices, (uint64_t)r->refit_n * 48);
+        place(r_at[i], r->req.rays, n * 32);
+        place(s_at[i], r->req.results, n * 16);
+        rays += n;
     }
-    ATR_TRY(grow_pinned(&L.h_late, &L.h_late_cap, verts + rays * 48));
+    if (stage) ATR_TRY(grow_pinned(&L.h_late, &L.h_late_cap, stage));
     if (rays) ATR_TRY(ctx->alloc(d_late, rays * 48));
-    char* const h_rays = static_cast<char*>(L.h_late) + verts;
-    char* const h_res = h_rays + rays * 32;
+    char* const h = static_cast<char*>(L.h_late);
     char* const d_rays = static_cast<char*>(*d_late);
     char* const d_res = d_rays + rays * 32;
     std::vector<CopyJob> jobs;
-    uint64_t va = 0, ra = 0;
-    for (const Request* r : late) {
-        jobs.push_back({static_cast<char*>(L.h_late) + va, r->req.vertices, (size_t)r->refit_n * 48});
-        if (r->req.num_rays) jobs.push_back({h_rays + ra * 32, r->req.rays, (size_t)r->req.num_rays * 32});
-        va += (uint64_t)r->refit_n * 48;
-        ra += r->req.num_rays;
+    for (size_t i = 0; i < late.size(); ++i) {
+        const Request* r = late[i];
+        if (v_at[i] >= 0) jobs.push_back({h + v_at[i], r->req.vertices, (size_t)r->refit_n * 48});
+        if (r_at[i] >= 0) jobs.push_back({h + r_at[i], r->req.rays, (size_t)r->req.num_rays * 32});
     }
-    par_copy(jobs);
-    if (rays) ATR_CUDA(cudaMemcpyAsync(d_rays, h_rays, rays * 32, cudaMemcpyHostToDevice, ctx->stream));
-    va = ra = 0;
-    for (Request* r : late) {
-        int s = atr::batch_refit_mesh(ctx, batch, r->refit_index,
-                                      reinterpret_cast<const float*>(static_cast<char*>(L.h_late) + va), 0, &r->sah);
-        if (s == ATR_OK && r->req.num_rays) {
+    if (!jobs.empty()) par_copy(jobs);
+    uint64_t ra = 0;
+    for (size_t i = 0; i < late.size(); ++i) {
+        Request* r = late[i];
+        const size_t n = r->req.num_rays;
+        if (n)
+            ATR_CUDA(cudaMemcpyAsync(d_rays + ra * 32,
+                                     r_at[i] >= 0 ? static_cast<const void*>(h + r_at[i]) : r->req.rays,
+                                     n * 32, cudaMemcpyHostToDevice, ctx->stream));
+        const void* v = v_at[i] >= 0 ? static_cast<const void*>(h + v_at[i]) : r->req.vertices;
+        int s = atr::batch_refit_mesh(ctx, batch, r->refit_index, static_cast<const float*>(v), 0, &r->sah);
+        if (s == ATR_OK && n) {
             const uint32_t roff[2] = {0, r->req.num_rays};
             const uint32_t gm[1] = {r->refit_index};
             s = atr_batch_trace(ctx, batch, reinterpret_cast<const float*>(d_rays + ra * 32), r->req.num_rays, roff,
@@ -395,13 +409,13 @@ int atr_server::run_late(Lane& L, const std::vector<Request*>& late, atr_batch* 
         if (s != ATR_OK) {
             r->status = s;
             set_msg(r, s);
-        } else if (r->req.num_rays) {
-            results->push_back({r->req.results, h_res + ra * 16, (size_t)r->req.num_rays * 16});
+        } else if (n) {
+            void* dst = s_at[i] >= 0 ? static_cast<void*>(h + s_at[i]) : r->req.results;
+            ATR_CUDA(cudaMemcpyAsync(dst, d_res + ra * 16, n * 16, cudaMemcpyDeviceToHost, ctx->stream));
+            if (s_at[i] >= 0) results->push_back({r->req.results, dst, n * 16});
         }
-        va += (uint64_t)r->refit_n * 48;
-        ra += r->req.num_rays;
+        ra += n;
     }
-    if (rays) ATR_CUDA(cudaMemcpyAsync(h_res, d_res, rays * 16, cudaMemcpyDeviceToHost, ctx->stream));
     return ATR_OK;
 }
 
