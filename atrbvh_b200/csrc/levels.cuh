@@ -40,9 +40,12 @@ __device__ __forceinline__ int4 make_rec(int cnt, float ns_cur, float ns_next, i
 // the tree on a tie pattern; argmax_priority ranks the lanes by removing
 // winners one at a time.  The full-warp path then needs two warp reductions:
 // the maximum value, then the lowest rank among the lanes holding it.
-struct ArgmaxPriority {
+// The kernels copy the table to shared memory four bytes at a time.
+struct alignas(16) ArgmaxPriority {
     uint8_t rank[kMaxTreelet + 1][32];
 };
+static_assert(alignof(ArgmaxPriority) >= sizeof(uint32_t) && sizeof(ArgmaxPriority) % sizeof(uint32_t) == 0,
+              "whole aligned words");
 
 constexpr int tree_winner(int m, uint32_t tied) {
     int val[32] = {};
