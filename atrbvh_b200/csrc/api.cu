@@ -140,6 +140,7 @@ int atr_ctx_create(int device, void* stream, atr_ctx** out) {
     if (e == cudaSuccess && atr::lbvh_prepare() != ATR_OK) e = cudaErrorInvalidValue;
     if (e == cudaSuccess && atr::atrbvh_prepare(c) != ATR_OK) e = cudaErrorInvalidValue;
     if (e == cudaSuccess && atr::trbvh_prepare(c) != ATR_OK) e = cudaErrorInvalidValue;
+    if (e == cudaSuccess && atr::trace_prepare(c) != ATR_OK) e = cudaErrorInvalidValue;
     if (e != cudaSuccess) {
         cudaFree(c->d_error);
         cudaFreeHost(c->h_stage);

@@ -265,11 +265,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
 template <int kStack, bool kMapped>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
                   const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter) {
-    static int blocks_per_sm = 0;
-    if (!blocks_per_sm) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_trace<kStack, kMapped>, kTraceThreads, 0);
-        if (blocks_per_sm < 1) blocks_per_sm = 1;
-    }
+    const int blocks_per_sm = ctx->trace_blocks[kStack > 64][kMapped];
     // Rays per warp: the paths of a warp's rays add up as far as they differ, so
     // few rays are spread over as many warps as run at once (1,000 rays through
     // 20,011 triangles: 57 us at one ray a warp, 93 at 32; 50,000 rays: 103 us at
@@ -340,6 +336,22 @@ __global__ void __launch_bounds__(256) k_bounce(const float4* __restrict__ verts
 }
 
 }  // namespace
+
+// Blocks of each instance that an SM holds (once per context: contexts launch from
+// threads of their own).
+int trace_prepare(atr_ctx* ctx) {
+    auto set = [&](int deep, int mapped, auto kernel) {
+        int* const b = &ctx->trace_blocks[deep][mapped];
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(b, kernel, kTraceThreads, 0);
+        if (e != cudaSuccess || *b < 1) *b = 1;
+        return e;
+    };
+    ATR_CUDA(set(0, 0, k_trace<64, false>));
+    ATR_CUDA(set(0, 1, k_trace<64, true>));
+    ATR_CUDA(set(1, 0, k_trace<256, false>));
+    ATR_CUDA(set(1, 1, k_trace<256, true>));
+    return ATR_OK;
+}
 
 int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
               int max_depth, const float4* rays, int64_t n, int any_hit, int4* res) {

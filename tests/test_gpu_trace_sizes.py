@@ -68,3 +68,42 @@ def test_captured_trace_replays_beside_direct_ones(ctx, deep):
         torch.cuda.synchronize()
         assert np.array_equal(a.cpu().numpy()[:, :2], want[:, :2])
         assert np.array_equal(b.cpu().numpy()[:, :2], want[:, :2])
+
+
+def test_contexts_trace_side_by_side(deep):
+    """Threads with a context each, as the server's lanes: launch shapes are the context's."""
+    import threading
+
+    import torch
+    scene, col, bvh, cp, mn, mx = deep
+    n, threads = 20011, 6
+    rays = ab.gen_rays_random(n, mn, mx, seed=3)
+    want = O.trace(cp, rays)
+    rd = torch.from_numpy(rays).cuda()
+    image = bvh.serialize()
+    res = torch.zeros((threads, n, 4), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    start = threading.Barrier(threads)
+    errors = []
+
+    def work(k):
+        try:
+            start.wait()
+            c = ab.Context(0)
+            own = ab.CudaBVH.from_image(c, image)
+            own.trace(rd.data_ptr(), n, res[k].data_ptr())
+            c.synchronize()
+            own.close()
+            c.close()
+        except BaseException as e:  # reported after the join
+            errors.append(e)
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(threads)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    got = res.cpu().numpy()
+    for k in range(threads):
+        assert np.array_equal(got[k][:, :2], want[:, :2]), k
