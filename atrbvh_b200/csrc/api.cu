@@ -134,7 +134,10 @@ int atr_ctx_create(int device, void* stream, atr_ctx** out) {
         return atr::cuda_fail(e, "cudaMemPoolCreate", __FILE__, __LINE__);
     }
     e = cudaMalloc(&c->d_error, 128);
+    // The context's stream does not wait for the legacy stream that clears the
+    // words, and the first trace already counts on them: wait here.
     if (e == cudaSuccess) e = cudaMemset(c->d_error, 0, 128);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&c->h_stage), atr_ctx::kStage, cudaHostAllocDefault);
     if (e == cudaSuccess) c->d_trace = reinterpret_cast<unsigned long long*>(c->d_error + 16);
     if (e == cudaSuccess && atr::lbvh_prepare() != ATR_OK) e = cudaErrorInvalidValue;
