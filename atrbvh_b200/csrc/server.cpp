@@ -93,8 +93,6 @@ struct Lane {
     size_t h_res_cap = 0;
     void* h_rverts = nullptr;  // refit vertices
     size_t h_rverts_cap = 0;
-    void* h_late = nullptr;  // vertices, rays and results of refits that join a batch
-    size_t h_late_cap = 0;
 };
 
 struct CopyJob {
@@ -255,13 +253,22 @@ struct atr_server {
         }
     }
 
-    // Take admissible requests for `lane`.  Caller holds mu.
-    std::vector<Request*> take(int lane) {
+    // Take admissible requests for `lane`; with `of`, refits of that batch's
+    // meshes only, beside the `taken` requests of the lane batch that built them.
+    // Caller holds mu.
+    std::vector<Request*> take(int lane, const BatchRec* of = nullptr, size_t taken = 0) {
         std::vector<Request*> out;
         uint64_t tris = 0;
         for (auto it = pending.begin(); it != pending.end();) {
-            if (out.size() >= cfg.max_batch_requests) break;
+            if (taken + out.size() >= cfg.max_batch_requests) break;
             Request* r = *it;
+            if (of) {
+                auto res = resident.find(r->req.mesh_id);
+                if (r->req.kind != ATR_REQ_REFIT || res == resident.end() || res->second.rec.get() != of) {
+                    ++it;
+                    continue;
+                }
+            }
             uint64_t need = kRayBytes * r->req.num_rays;
             if (r->req.kind == ATR_REQ_REFIT) {
                 auto bld = building.find(r->req.mesh_id);
@@ -312,38 +319,9 @@ struct atr_server {
         return out;
     }
 
-    // Waiting refits of the meshes that `lane` has just built in `builds` (kept
-    // resident, no other build of them in flight), with the mesh's index: they
-    // join the batch that built them.  Takes the lock.
-    std::vector<Request*> join_refits(int lane, const std::vector<Request*>& builds, size_t taken) {
-        std::vector<Request*> out;
-        std::lock_guard<std::mutex> lock(mu);
-        for (auto it = pending.begin(); it != pending.end();) {
-            Request* r = *it;
-            size_t m = builds.size();
-            if (r->req.kind == ATR_REQ_REFIT)
-                for (m = 0; m < builds.size(); ++m)
-                    if (builds[m]->req.mesh_id == r->req.mesh_id && builds[m]->req.keep_resident) break;
-            auto bld = building.find(r->req.mesh_id);
-            if (m == builds.size() || bld == building.end() || bld->second != 1) { ++it; continue; }
-            const uint64_t need = kRayBytes * r->req.num_rays + 64ull * builds[m]->req.num_triangles;
-            if (taken + out.size() >= cfg.max_batch_requests || !make_room(need)) break;
-            r->refit_index = (uint32_t)m;
-            r->refit_n = builds[m]->req.num_triangles;
-            r->bytes = need;
-            inflight_bytes += need;
-            st.peak_bytes = std::max(st.peak_bytes, inflight_bytes + resident_bytes);
-            r->t_taken = Clock::now();
-            r->lane = (uint32_t)lane;
-            out.push_back(r);
-            it = pending.erase(it);
-        }
-        return out;
-    }
-
     int run_batch(Lane& L, std::vector<Request*>& work, std::shared_ptr<BatchRec>* new_rec, std::vector<uint32_t>* build_index);
-    int run_late(Lane& L, const std::vector<Request*>& late, atr_batch* batch, void** d_late,
-                 std::vector<CopyJob>* results);
+    void complete(const Lane& L, const std::vector<Request*>& work, const std::shared_ptr<BatchRec>& rec,
+                  const std::vector<uint32_t>& index, int s, const std::string& msg);
     void lane_loop(Lane* L);
 };
 
@@ -354,70 +332,6 @@ void set_msg(Request* r, int st) {
 }
 
 }  // namespace
-
-// Enqueues the refits that joined a batch, behind its builds and their rays:
-// staging and device buffers of their own (*d_late, the caller releases it), the
-// copies of their results, and what is left to copy once the stream is done.
-int atr_server::run_late(Lane& L, const std::vector<Request*>& late, atr_batch* batch, void** d_late,
-                         std::vector<CopyJob>* results) {
-    atr_ctx* ctx = L.ctx;
-    // Page-locked buffers are copied from and to directly; staging holds the
-    // pageable ones only, packed (pinning more of it while lanes run stalls them).
-    uint64_t rays = 0, stage = 0;
-    std::vector<int64_t> v_at(late.size(), -1), r_at(late.size(), -1), s_at(late.size(), -1);  // -1: direct
-    for (size_t i = 0; i < late.size(); ++i) {
-        const Request* r = late[i];
-        const uint64_t n = r->req.num_rays;
-        auto place = [&](int64_t& at, const void* p, uint64_t bytes) {
-            if (!bytes || is_pinned(p)) return;
-            at = (int64_t)stage;
-            stage += bytes;
-        };
-        place(v_at[i], r->req.vertices, (uint64_t)r->refit_n * 48);
-        place(r_at[i], r->req.rays, n * 32);
-        place(s_at[i], r->req.results, n * 16);
-        rays += n;
-    }
-    if (stage) ATR_TRY(grow_pinned(&L.h_late, &L.h_late_cap, stage));
-    if (rays) ATR_TRY(ctx->alloc(d_late, rays * 48));
-    char* const h = static_cast<char*>(L.h_late);
-    char* const d_rays = static_cast<char*>(*d_late);
-    char* const d_res = d_rays + rays * 32;
-    std::vector<CopyJob> jobs;
-    for (size_t i = 0; i < late.size(); ++i) {
-        const Request* r = late[i];
-        if (v_at[i] >= 0) jobs.push_back({h + v_at[i], r->req.vertices, (size_t)r->refit_n * 48});
-        if (r_at[i] >= 0) jobs.push_back({h + r_at[i], r->req.rays, (size_t)r->req.num_rays * 32});
-    }
-    if (!jobs.empty()) par_copy(jobs);
-    uint64_t ra = 0;
-    for (size_t i = 0; i < late.size(); ++i) {
-        Request* r = late[i];
-        const size_t n = r->req.num_rays;
-        if (n)
-            ATR_CUDA(cudaMemcpyAsync(d_rays + ra * 32,
-                                     r_at[i] >= 0 ? static_cast<const void*>(h + r_at[i]) : r->req.rays,
-                                     n * 32, cudaMemcpyHostToDevice, ctx->stream));
-        const void* v = v_at[i] >= 0 ? static_cast<const void*>(h + v_at[i]) : r->req.vertices;
-        int s = atr::batch_refit_mesh(ctx, batch, r->refit_index, static_cast<const float*>(v), 0, &r->sah);
-        if (s == ATR_OK && n) {
-            const uint32_t roff[2] = {0, r->req.num_rays};
-            const uint32_t gm[1] = {r->refit_index};
-            s = atr_batch_trace(ctx, batch, reinterpret_cast<const float*>(d_rays + ra * 32), r->req.num_rays, roff,
-                                gm, 1, 0, reinterpret_cast<int32_t*>(d_res + ra * 16));
-        }
-        if (s != ATR_OK) {
-            r->status = s;
-            set_msg(r, s);
-        } else if (n) {
-            void* dst = s_at[i] >= 0 ? static_cast<void*>(h + s_at[i]) : r->req.results;
-            ATR_CUDA(cudaMemcpyAsync(dst, d_res + ra * 16, n * 16, cudaMemcpyDeviceToHost, ctx->stream));
-            if (s_at[i] >= 0) results->push_back({r->req.results, dst, n * 16});
-        }
-        ra += n;
-    }
-    return ATR_OK;
-}
 
 int atr_server::run_batch(Lane& L, std::vector<Request*>& work, std::shared_ptr<BatchRec>* new_rec,
                           std::vector<uint32_t>* build_index) {
@@ -627,30 +541,12 @@ int atr_server::run_batch(Lane& L, std::vector<Request*>& work, std::shared_ptr<
                                         (size_t)work[i]->req.num_rays * 16, cudaMemcpyDeviceToHost, ctx->stream);
         if (e != cudaSuccess) { release_rays(); return atr::cuda_fail(e, "cudaMemcpyAsync(results)", __FILE__, __LINE__); }
     }
-    // 4. Refits that were waiting for this batch's builds join it: their copies
-    // and kernels follow on the stream while the batch's own rays are traced, in
-    // place of a batch of their own once this one has been taken apart.
-    std::vector<CopyJob> out;
-    void* d_late = nullptr;
-    const size_t own = work.size();
-    if (*new_rec) {
-        const std::vector<Request*> late = join_refits(L.id, builds, work.size());
-        if (!late.empty()) {
-            work.insert(work.end(), late.begin(), late.end());
-            const int st_late = run_late(L, late, (*new_rec)->batch, &d_late, &out);
-            for (Request* r : late)
-                if (st_late != ATR_OK && r->status == ATR_OK) {
-                    r->status = st_late;
-                    set_msg(r, st_late);
-                }
-        }
-    }
     const int s = atr_ctx_synchronize(ctx);
     release_rays();
-    ctx->release(d_late);
     const Clock::time_point t_done = Clock::now();
     ATR_TRY(s);
-    for (size_t i = 0; i < own; ++i)
+    std::vector<CopyJob> out;
+    for (size_t i = 0; i < work.size(); ++i)
         if (work[i]->req.num_rays && work[i]->status == ATR_OK && !res_pinned[i])
             out.push_back({work[i]->req.results, static_cast<char*>(L.h_res) + stage_at[i] * 16,
                            (size_t)work[i]->req.num_rays * 16});
@@ -662,6 +558,70 @@ int atr_server::run_batch(Lane& L, std::vector<Request*>& work, std::shared_ptr<
         st.lane_batch_ms += ms_between(t_start, Clock::now());
     }
     return ATR_OK;
+}
+
+// Books what run_batch did with `work` (its status s and message): new meshes
+// become resident, every request is finished.  Caller holds mu.
+void atr_server::complete(const Lane& L, const std::vector<Request*>& work, const std::shared_ptr<BatchRec>& rec,
+                          const std::vector<uint32_t>& index, int s, const std::string& msg) {
+    ++use_clock;
+    if (rec && s != ATR_OK) {
+        atr_batch_destroy(rec->batch);
+        rec->batch = nullptr;
+    }
+    if (rec && s == ATR_OK) {
+        size_t m = 0;
+        for (Request* r : work) {
+            if (r->req.kind != ATR_REQ_BUILD) continue;
+            if (r->req.keep_resident) {
+                auto old = resident.find(r->req.mesh_id);
+                if (old != resident.end()) {
+                    auto orec = old->second.rec;
+                    resident.erase(old);
+                    unref(orec);
+                }
+                resident[r->req.mesh_id] = Resident{rec, index[m], r->req.num_triangles};
+                ++rec->live;
+            }
+            ++m;
+        }
+        rec->last_use = use_clock;
+        if (rec->live) {
+            batches.push_back(rec);
+            resident_bytes += rec->bytes;
+        } else {
+            atr_batch_destroy(rec->batch);
+            rec->batch = nullptr;
+        }
+    }
+    for (Request* r : work) {
+        inflight_bytes -= r->bytes;
+        if (r->req.kind == ATR_REQ_REFIT && r->refit_rec) {
+            auto f = resident.find(r->req.mesh_id);
+            if (f != resident.end() && f->second.busy_lane == L.id) f->second.busy_lane = -1;
+            --r->refit_rec->busy;
+            r->refit_rec->last_use = use_clock;
+            r->refit_rec.reset();
+        }
+        if (s != ATR_OK) {
+            finish(r, s, msg.c_str());
+        } else {
+            if (r->status == ATR_OK) {
+                if (r->req.kind == ATR_REQ_BUILD) {
+                    ++st.builds;
+                    st.triangles_built += r->req.num_triangles;
+                } else {
+                    ++st.refits;
+                    auto f = resident.find(r->req.mesh_id);
+                    if (f != resident.end()) st.triangles_refit += f->second.n;
+                }
+                st.rays_traced += r->req.num_rays;
+            }
+            finish(r, r->status, r->status == ATR_OK ? nullptr : r->error.c_str());
+        }
+    }
+    // Batches released while this lane used them.
+    for (auto& b : std::vector<std::shared_ptr<BatchRec>>(batches)) maybe_free(b);
 }
 
 void atr_server::lane_loop(Lane* L) {
@@ -682,81 +642,35 @@ void atr_server::lane_loop(Lane* L) {
                               [](Request* r) { return r->req.kind == ATR_REQ_BUILD; });
         account_busy(+1);
         ++st.lane_batches;
-        st.max_batch_requests_seen = std::max(st.max_batch_requests_seen, (uint32_t)work.size());
-        for (Request* r : work) r->batch_requests = (uint32_t)work.size();
-        lock.unlock();
-
+        auto run = [&](std::vector<Request*>& part, std::shared_ptr<BatchRec>* rec, std::vector<uint32_t>* index) {
+            lock.unlock();
+            const int s = run_batch(*L, part, rec, index);
+            const std::string msg = s == ATR_OK ? std::string() : std::string(atr_last_error());
+            lock.lock();
+            complete(*L, part, *rec, *index, s, msg);
+        };
         std::shared_ptr<BatchRec> rec;
         std::vector<uint32_t> index;
-        const int s = run_batch(*L, work, &rec, &index);
-        const std::string msg = s == ATR_OK ? std::string() : std::string(atr_last_error());
-
-        lock.lock();
-        account_busy(-1);
-        ++use_clock;
-        // Refits may have joined.
-        st.max_batch_requests_seen = std::max(st.max_batch_requests_seen, (uint32_t)work.size());
-        for (Request* r : work) r->batch_requests = (uint32_t)work.size();
-        // Resident bookkeeping for new meshes.
-        if (rec && s != ATR_OK) {
-            atr_batch_destroy(rec->batch);
-            rec->batch = nullptr;
-        }
-        if (rec && s == ATR_OK) {
-            size_t m = 0;
-            for (Request* r : work) {
-                if (r->req.kind != ATR_REQ_BUILD) continue;
-                if (r->req.keep_resident) {
-                    auto old = resident.find(r->req.mesh_id);
-                    if (old != resident.end()) {
-                        auto orec = old->second.rec;
-                        resident.erase(old);
-                        unref(orec);
-                    }
-                    resident[r->req.mesh_id] = Resident{rec, index[m], r->req.num_triangles};
-                    ++rec->live;
-                }
-                ++m;
-            }
-            rec->last_use = use_clock;
-            if (rec->live) {
-                batches.push_back(rec);
-                resident_bytes += rec->bytes;
-            } else {
-                atr_batch_destroy(rec->batch);
-                rec->batch = nullptr;
-            }
-        }
-        for (Request* r : work) {
-            inflight_bytes -= r->bytes;
-            if (r->req.kind == ATR_REQ_REFIT && r->refit_rec) {
-                auto f = resident.find(r->req.mesh_id);
-                if (f != resident.end() && f->second.busy_lane == L->id) f->second.busy_lane = -1;
-                --r->refit_rec->busy;
-                r->refit_rec->last_use = use_clock;
-                r->refit_rec.reset();
-            }
-            if (s != ATR_OK) {
-                finish(r, s, msg.c_str());
-            } else {
-                if (r->status == ATR_OK) {
-                    if (r->req.kind == ATR_REQ_BUILD) {
-                        ++st.builds;
-                        st.triangles_built += r->req.num_triangles;
-                    } else {
-                        ++st.refits;
-                        auto f = resident.find(r->req.mesh_id);
-                        if (f != resident.end()) st.triangles_refit += f->second.n;
-                    }
-                    st.rays_traced += r->req.num_rays;
-                }
-                finish(r, r->status, r->status == ATR_OK ? nullptr : r->error.c_str());
-            }
-        }
-        // Batches released while this lane used them.
-        for (auto& b : std::vector<std::shared_ptr<BatchRec>>(batches)) maybe_free(b);
+        run(work, &rec, &index);
+        // Refits that waited for a mesh of this batch follow as its second part.
+        // The builds are finished by now: their results do not wait for the
+        // refits, and the refits' errors are their own.
+        std::vector<Request*> late;
+        if (rec && rec->live) late = take(L->id, rec.get(), work.size());
+        const uint32_t members = (uint32_t)(work.size() + late.size());
+        st.max_batch_requests_seen = std::max(st.max_batch_requests_seen, members);
+        for (Request* r : work) r->batch_requests = members;
+        for (Request* r : late) r->batch_requests = members;
         cv_done.notify_all();
         cv_work.notify_all();
+        if (!late.empty()) {
+            std::shared_ptr<BatchRec> none;
+            index.clear();
+            run(late, &none, &index);
+            cv_done.notify_all();
+            cv_work.notify_all();
+        }
+        account_busy(-1);
     }
 }
 
@@ -928,7 +842,6 @@ int atr_server_destroy(atr_server* s) {
         if (L->h_rays) cudaFreeHost(L->h_rays);
         if (L->h_res) cudaFreeHost(L->h_res);
         if (L->h_rverts) cudaFreeHost(L->h_rverts);
-        if (L->h_late) cudaFreeHost(L->h_late);
         atr_ctx_destroy(L->ctx);
     }
     delete s;

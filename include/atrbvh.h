@@ -471,9 +471,10 @@ int atr_batch_apply_tuning(atr_ctx* ctx, atr_batch* batch, const atr_tune_table*
  * builds the new meshes in one segmented batch, refits the resident ones,
  * traces all their rays in one merged queue and copies the results back, so
  * requests that arrive while other lanes are busy run beside them on the
- * device.  Refits that wait for a mesh of the batch join it once the mesh is
- * built.  Each result equals that of the same request run alone.  Host
- * buffers of a request must stay valid until atr_server_wait returns it. */
+ * device.  Refits that wait for a mesh of the batch follow as its second part,
+ * once the results of the builds are out (batch_requests counts them too).
+ * Each result equals that of the same request run alone.  Host buffers of a
+ * request must stay valid until atr_server_wait returns it. */
 typedef struct atr_server atr_server;
 
 enum { ATR_REQ_BUILD = 0, ATR_REQ_REFIT = 1 };

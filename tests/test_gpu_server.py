@@ -168,3 +168,105 @@ def test_server_pinned_request_buffers_equal_pageable():
     for k in range(len(reqs)):
         assert np.array_equal(outs[k], outs_alone[k]), f"request {k}"
         assert np.float32(res_mix[k]["sah"]) == np.float32(res_alone[k]["sah"]), k
+
+
+def _buffers(reqs, kind):
+    """The requests' arrays page-locked, pageable, or by turns."""
+    if kind == "pageable":
+        return reqs, [np.full((len(r[3]), 4), -7, np.int32) for r in reqs]
+    pin = [kind == "pinned" or k % 2 == 0 for k in range(3 * len(reqs))]
+    out = []
+    for k, (what, mid, v, rays) in enumerate(reqs):
+        v = ab.pinned_like(v) if pin[3 * k] else v
+        out.append((what, mid, v, ab.pinned_like(rays) if pin[3 * k + 1] and len(rays) else rays))
+    res = [np.full((len(r[3]), 4), -7, np.int32) for r in reqs]
+    return out, [ab.pinned_like(o) if pin[3 * k + 2] and len(o) else o for k, o in enumerate(res)]
+
+
+def _submit_all(srv, reqs, outs):
+    stamps, tickets = [], []
+    for (kind, mid, v, rays), out in zip(reqs, outs):
+        stamps.append(time.perf_counter())
+        tickets.append(srv.submit(kind, mid, v, rays if len(rays) else None, out if len(rays) else None))
+    return stamps, [srv.wait(t) for t in tickets]
+
+
+def _joining(n=400000, refits=3):
+    """A build that lasts and, at once, refits of its mesh: one without rays."""
+    v = _mesh(n, 21)
+    none = np.zeros((0, 8), np.float32)
+    reqs = [(ab.REQ_BUILD, 5, v, _rays(v, 6000, 1))]
+    for k in range(refits):
+        w = _jitter(v, 300 + k)
+        reqs.append((ab.REQ_REFIT, 5, w, none if k == 1 else _rays(w, 4000 + k, 2 + k)))
+    return reqs
+
+
+def _same(outs, res, want_outs, want_res):
+    assert all(r["status"] == 0 for r in res), [r["error"] for r in res if r["status"]]
+    for k in range(len(outs)):
+        assert np.array_equal(outs[k], want_outs[k]), k
+        assert np.float32(res[k]["sah"]) == np.float32(want_res[k]["sah"]), k
+
+
+@pytest.mark.parametrize("kind", ["pageable", "pinned", "mixed"])
+def test_server_refits_follow_the_build_they_wait_for(kind):
+    """Refits that wait for a build are the second part of its batch; two of one
+    mesh apply in order, one has no rays."""
+    reqs, outs = _buffers(_joining(), kind)
+    srv = ab.Server(lanes=1, max_batch_requests=8)
+    _, res = _submit_all(srv, reqs, outs)
+    alone = ab.Server(lanes=1, max_batch_requests=1)
+    want_outs = [np.full((len(r[3]), 4), -7, np.int32) for r in reqs]
+    want = [alone.wait(alone.submit(k, m, v, r if len(r) else None, o if len(r) else None))
+            for (k, m, v, r), o in zip(reqs, want_outs)]
+    assert [r["batch_requests"] for r in res] == [len(reqs)] * len(reqs)
+    assert srv.stats()["lane_batches"] == 1
+    srv.close()
+    alone.close()
+    _same(outs, res, want_outs, want)
+
+
+def test_server_builds_do_not_wait_for_refits_that_join():
+    reqs, outs = _buffers(_joining(refits=7), "pageable")
+    srv = ab.Server(lanes=1, max_batch_requests=8)
+    stamps, res = _submit_all(srv, reqs, outs)
+    srv.close()
+    assert res[0]["batch_requests"] == len(reqs)
+    done = [s + r["latency_ms"] / 1e3 for s, r in zip(stamps, res)]
+    # Seven refits stage 19 MB each, copy it and refit 400,000 triangles.
+    assert min(done[1:]) - done[0] > 1e-3, [r["latency_ms"] for r in res]
+
+
+def test_server_join_ends_at_the_batch_limit():
+    reqs, outs = _buffers(_joining(), "pageable")
+    srv = ab.Server(lanes=1, max_batch_requests=2)
+    _, res = _submit_all(srv, reqs, outs)
+    st = srv.stats()
+    alone = ab.Server(lanes=1, max_batch_requests=1)
+    want_outs, want = _buffers(reqs, "pageable")[1], None
+    _, want = _submit_all(alone, reqs, want_outs)
+    srv.close()
+    alone.close()
+    assert res[0]["batch_requests"] == res[1]["batch_requests"] == 2 and st["max_batch_requests_seen"] == 2
+    _same(outs, res, want_outs, want)
+
+
+def test_server_refits_wait_for_every_build_of_their_mesh():
+    """Build, refit, build, refit of one id at once: both refits are of the second build."""
+    a, b = _mesh(300000, 31), _mesh(300000, 32)
+    r = _rays(a, 5000, 4)
+    reqs = [(ab.REQ_BUILD, 9, a, r), (ab.REQ_REFIT, 9, _jitter(b, 1), r),
+            (ab.REQ_BUILD, 9, b, r), (ab.REQ_REFIT, 9, _jitter(b, 2), r)]
+    outs = _buffers(reqs, "pageable")[1]
+    srv = ab.Server(lanes=1, max_batch_requests=8)
+    _, res = _submit_all(srv, reqs, outs)
+    srv.close()
+    order = [0, 2, 1, 3]
+    alone = ab.Server(lanes=1, max_batch_requests=1)
+    want_outs, want = [None] * 4, [None] * 4
+    for k in order:
+        want_outs[k] = np.full((len(r), 4), -7, np.int32)
+        want[k] = alone.wait(alone.submit(*reqs[k], want_outs[k]))
+    alone.close()
+    _same(outs, res, want_outs, want)
