@@ -142,7 +142,6 @@ int atr_ctx_create(int device, void* stream, atr_ctx** out) {
     if (e == cudaSuccess) c->d_trace = reinterpret_cast<unsigned long long*>(c->d_error + 16);
     if (e == cudaSuccess && atr::lbvh_prepare() != ATR_OK) e = cudaErrorInvalidValue;
     if (e == cudaSuccess && atr::atrbvh_prepare(c) != ATR_OK) e = cudaErrorInvalidValue;
-    if (e == cudaSuccess && atr::trbvh_prepare(c) != ATR_OK) e = cudaErrorInvalidValue;
     if (e == cudaSuccess && atr::trace_prepare(c) != ATR_OK) e = cudaErrorInvalidValue;
     if (e != cudaSuccess) {
         cudaFree(c->d_error);

@@ -1509,7 +1509,7 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
 }
 
 // Kernel attributes (once per context).
-int atrbvh_prepare(atr_ctx* ctx) { return top_cluster(k_atr_top, 0, &ctx->top_ctas); }
+int atrbvh_prepare(atr_ctx* ctx) { return top_cluster(k_atr_top, &ctx->top_ctas); }
 
 }  // namespace atr
 

@@ -110,7 +110,7 @@ struct atr_ctx {
     // four-lane groups (eight per warp); -1 = never.
     int atr_quad_min = 20000;
     int atr_warp_max = 4096;
-    int top_ctas = 8, tr_top_ctas = 8;  // cluster sizes of the ATRBVH and TRBVH top kernels
+    int top_ctas = 8;  // cluster size of the ATRBVH top kernel
     int trace_blocks[2][2] = {{1, 1}, {1, 1}};  // traversal's blocks per SM: [stack of 256][several meshes]
     struct Phase {
         std::string name;
@@ -296,7 +296,6 @@ int atrbvh_group_width(int max_tsize);
 int atrbvh_prepare(atr_ctx* ctx);  // kernel attributes; once per context
 int trbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_nodes, int iterations,
               const uint8_t* seg_iters, float ci, float ct, const int2* karras_ranges = nullptr);
-int trbvh_prepare(atr_ctx* ctx);  // kernel attributes; once per context
 int trace_prepare(atr_ctx* ctx);  // launch shapes; once per context
 
 int sort_ray_words(atr_ctx* ctx, const uint32_t* words, const uint32_t* diff, uint32_t n, uint32_t* keys_a,

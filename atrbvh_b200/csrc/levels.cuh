@@ -1,6 +1,6 @@
 // The bottom-up order of a treelet pass, shared by the ATRBVH and TRBVH
 // optimisers: node records, the level of every treelet root, the roots listed
-// level by level, and the cluster that takes the narrow levels at the top.
+// level by level, and the cluster that takes small ATRBVH trees' narrow levels.
 #pragma once
 
 #include "common.cuh"
@@ -451,14 +451,13 @@ __device__ __forceinline__ void top_levels(const Segs& segs, const LevelRefs& lv
 }
 
 // Launch shape of a top kernel: one cluster.
-inline cudaLaunchConfig_t top_config(int ctas, cudaLaunchAttribute* at, cudaStream_t s, size_t smem = 0) {
+inline cudaLaunchConfig_t top_config(int ctas, cudaLaunchAttribute* at, cudaStream_t s) {
     at->id = cudaLaunchAttributeClusterDimension;
     at->val.clusterDim.x = (unsigned)ctas;
     at->val.clusterDim.y = at->val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(kTopWarps * 32);
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 1;
@@ -468,10 +467,10 @@ inline cudaLaunchConfig_t top_config(int ctas, cudaLaunchAttribute* at, cudaStre
 // The largest cluster `kernel` may be launched with: 16 CTAs (above 8 is
 // non-portable) where the device runs such a cluster, else 8.
 template <class K>
-int top_cluster(K kernel, size_t smem, int* ctas) {
+int top_cluster(K kernel, int* ctas) {
     ATR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchAttribute at{};
-    const cudaLaunchConfig_t cfg = top_config(16, &at, nullptr, smem);
+    const cudaLaunchConfig_t cfg = top_config(16, &at, nullptr);
     int clusters = 0;
     const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
     if (e != cudaSuccess) cudaGetLastError();

@@ -18,13 +18,14 @@
 // An iteration runs level by level as ATRBVH's does (levels.cuh): one climb
 // from every leaf finishes the nodes that are not treelet roots and levels the
 // roots, one pass lists them, then each level's treelets are restructured in one
-// launch, a warp each, and the narrow levels at the top by one cluster of CTAs.
-// The dataflow kernel k_trbvh takes a top that does not fit the cluster kernel.
+// launch, a warp each; the dataflow kernel k_trbvh takes the narrow levels above.
 // Bound by the subset programme's issue on the wide levels and by one treelet's
 // latency on the narrow ones.  300,007 uniform triangles, 3 iterations:
 // 1.59 -> 0.90 ms against one climb that restructured treelets as its warps
 // reached them (a warp's up to eight one after another, 17 % of the warps
-// resident).
+// resident).  ATRBVH's cluster for the narrow levels is no gain here, cluster |
+// dataflow: 1,003 triangles 304 | 288 us, 65,536 568 | 562, 262,144 850 | 843,
+// 1,000,003 1,791 | 1,783, 16.8M 22.09 | 22.11 ms.
 
 #include "common.cuh"
 #include "internal.h"
@@ -396,19 +397,6 @@ __global__ void __launch_bounds__(kTrWarps * 32, 3) k_tr_level(TreeRefs g, Segs 
         restructure_root(g, segs, lv, lv.order[e], ci, s_tr[w], s_t);
 }
 
-// The levels above L, by one cluster.
-__global__ void __launch_bounds__(kTopWarps * 32, 1) k_tr_top(TreeRefs g, Segs segs, LevelRefs lv, TopRefs tr, int L,
-                                                              float ci) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    TrShared* const s_tr = reinterpret_cast<TrShared*>(smem_raw);
-    __shared__ TrTables s_t;
-    __shared__ uint32_t s_off[kTopLevels + 1];
-    __shared__ uint32_t s_max;
-    load_tables(s_t);
-    top_levels(segs, lv, tr, L, s_off, &s_max,
-               [&](uint2 q) { restructure_root(g, segs, lv, q, ci, s_tr[threadIdx.x >> 5], s_t); });
-}
-
 // The dataflow pass: climbs from the frontier below the levels above L (all
 // that lies under a start is final); the second thread to reach a node finishes
 // it, and a warp restructures the treelets its lanes reach one after another.
@@ -471,7 +459,7 @@ int trbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_no
     ATR_TRY(ctx->alloc(&scratch, b_rec + b_kid + b_ctr + ls.bytes()));
     char* p = static_cast<char*>(scratch);
     LevelRefs lv{};
-    TopRefs tr{};
+    TopRefs tr{};  // no cluster here
     lv.rec = reinterpret_cast<int4*>(p); p += b_rec;
     lv.kids = reinterpret_cast<int4*>(p); p += b_kid;
     lv.counters = reinterpret_cast<uint32_t*>(p); p += b_ctr;
@@ -480,7 +468,6 @@ int trbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_no
     cudaStream_t s = ctx->stream;
     const unsigned climb = (segs.n + kLvBlock - 1) / kLvBlock, list = (segs.n + kListBlock - 1) / kListBlock;
     const unsigned grid = (unsigned)ctx->num_sms * 3;  // grid-stride over a level's roots
-    const size_t top_smem = kTopWarps * sizeof(TrShared);
     cudaError_t e = cudaSuccess;
     ctx->phase_begin("trbvh");
     for (int it = 0; it < iterations && e == cudaSuccess; ++it) {
@@ -492,24 +479,17 @@ int trbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_no
                                             it == 0 ? karras_ranges : nullptr);
         k_level_hist<<<list, 256, 0, s>>>(segs, lv, seg_iters, it, L);
         for (int lev = 1; lev <= L; ++lev) k_tr_level<<<grid, kTrWarps * 32, 0, s>>>(g, segs, lv, lev, ci);
-        cudaLaunchAttribute at{};
-        const cudaLaunchConfig_t cfg = top_config(ctx->tr_top_ctas, &at, s, top_smem);
-        e = cudaLaunchKernelEx(&cfg, k_tr_top, g, segs, lv, tr, L, ci);
+        // The climb's arrivals; the dataflow pass counts its own.
+        if (zero_words_async(ctx, lv.counters, inner) != ATR_OK) e = cudaErrorLaunchFailure;
+        if (e != cudaSuccess) break;
         k_trbvh<<<grid, kTrWarps * 32, 0, s>>>(g, segs, lv, ci);
-        ctx->launches += 4 + (uint64_t)L;
+        ctx->launches += 3 + (uint64_t)L;
     }
     ctx->phase_end();
     if (e == cudaSuccess) e = cudaGetLastError();
     ctx->release(scratch);
     if (e != cudaSuccess) return cuda_fail(e, "TRBVH launch", __FILE__, __LINE__);
     return ATR_OK;
-}
-
-// Kernel attributes (once per context).
-int trbvh_prepare(atr_ctx* ctx) {
-    constexpr size_t smem = kTopWarps * sizeof(TrShared);
-    ATR_CUDA(cudaFuncSetAttribute(k_tr_top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return top_cluster(k_tr_top, smem, &ctx->tr_top_ctas);
 }
 
 }  // namespace atr
