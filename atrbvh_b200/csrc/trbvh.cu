@@ -104,9 +104,18 @@ __device__ __forceinline__ void size_round(TrShared& sm, const uint8_t* __restri
     __syncwarp();
 }
 
+// A child record from the tree itself.  Called by all lanes or one.
+__device__ __forceinline__ int4 tree_kids(const TreeRefs& g, int nb, int x) {
+    const int l = ld_cg(g.left + nb + x), r = ld_cg(g.right + nb + x);
+    return make_int4(l, r, __float_as_int(ld_cg(g.area + nb + l)), __float_as_int(ld_cg(g.area + nb + r)));
+}
+
 // One treelet by the whole warp: root and its child record rk, nodesSah and
 // triangle count.  KD and rec start at the mesh's first inner node and node.
-__device__ bool process_trbvh(const TreeRefs& g, int nb, uint32_t n, int root, int4 rk, int4* KD, int4* rec,
+// kTight: there are neither, child records come from the tree and nodesSah is in
+// `ns`, which starts at the mesh's first node.
+template <bool kTight>
+__device__ bool process_trbvh(const TreeRefs& g, int nb, uint32_t n, int root, int4 rk, int4* KD, int4* rec, float* ns,
                               float root_sah, int tri_count, float ci, float ct, TrShared& sm,
                               const uint8_t* __restrict__ s_prio, const uint8_t* __restrict__ s_by_size) {
     const int lane = threadIdx.x & 31;
@@ -126,7 +135,8 @@ __device__ bool process_trbvh(const TreeRefs& g, int nb, uint32_t n, int root, i
     auto join = [&](int node, float area) {
         s_node = node;
         s_area = area;
-        if (is_internal(node, n)) cp_async16_cg(sm.kid + lane, KD + node);
+        if constexpr (!kTight)
+            if (is_internal(node, n)) cp_async16_cg(sm.kid + lane, KD + node);
     };
     if (lane < 2) join(lane == 0 ? rk.x : rk.y, __int_as_float(lane == 0 ? rk.z : rk.w));
 #pragma unroll
@@ -157,10 +167,15 @@ __device__ bool process_trbvh(const TreeRefs& g, int nb, uint32_t n, int root, i
             cp_async_wait_all();
             return false;
         }
-        if (lane == largest) cp_async_wait_all();
-        __syncwarp();
-        const int4 k = sm.kid[largest];
-        __syncwarp();
+        int4 k;
+        if constexpr (kTight) {
+            k = tree_kids(g, nb, rep);
+        } else {
+            if (lane == largest) cp_async_wait_all();
+            __syncwarp();
+            k = sm.kid[largest];
+            __syncwarp();
+        }
         if (lane == it + 1) internal_node = rep;
         if (lane == largest) join(k.x, __int_as_float(k.z));
         else if (lane == it + 2) join(k.y, __int_as_float(k.w));
@@ -170,7 +185,7 @@ __device__ bool process_trbvh(const TreeRefs& g, int nb, uint32_t n, int root, i
     if (lane < kTr) {
         s_mn = ld_cg(BMN + s_node);
         s_mx = ld_cg(BMX + s_node);
-        s_sah = is_internal(s_node, n) ? ld_cg(rec_f(rec, s_node, 1)) : __fmul_rn(ct, s_area);
+        s_sah = is_internal(s_node, n) ? ld_cg(kTight ? ns + s_node : rec_f(rec, s_node, 1)) : __fmul_rn(ct, s_area);
     }
     cp_async_wait_all();
 
@@ -323,7 +338,7 @@ __device__ bool process_trbvh(const TreeRefs& g, int nb, uint32_t n, int root, i
                 BMN[lc] = mn;
                 BMX[lc] = mx;
                 AR[lc] = la = box_area(mn, mx);
-                *rec_f(rec, lc, 1) = sm.cost[P];
+                *(kTight ? ns + lc : rec_f(rec, lc, 1)) = sm.cost[P];
                 const int pos = __popc(lb & lt);
                 sm.stack_node[pos] = lc;
                 sm.stack_set[pos] = P;
@@ -334,12 +349,12 @@ __device__ bool process_trbvh(const TreeRefs& g, int nb, uint32_t n, int root, i
                 BMN[rc] = mn;
                 BMX[rc] = mx;
                 AR[rc] = ra = box_area(mn, mx);
-                *rec_f(rec, rc, 1) = sm.cost[P];
+                *(kTight ? ns + rc : rec_f(rec, rc, 1)) = sm.cost[P];
                 const int pos = __popc(lb) + __popc(rb & lt);
                 sm.stack_node[pos] = rc;
                 sm.stack_set[pos] = Q;
             }
-            KD[e_node] = make_int4(lc, rc, __float_as_int(la), __float_as_int(ra));
+            if constexpr (!kTight) KD[e_node] = make_int4(lc, rc, __float_as_int(la), __float_as_int(ra));
         }
         __syncwarp();
         size = __popc(lb) + __popc(rb);
@@ -377,7 +392,7 @@ __device__ __forceinline__ void restructure_root(const TreeRefs& g, const Segs& 
     const float sah = __fadd_rn(__fadd_rn(__fmul_rn(ci, ld_cg(g.area + nb + x)), ld_cg(rec_f(rec, rk.x, 1))),
                                 ld_cg(rec_f(rec, rk.y, 1)));
     if ((threadIdx.x & 31) == 0) *rec_f(rec, x, 1) = sah;
-    if (!process_trbvh(g, nb, n, x, rk, kd, rec, sah, cnt, ci, lv.ct, sm, t.prio, t.by_size) &&
+    if (!process_trbvh<false>(g, nb, n, x, rk, kd, rec, nullptr, sah, cnt, ci, lv.ct, sm, t.prio, t.by_size) &&
         (threadIdx.x & 31) == 0)
         set_error_bits(lv.err, kErrTreeletClimb);
     __syncwarp();
@@ -445,6 +460,119 @@ __global__ void __launch_bounds__(kTrWarps * 32) k_trbvh(TreeRefs g, Segs segs, 
     }
 }
 
+// One climb that restructures treelets as its warps reach them, for trees whose
+// level passes find no memory: 20 bytes of scratch a triangle (counts and nodesSah
+// per node, arrivals) in place of 75 to 82.  Level passes | this, 3 iterations:
+// 20,011 triangles 456 | 499 us, 100,003 615 | 623, 1,000,003 1,783 | 2,716, 16.8M
+// 22.1 | 39.7 ms.
+__global__ void __launch_bounds__(kTrWarps * 32) k_tr_tight(TreeRefs g, Segs segs, int32_t* __restrict__ counts,
+                                                            float* __restrict__ nsah, uint32_t* __restrict__ counters,
+                                                            const uint8_t* __restrict__ seg_iters, int iteration,
+                                                            float ci, float ct, uint32_t* __restrict__ err) {
+    __shared__ TrShared s_tr[kTrWarps];
+    __shared__ TrTables s_t;
+    load_tables(s_t);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    int cur = -1, base = 0, cbase = 0;
+    uint32_t n = 2;
+    if (i < segs.n) {
+        const uint32_t m = segs.seg_of_tri(i), s0 = segs.tri_begin(m);
+        n = segs.tri_end(m) - s0;
+        base = segs.node_base(m);
+        cbase = segs.inner_base(m);
+        if (!seg_iters || iteration < (int)seg_iters[m]) {
+            const int leaf = base + (int)(i - s0) + (int)n - 1;
+            counts[leaf] = 1;
+            nsah[leaf] = __fmul_rn(ct, g.area[leaf]);
+            cur = g.parent[leaf];
+        }
+    }
+    const int gamma = kTr << iteration;
+    while (__any_sync(kFull, cur >= 0)) {
+        int cnt = 0;
+        float sah = 0.0f;
+        if (cur >= 0) {
+            // The other lanes' parts of the treelets below are ordered before this
+            // by the warp barrier that follows them.
+            fence_acq_rel_gpu();
+            if (atomic_add_acq_rel_gpu(&counters[cbase + cur], 1u) == 0u) {
+                cur = -1;
+            } else {
+                const int x = base + cur;
+                const int l = base + ld_cg(g.left + x), r = base + ld_cg(g.right + x);
+                cnt = ld_cg(counts + l) + ld_cg(counts + r);
+                sah = __fadd_rn(__fadd_rn(__fmul_rn(ci, ld_cg(g.area + x)), ld_cg(nsah + l)), ld_cg(nsah + r));
+                counts[x] = cnt;
+                nsah[x] = sah;
+            }
+        }
+        unsigned vote = __ballot_sync(kFull, cnt >= gamma);
+        __syncwarp();
+        while (vote) {
+            const int rl = __ffs(vote) - 1;
+            const int root = __shfl_sync(kFull, cur, rl), nb = __shfl_sync(kFull, base, rl);
+            const int rcnt = __shfl_sync(kFull, cnt, rl);
+            const float rsah = __shfl_sync(kFull, sah, rl);
+            const uint32_t rn = __shfl_sync(kFull, n, rl);
+            if (!process_trbvh<true>(g, nb, rn, root, tree_kids(g, nb, root), nullptr, nullptr, nsah + nb, rsah, rcnt,
+                                     ci, ct, s_tr[w], s_t.prio, s_t.by_size) &&
+                lane == 0)
+                set_error_bits(err, kErrTreeletClimb);
+            __syncwarp();
+            vote &= vote - 1;
+        }
+        if (cur >= 0) cur = ld_cg(g.parent + base + cur);
+    }
+}
+
+int trbvh_tight(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_nodes, int iterations,
+                const uint8_t* seg_iters, float ci, float ct) {
+    const size_t inner = segs.n - segs.count, b4 = align256(total_nodes * 4);
+    void* scratch = nullptr;
+    ATR_TRY(ctx->alloc(&scratch, 2 * b4 + align256(inner * 4)));
+    char* const p = static_cast<char*>(scratch);
+    uint32_t* const counters = reinterpret_cast<uint32_t*>(p + 2 * b4);
+    constexpr int kThreads = kTrWarps * 32;
+    int st = ATR_OK;
+    ctx->phase_begin("trbvh");
+    for (int it = 0; it < iterations && st == ATR_OK; ++it) {
+        st = zero_words_async(ctx, counters, inner);
+        if (st != ATR_OK) break;
+        k_tr_tight<<<(segs.n + kThreads - 1) / kThreads, kThreads, 0, ctx->stream>>>(
+            g, segs, reinterpret_cast<int32_t*>(p), reinterpret_cast<float*>(p + b4), counters, seg_iters, it, ci, ct,
+            ctx->d_error);
+        ctx->launches += 1;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) st = cuda_fail(e, "k_tr_tight launch", __FILE__, __LINE__);
+    }
+    ctx->phase_end();
+    ctx->release(scratch);
+    return st;
+}
+
+// Whether `bytes` of scratch can be had: eagerly the allocation itself tells; a
+// captured one is only made when the graph is instantiated or launched, so the
+// device's free memory decides for it.
+int level_scratch(atr_ctx* ctx, void** p, size_t bytes, bool* fits) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    ATR_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+    *fits = true;
+    if (cap != cudaStreamCaptureStatusNone) {
+        size_t avail = 0, all = 0;
+        ATR_CUDA(cudaMemGetInfo(&avail, &all));
+        *fits = bytes <= avail;
+        return *fits ? ctx->alloc(p, bytes) : ATR_OK;
+    }
+    const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+    if (e == cudaSuccess) return ATR_OK;
+    *p = nullptr;
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
+    cudaGetLastError();
+    *fits = false;
+    return ATR_OK;
+}
+
 }  // namespace
 
 // TRBVH (treelet 7) over every mesh of `segs`; seg_iters optionally gives
@@ -456,7 +584,9 @@ int trbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_no
     const LevelScratch ls(segs.n, kTr, auto_levels(segs.n, kTr));
     const size_t b_rec = align256(total_nodes * 16), b_kid = align256(inner * 16), b_ctr = align256(inner * 4);
     void* scratch = nullptr;
-    ATR_TRY(ctx->alloc(&scratch, b_rec + b_kid + b_ctr + ls.bytes()));
+    bool fits = false;
+    ATR_TRY(level_scratch(ctx, &scratch, b_rec + b_kid + b_ctr + ls.bytes(), &fits));
+    if (!fits) return trbvh_tight(ctx, g, segs, total_nodes, iterations, seg_iters, ci, ct);
     char* p = static_cast<char*>(scratch);
     LevelRefs lv{};
     TopRefs tr{};  // no cluster here

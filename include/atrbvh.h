@@ -225,7 +225,9 @@ int atr_device_sort_pairs(atr_ctx* ctx, void* keys, uint32_t* values, uint32_t c
 int atr_optimize_atrbvh(atr_ctx* ctx, atr_tree* tree, int treelet_size, int iterations,
                         float ci, float ct);
 /* TRBVHOptimizer(treeletSize, iterations)::Optimize
- * (BVHRT-Core/src/TRBVHOptimizer.h:27, .cpp:21-128); treelet size 7. */
+ * (BVHRT-Core/src/TRBVHOptimizer.h:27, .cpp:21-128); treelet size 7.  Takes 75
+ * to 82 bytes of scratch a triangle, or 20 (and more time from 100,000 triangles
+ * on) where the device has no more; the tree is the same. */
 int atr_optimize_trbvh(atr_ctx* ctx, atr_tree* tree, int treelet_size, int iterations,
                        float ci, float ct);
 /* Bottom-up box refit of an existing topology from the scene's current
