@@ -218,6 +218,7 @@ int atr_ctx_set_tuning(atr_ctx* ctx, int knob, int value) {
             ATR_REQUIRE(value >= 0 && value <= 64, ATR_ERR_INVALID_ARG,
                         "atr_ctx_set_tuning: level passes %d outside [0, 64]", value);
             ctx->atr_levels = value;
+            ctx->atr_levels_set = true;
             return ATR_OK;
         case ATR_TUNE_QUAD_MIN:
             ATR_REQUIRE(value >= -1, ATR_ERR_INVALID_ARG, "atr_ctx_set_tuning: quad threshold %d below -1", value);

@@ -1350,9 +1350,11 @@ void launch_level_g(int warps, unsigned blocks, cudaStream_t s, const TreeRefs& 
     }
 }
 
-constexpr int kDefaultLevels = 12;  // atr_ctx::atr_levels unless tuned
-// ATRBVH(9, 2) with the cluster and with the dataflow pass: 1,003 triangles 151
-// and 177 us, 65,536 311 and 321, 1,000,003 921 and 890.
+// ATRBVH(9, 2) by the cluster | by 12 level passes and the dataflow pass, uniform
+// triangles: 1,003 173 | 236 us, 20,011 284 | 322, 65,536 349 | 374, 131,072 410 |
+// 435, 262,144 476 | 486, 524,288 573 | 577, 1,000,003 724 | 720, 4,194,304 1,692 |
+// 1,672.  The two cross between 524,288 and 1,000,003; from the line to there the
+// cluster would be worth another 1 to 3 %.
 constexpr uint32_t kClusterTriangles = 131072;
 
 }  // namespace
@@ -1376,7 +1378,7 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
     // takes the rest; above, and with a number the context asks for, the dataflow
     // pass does, whose climbs advance without waiting for the slowest treelet of a
     // level.
-    const bool cluster = ctx->atr_levels == kDefaultLevels && segs.n <= kClusterTriangles;
+    const bool cluster = !ctx->atr_levels_set && segs.n <= kClusterTriangles;
     auto levels_of = [&](int it) { return cluster ? auto_levels(segs.n, tsize << it) : ctx->atr_levels; };
     const int L0 = levels_of(0);
     void* scratch = nullptr;

@@ -261,7 +261,7 @@ int atr_batch_build(atr_ctx* ctx, atr_batch* b, int optimizer, int treelet_size,
                 iterations);
     if (!use_graph) return batch_run(ctx, b, optimizer, treelet_size, iterations, ci, ct);
     const int key[10] = {optimizer,        treelet_size,       iterations,      b->per_mesh_params ? 1 : 0,
-                         ctx->atr_warps,   ctx->atr_group_min, ctx->sort_bits,  ctx->atr_levels,
+                         ctx->atr_warps,   ctx->atr_group_min, ctx->sort_bits,  ctx->atr_levels_set ? ctx->atr_levels : -1,
                          ctx->atr_quad_min, ctx->atr_warp_max};
     const bool same = b->graph && std::memcmp(key, b->graph_key, sizeof(key)) == 0 && b->graph_cf[0] == ci &&
                       b->graph_cf[1] == ct;

@@ -106,6 +106,7 @@ struct atr_ctx {
     // ATRBVH levels restructured by the level passes (one thread per
     // treelet) before the dataflow pass takes the rest; 0 = dataflow only.
     int atr_levels = 12;
+    bool atr_levels_set = false;  // a number the caller asked for; else small trees follow their size
     // A level pass over at least this many treelet roots restructures them in
     // four-lane groups (eight per warp); -1 = never.
     int atr_quad_min = 20000;

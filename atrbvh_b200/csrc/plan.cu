@@ -52,7 +52,7 @@ void plan_tuning_key(const atr_ctx* ctx, int key[6]) {
     key[0] = ctx->atr_warps;
     key[1] = ctx->atr_group_min;
     key[2] = ctx->sort_bits;
-    key[3] = ctx->atr_levels;
+    key[3] = ctx->atr_levels_set ? ctx->atr_levels : -1;
     key[4] = ctx->atr_quad_min;
     key[5] = ctx->atr_warp_max;
 }

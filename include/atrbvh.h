@@ -113,9 +113,9 @@ int atr_ctx_get_stream(atr_ctx* ctx, void** stream);
  *                           4 passes over 30-bit codes, 8 over 63-bit) or 10
  *                           (3 and 7 passes).
  *   ATR_TUNE_ATR_LEVELS     ATRBVH levels of treelet roots restructured level
- *                           by level in lane groups (0..64; default 12, which
- *                           follows the size up to 131,072 triangles; 0 = all
- *                           by the bottom-up warp pass).
+ *                           by level in lane groups (0..64; 0 = all by the
+ *                           bottom-up warp pass; until a number is set, 12, or
+ *                           by size up to 131,072 triangles).
  *   ATR_TUNE_QUAD_MIN       fewest treelet roots of one level that the level
  *                           pass restructures in four-lane groups, eight per
  *                           warp, instead of 32/G per warp (-1 = never;

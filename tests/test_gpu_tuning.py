@@ -131,3 +131,36 @@ def test_batch_autotune_never_slower_than_defaults(tuned_ctx):
     b.close()
     tuned_ctx.set_tuning(ab.TUNE_ATR_WARPS, warps0)
     tuned_ctx.set_tuning(ab.TUNE_SORT_BITS, bits0)
+
+
+def test_level_passes_asked_for_are_the_ones_run(tuned_ctx):
+    """Until a number is set, small trees follow their size; 12 set means 12, also
+    for a plan captured before."""
+    v = scene_case("u1000")
+    mn, mx = O.scene_aabb(v)
+    want = O.atrbvh(O.build_lbvh(v, mn, mx)[0], 9, 2)
+    scene = ab.SceneWrapper(tuned_ctx, v, mn, mx)
+    plan = ab.BuildPlan(scene, flatten=False)
+
+    def launches():
+        out = []
+        tree = ab.LBVHBuilder().BuildTree(scene)
+        n0 = tuned_ctx.launch_count()
+        ab.AgglomerativeTreeletOptimizer(9, 2).Optimize(tree)
+        out.append(tuned_ctx.launch_count() - n0)
+        assert_trees_equal(ab.BVHTreeInstanceManager().DeviceToHostTree(tree), want, "eager")
+        n0 = tuned_ctx.launch_count()
+        plan.run()
+        out.append(tuned_ctx.launch_count() - n0)
+        tuned_ctx.synchronize()
+        return out
+
+    by_size = launches()
+    assert tuned_ctx.get_tuning(ab.TUNE_ATR_LEVELS) == 12
+    tuned_ctx.set_tuning(ab.TUNE_ATR_LEVELS, 12)
+    twelve = launches()
+    tuned_ctx.set_tuning(ab.TUNE_ATR_LEVELS, 11)
+    eleven = launches()
+    # Two iterations: a launch each less; both have more than the few wide levels.
+    assert [a - b for a, b in zip(twelve, eleven)] == [2, 2]
+    assert all(a > b for a, b in zip(eleven, by_size))
