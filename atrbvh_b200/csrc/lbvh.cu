@@ -1194,6 +1194,9 @@ int build_typed(atr_ctx* ctx, const Segs& segs, uint32_t mesh_tiles, const float
     int32_t* slot = reinterpret_cast<int32_t*>(ap); ap += align256(inner * 4);
     BuildEdge* edges = reinterpret_cast<BuildEdge*>(ap);
     if (one_tile) {
+        // The codes are part of the sort's launch; the phase is reported all the same.
+        ctx->phase_begin("morton");
+        ctx->phase_end();
         ctx->phase_begin("sort");
         k_sort_tile<K><<<tiles, kTileThreads, tile_smem<K>(), s>>>(segs, verts, d_bounds, pr, keys, idx);
         ctx->phase_end();

@@ -137,7 +137,9 @@ int atr_ctx_set_tuning(atr_ctx* ctx, int knob, int value);
 int atr_ctx_get_tuning(atr_ctx* ctx, int knob, int* value);
 /* Number of kernels this context has enqueued since it was created. */
 int atr_ctx_launch_count(atr_ctx* ctx, uint64_t* count);
-/* Per-phase CUDA-event timing of the next builds (milliseconds). */
+/* Per-phase CUDA-event timing of the next builds (milliseconds).  Meshes of at
+ * most 3,072 triangles (a batch of nothing larger) make their codes in the
+ * sort's launch: "morton" is then next to nothing and "sort" holds both. */
 int atr_ctx_set_timing(atr_ctx* ctx, int enable);
 int atr_ctx_phase_times(atr_ctx* ctx, float* ms, int capacity, int* count);
 /* Comma-separated phase names matching the last atr_ctx_phase_times call. */

@@ -34,3 +34,25 @@ def test_plan_phase_times_after_replay(ctx):
     assert ph["flatten"] <= flatten_ms * 1.02 + 0.01
     plan.close()
     scene.close()
+
+
+@pytest.mark.parametrize("case", ["u17", "u1000", "u4097"])
+def test_every_build_reports_the_same_phases(ctx, case):
+    """Also builds whose codes are part of the sort's launch (meshes of one sort tile)."""
+    v = scene_case(case)
+    mn, mx = O.scene_aabb(v)
+    scene = ab.SceneWrapper(ctx, v, mn, mx)
+    plan = ab.BuildPlan(scene, flatten=False)
+    ctx.set_timing(True)
+    try:
+        tree = ab.LBVHBuilder().BuildTree(scene)
+        eager = [name for name, _ in ctx.phase_times()]
+        plan.run(graph=True)
+        captured = [name for name, _ in plan.phase_times()]
+    finally:
+        ctx.set_timing(False)
+    assert eager == ["morton", "sort", "build"]
+    assert captured == ["morton", "sort", "build", "atrbvh", "collapse"]
+    tree.close()
+    plan.close()
+    scene.close()
