@@ -13,7 +13,9 @@
 // Block size (2, 4, 8 warps) and digit width (8, 10 bits) change only the
 // speed, so they are tuned afterwards on the kept pair, checking that the SAH
 // does not move.  Times are CUDA-event medians of `reps` builds after one
-// warm-up build.
+// warm-up build, with the sizes given per mesh, as a table is applied: builds of
+// one size for all meshes have kernels of their own for some sizes (atrbvh.cu),
+// which would win here and then not run.
 
 #include <algorithm>
 #include <cmath>
@@ -77,7 +79,10 @@ int sample_sah(atr_ctx* ctx, const Sample& s, double* out) {
 }
 
 // Median device time of `reps` builds after one warm-up build.
-int time_builds(atr_ctx* ctx, atr_batch* b, int treelet, int iters, uint32_t reps, float* ms) {
+int time_builds(atr_ctx* ctx, const Sample& s, int treelet, int iters, uint32_t reps, float* ms) {
+    atr_batch* const b = s.b;
+    const std::vector<uint8_t> ts(s.off.size() - 1, (uint8_t)treelet), it(s.off.size() - 1, (uint8_t)iters);
+    ATR_TRY(atr_batch_set_params(ctx, b, ts.data(), it.data()));
     ATR_TRY(atr_batch_build(ctx, b, 1, treelet, iters, 1.2f, 1.0f, 0));
     cudaEvent_t e0, e1;
     ATR_CUDA(cudaEventCreate(&e0));
@@ -147,7 +152,7 @@ int atr_autotune(atr_ctx* ctx, const atr_autotune_config* cfg, atr_tune_table* o
         ctx->sort_bits = bits0;
         double sah_ref = 0.0, sah = 0.0;
         float ms_ref = 0.0f;
-        st = time_builds(ctx, s.b, 9, 2, cfg->reps, &ms_ref);
+        st = time_builds(ctx, s, 9, 2, cfg->reps, &ms_ref);
         if (st == ATR_OK) st = sample_sah(ctx, s, &sah_ref);
         int best_t = 9, best_i = 2;
         float best_ms = ms_ref;
@@ -156,7 +161,7 @@ int atr_autotune(atr_ctx* ctx, const atr_autotune_config* cfg, atr_tune_table* o
             for (int it = 1; it <= 3 && st == ATR_OK; ++it) {
                 if (t == 9 && it == 2) continue;
                 float ms = 0.0f;
-                st = time_builds(ctx, s.b, t, it, cfg->reps, &ms);
+                st = time_builds(ctx, s, t, it, cfg->reps, &ms);
                 if (st == ATR_OK) st = sample_sah(ctx, s, &sah);
                 if (st == ATR_OK && sah <= sah_ref * (1.0 + cfg->sah_tolerance) && ms < best_ms) {
                     best_t = t;
@@ -172,7 +177,7 @@ int atr_autotune(atr_ctx* ctx, const atr_autotune_config* cfg, atr_tune_table* o
                 ctx->atr_warps = w;
                 ctx->sort_bits = bits;
                 float ms = 0.0f;
-                st = time_builds(ctx, s.b, best_t, best_i, cfg->reps, &ms);
+                st = time_builds(ctx, s, best_t, best_i, cfg->reps, &ms);
                 if (st == ATR_OK) st = sample_sah(ctx, s, &sah);
                 if (st == ATR_OK && sah != best_sah) {
                     set_error("atr_autotune: SAH changed with launch tuning (class %u)", c);
