@@ -1250,7 +1250,7 @@ void trace_one(const F4* nodes, const F4* woop, const int32_t* tri_index, const 
     const float idy = 1.0f / (fabsf(dy) > ooeps ? dy : copysignf(ooeps, dy));
     const float idz = 1.0f / (fabsf(dz) > ooeps ? dz : copysignf(ooeps, dz));
     const float oodx = ox * idx, oody = oy * idy, oodz = oz * idz;
-    int stack[64];
+    int stack[256];  // layouts of up to 254 levels, as the device takes
     int sp = 0;
     stack[0] = kSentinel;
     int leafAddr = 0, nodeAddr = 0, hitIndex = -1;

@@ -1,7 +1,7 @@
 """Traversal at the ray counts where a launch changes shape: rays per warp
 follow the count (1, 2, 4, ... 32), warps fetch again, launches follow one
-another on the context's ray counter, and layouts are deeper than the part of
-the stack in shared memory."""
+another on the context's ray counter; and at stack depths past the register and
+the 16 entries in shared memory, in both stack sizes and over several meshes."""
 from __future__ import annotations
 
 import numpy as np
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def deep(ctx):
-    """A layout of 30 and more levels: points that close in on a corner, among others."""
+    """A layout of more than 20 levels: points that close in on a corner, among others."""
     v = O.gen_scene(O.SCENE_UNIFORM, 3001, 4)
     k = np.arange(1500)
     v[:1500, :, :3] *= (0.97 ** (k % 150))[:, None, None].astype(np.float32)
@@ -107,3 +107,118 @@ def test_contexts_trace_side_by_side(deep):
     got = res.cpu().numpy()
     for k in range(threads):
         assert np.array_equal(got[k][:, :2], want[:, :2]), k
+
+
+# ---- deep stacks ---------------------------------------------------------------
+# A ray's stack grows while the nearer of two boxes it meets is the larger subtree's.
+
+def _corner(levels: int, copies: int) -> np.ndarray:
+    """Triangles across the first octant whose boxes start at the origin, each
+    about half the one before along one axis: the 63-bit radix tree is a chain with
+    the smaller boxes on the left.  Copies of the smallest lengthen it by their
+    number's logarithm (equal codes)."""
+    half = np.array([[0.75 * 2.0 ** -((k + 2 - a) // 3 + 1) for a in range(3)] for k in range(levels)])
+    half = np.concatenate([half, np.repeat(half[-1:], copies, 0)])
+    v = np.zeros((len(half), 3, 4), np.float32)
+    for a in range(3):
+        v[:, a, a] = 2 * half[:, a]
+    return v
+
+
+def _shrinking(n: int, f: float) -> np.ndarray:
+    """As _corner, each a little smaller: ATRBVH makes long chains of them."""
+    half = 0.5 * (1 + f) ** -np.arange(n, dtype=float)
+    v = np.zeros((n, 3, 4), np.float32)
+    for a in range(3):
+        v[:, a, a] = 2 * half * (1 + 0.1 * a)
+    return v
+
+
+def _rays_out(v: np.ndarray, n: int, seed: int) -> np.ndarray:
+    """Rays that leave from inside the boxes, at the scale of one of the triangles."""
+    rng = np.random.default_rng(seed)
+    size = v[rng.integers(0, len(v), n)][:, [0, 1, 2], [0, 1, 2]]
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, :3] = size * rng.uniform(0.02, 0.3, (n, 3))
+    d = size * rng.uniform(0.05, 1.0, (n, 3))
+    rays[:, 4:7] = d / np.linalg.norm(d, axis=1)[:, None]
+    rays[:, 7] = 1e30
+    return rays
+
+
+def _stack_peak(cp, ray) -> int:
+    """Entries a ray's stack holds at most, the one in the register included."""
+    nodes = cp.nodes.reshape(-1, 16)
+    box = nodes[:, :12].view(np.float32)
+    o, inv = ray[:3].astype(float), 1.0 / ray[4:7].astype(float)
+    stack, peak, at = [], 0, 0
+    while True:
+        if at >= 0:
+            spans = []
+            for k in (0, 1):
+                n = box[at // 4].astype(float)
+                a = (n[[4 * k, 4 * k + 2, 8 + 2 * k]] - o) * inv
+                b = (n[[4 * k + 1, 4 * k + 3, 9 + 2 * k]] - o) * inv
+                spans.append((max(ray[3], np.minimum(a, b).max()), min(ray[7], np.maximum(a, b).min())))
+            order = (1, 0) if spans[1][0] < spans[0][0] else (0, 1)
+            go = [int(nodes[at // 4, 12 + k]) for k in order if spans[k][1] >= spans[k][0]]
+            stack += go[1:]
+            peak = max(peak, len(stack))
+            if go:
+                at = go[0]
+                continue
+        if not stack:
+            return peak
+        at = stack.pop()
+
+
+@pytest.mark.parametrize("levels,copies,depth,peak", [(16, 0, 15, 15), (17, 0, 16, 16), (18, 0, 17, 17), (50, 0, 49, 49),
+                                                      (60, 4, 62, 62), (60, 8, 63, 63), (60, 512, 69, 69)])
+def test_deep_stacks(ctx, levels, copies, depth, peak):
+    """Stacks around the shared-memory entries, and layouts either side of the
+    63 levels that the smaller stack takes."""
+    import torch
+    v = _corner(levels, copies)
+    mn, mx = np.zeros(3, np.float32), np.ones(3, np.float32)
+    scene = ab.SceneWrapper(ctx, v, mn, mx)
+    tree = ab.LBVHBuilder(True).BuildTree(scene)
+    col, _ = ab.BVHTreeCollapser().Collapse(tree, max_leaf=1)
+    bvh = ab.CudaBVH(col, scene)
+    cp = O.flatten(O.collapse(O.build_lbvh(v, mn, mx, bits=63)[0], max_leaf=1), v)
+    assert bvh.view().max_depth == depth
+    n = 5003
+    rays = _rays_out(v, n, levels)
+    assert max(_stack_peak(cp, r) for r in rays[:200]) == peak
+    rd = torch.from_numpy(rays).cuda()
+    for any_hit in (False, True):
+        res = torch.full((n, 4), -7, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        bvh.trace(rd.data_ptr(), n, res.data_ptr(), any_hit=any_hit)
+        ctx.synchronize()
+        assert np.array_equal(res.cpu().numpy()[:, :2], O.trace(cp, rays, any_hit=any_hit)[:, :2]), any_hit
+
+
+def test_deep_stacks_over_several_meshes(ctx):
+    import torch
+    meshes = [_shrinking(400, 0.05), O.gen_scene(O.SCENE_UNIFORM, 300, 3)]
+    off = np.concatenate([[0], np.cumsum([len(v) for v in meshes])]).astype(np.uint32)
+    batch = ab.Batch(ctx, np.concatenate(meshes), off)
+    batch.build(ab.Batch.ATRBVH, 9, 2)
+    batch.collapse(max_leaf=1)
+    batch.flatten()
+    n = 3001
+    rays, want = [], []
+    for k, v in enumerate(meshes):
+        mn, mx = O.scene_aabb(v)
+        cp = O.flatten(O.collapse(O.atrbvh(O.build_lbvh(v, mn, mx)[0], 9, 2), max_leaf=1), v)
+        rays.append(_rays_out(v, n, 5) if k == 0 else ab.gen_rays_random(n, mn, mx, seed=2).reshape(-1, 8))
+        want.append(O.trace(cp, rays[-1]))
+        if k == 0:
+            assert max(_stack_peak(cp, r) for r in rays[0][:100]) > 64
+    assert batch.compact_view(0).max_depth > 63
+    rd = torch.from_numpy(np.concatenate(rays)).cuda()
+    res = torch.full((2 * n, 4), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    batch.trace(rd.data_ptr(), 2 * n, [0, n, 2 * n], [0, 1], res.data_ptr())
+    ctx.synchronize()
+    assert np.array_equal(res.cpu().numpy()[:, :2], np.concatenate(want)[:, :2])
