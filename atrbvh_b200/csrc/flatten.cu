@@ -157,7 +157,8 @@ __global__ void __launch_bounds__(256) k_flat_top(Segs segs, const int4* __restr
     const SegPos q = seg_pos(segs, gi);
     if (q.li >= q.n - 1) return;
     const int x = (int)q.li;
-    if (data[q.nb + x] >= 0) return;  // a collapsed leaf has no step
+    // A collapsed leaf has no step; the root (node 0) has one whatever its data says.
+    if (data[q.nb + x] >= 0 && x != 0) return;
     int4 s = __ldg(step + q.cb + x);
     if (step_inner(s) < kTopInner) return;
     int4 at = make_int4(0, 0, 1, 0);

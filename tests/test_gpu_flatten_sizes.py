@@ -41,3 +41,26 @@ def test_layouts_equal_the_oracle(ctx, max_leaf):
             assert np.array_equal(nodes, want.nodes)
             assert np.array_equal(woop.view(np.int32), want.woop.view(np.int32))
             assert np.array_equal(tri, want.tri_index)
+
+
+class _Words:
+    """A device array of int32 at an address, for torch."""
+
+    def __init__(self, ptr, n):
+        self.__cuda_array_interface__ = {"shape": (n,), "typestr": "<i4", "data": (ptr, False), "version": 2}
+
+
+@pytest.mark.parametrize("n", [100, 1031])
+def test_the_root_is_part_of_the_layout_whatever_its_data_says(ctx, n):
+    """A collapsed tree's arrays are the caller's to write through its view."""
+    import torch
+    v = O.gen_scene(O.SCENE_UNIFORM, n, n)
+    scene = ab.SceneWrapper(ctx, v, *O.scene_aabb(v))
+    tree = ab.LBVHBuilder().BuildTree(scene)
+    col, _ = ab.BVHTreeCollapser().Collapse(tree, max_leaf=4)
+    want = ab.CudaBVH(col, scene).serialize()
+    data = torch.as_tensor(_Words(col.view().data, 2 * n - 1), device="cuda")
+    assert int(data[0]) < 0
+    data[0] = 5
+    torch.cuda.synchronize()
+    assert ab.CudaBVH(col, scene).serialize() == want
