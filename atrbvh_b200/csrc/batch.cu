@@ -52,6 +52,7 @@ struct atr_batch {
     int64_t* d_sizes = nullptr;  // per mesh: nodes then woop entries
     std::vector<int64_t> h_sizes;
     std::atomic<int32_t> max_depth{0};  // refits of different meshes may raise it from several lanes
+    size_t largest_layout = 0;          // bytes of the largest mesh's nodes and Woop entries when last flattened
     bool flattened = false;
     // Parameters of the last atr_batch_collapse (reused when one mesh is refit).
     float col_ci = 1.2f, col_ct = 1.0f;
@@ -401,6 +402,10 @@ int atr_batch_flatten(atr_ctx* ctx, atr_batch* b) {
                              ctx->stream));
     ATR_CUDA(cudaStreamSynchronize(ctx->stream));
     b->max_depth = (int32_t)b->h_sizes[2ull * b->count];
+    b->largest_layout = 0;
+    for (uint32_t m = 0; m < b->count; ++m)
+        b->largest_layout = std::max(b->largest_layout,
+                                     (size_t)b->h_sizes[m] * 64 + (size_t)b->h_sizes[b->count + m] * 16);
     b->flattened = true;
     return ATR_OK;
 }
@@ -454,7 +459,7 @@ int atr_batch_trace(atr_ctx* ctx, const atr_batch* b, const float* rays, int64_t
         return cuda_fail(e, "cudaMemcpyAsync(ray groups)", __FILE__, __LINE__);
     }
     const int st = trace_batch(ctx, b->cp_nodes, b->cp_woop, b->cp_tri, map, map + groups + 1, b->d_tri_off, groups,
-                               b->max_depth, reinterpret_cast<const float4*>(rays), num_rays, any_hit,
+                               b->max_depth, b->largest_layout, reinterpret_cast<const float4*>(rays), num_rays, any_hit,
                                reinterpret_cast<int4*>(results));
     ctx->release(map);
     return st;

@@ -112,7 +112,7 @@ struct atr_ctx {
     int atr_quad_min = 20000;
     int atr_warp_max = 4096;
     int top_ctas = 8;  // cluster size of the ATRBVH top kernel
-    int trace_blocks[2][2] = {{1, 1}, {1, 1}};  // traversal's blocks per SM: [stack of 256][several meshes]
+    int trace_blocks[2][2][2] = {};  // traversal's blocks per SM: [stack of 256][several meshes][far beyond L2]
     struct Phase {
         std::string name;
         cudaEvent_t a, b;
@@ -251,9 +251,9 @@ int flatten_segs(atr_ctx* ctx, const Segs& segs, const CollapsedOut& c, const fl
                  float4* woop, int32_t* tri_index, int64_t* d_sizes);
 struct RayMeshMap;  // trace.cu
 int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
-              int max_depth, const float4* rays, int64_t n, int any_hit, int4* res);
+              int max_depth, size_t layout_bytes, const float4* rays, int64_t n, int any_hit, int4* res);
 int trace_batch(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const uint32_t* ray_off,
-                const uint32_t* group_mesh, const uint32_t* tri_off, uint32_t groups, int max_depth,
+                const uint32_t* group_mesh, const uint32_t* tri_off, uint32_t groups, int max_depth, size_t layout_bytes,
                 const float4* rays, int64_t n, int any_hit, int4* res);
 // Bottom-up box refit of one tree (local indices) from vertices of its mesh.
 int refit_arrays(atr_ctx* ctx, uint32_t n, const TreeOut& t, const float4* verts);

@@ -13,8 +13,8 @@
 // same operations.
 //
 // Warps are persistent: lanes whose ray is done wait until fewer than 20 lanes
-// of the warp have work (the reference's dynamic fetch), then take new rays
-// from a global counter.  Between two fetches the warp steps as one, every step
+// of the warp have work (the reference's dynamic fetch; 16 for the largest
+// layouts), then take new rays from a global counter.  Between two fetches the warp steps as one, every step
 // either a descent or a leaf test, chosen by vote: left to diverge, the lanes
 // of a warp met again only by chance and an instruction served 6.6 of 32 lanes
 // (1M sorted incoherent rays; 8.8 for pinhole rays); voting serves 11 and 13.
@@ -24,6 +24,8 @@
 // each 0.66 -> 0.48 ms (4.2M triangles).  Measured and not kept: 12 or 16 blocks a
 // SM (spills), prefetching the pushed child, fetching at 12 or 28 lanes.
 //
+#include <type_traits>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -43,7 +45,42 @@ struct RayMeshMap {
 namespace {
 
 constexpr int kSentinel = 0x76543210;
-constexpr int kDynamicFetch = 20;
+
+// How a warp steps: lanes with work below which it fetches rays; how many times as
+// many lanes must wait to descend as at leaves for a descent; whether a leaf step
+// runs each lane's leaf to its end.  The near stepping is compiled in (read from
+// arguments it cost up to 0.6 %).
+struct Stepping {
+    int fetch, weight;
+    bool whole_leaf;
+};
+constexpr Stepping kNear = {20, 2, false};
+// By the bytes of the layout's nodes and Woop entries (126 MB of L2).  Far beyond
+// L2 the fetches' misses bound the trace, and more lanes at work lose more than they
+// hide: a leaf's remaining sectors leave the L1 between two of its lane's steps, and
+// rays in flight push each other's nodes out.  8.4M random rays, closest | any hit,
+// ms, by each lane at its own step (as before the vote) / 20, 2, false / 20, 2, true
+// / 16, 1, true:
+//   uniform    62 MB    8.0 / 5.59 / 5.64 / 5.71   | 6.8 / 4.75 / 4.78 / 4.85
+//   uniform   459 MB   13.8 / 10.0 / 9.98 / 9.99   | 7.5 / 5.91 / 5.88 / 5.80
+//   clustered 447 MB    5.6 / 3.46 / 3.44 / 3.75   | 4.7 / 2.80 / 2.82 / 3.04
+//   uniform   679 MB   17.3 / 14.9 / 14.2 / 13.8   | 8.3 / 7.66 / 7.30 / 7.07
+//   clustered 665 MB    6.1 / 4.14 / 4.08 / 4.30   | 4.8 / 3.05 / 3.03 / 3.20
+//   uniform   898 MB   20.9 / 20.0 / 19.2 / 18.2   | 9.2 / 9.38 / 8.93 / 8.51
+//   clustered 875 MB    6.3 / 4.53 / 4.40 / 4.53   | 4.9 / 3.34 / 3.28 / 3.35
+//   uniform  1.33 GB   27.6 / 28.4 / 27.5 / 25.3   | 10.8 / 11.6 / 11.2 / 10.5
+//   clustered 1.28 GB   6.8 / 5.78 / 5.53 / 5.39   | 5.0 / 4.18 / 4.11 / 3.92
+//   uniform  1.77 GB   33.7 / 35.3 / 34.5 / 31.4   | 12.0 / 13.1 / 12.8 / 11.9
+//   uniform  2.63 GB   44.7 / 47.4 / 46.3 / 42.0   | 13.6 / 15.3 / 14.9 / 13.9
+// With at most twice the rays that the GPU holds at once (189,440) rays do not push
+// each other out yet: 16.8M uniform triangles, closest hit of 100,003, 300,007 and
+// 400,009 rays by 20, 2, false / 16, 1, true: 0.80 / 0.79, 1.50 / 1.55, 2.04 / 1.90.
+Stepping stepping(size_t layout_bytes, int64_t rays, int64_t held) {
+    if (rays <= 2 * held) return kNear;
+    if (layout_bytes >= 1100000000) return {16, 1, true};
+    if (layout_bytes >= 600000000) return {20, 2, true};
+    return kNear;
+}
 
 __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
 __device__ __forceinline__ int imax(int a, int b) { return a > b ? a : b; }
@@ -68,15 +105,14 @@ __device__ __forceinline__ void ld32(const float4* p, float4& a, float4& b) {
 
 constexpr int kTraceThreads = 128;
 constexpr int kSharedStack = 16;
-constexpr int kLeafWeight = 2;
 
-template <int kStack, bool kMapped>
+template <int kStack, bool kMapped, bool kFar>
 __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restrict__ nodes_all,
                                                const float4* __restrict__ woop_all,
                                                const int* __restrict__ tri_all, RayMeshMap map,
                                                const float4* __restrict__ rays, int64_t nrays, int any_hit,
                                                int4* __restrict__ results, unsigned long long* __restrict__ counter,
-                                               int lanes, uint32_t* __restrict__ err) {
+                                               int lanes, Stepping far, uint32_t* __restrict__ err) {
     // The stack's top entry is held in a register (top), so a pop does not
     // wait for a load; of the sp entries below it the first kSharedStack are
     // in shared memory (one bank per lane whatever the lanes' depths), the
@@ -86,7 +122,8 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
     const int lane = threadIdx.x & 31;
     if (lane >= lanes) return;
     const unsigned team = lanes == 32 ? kFull : (1u << lanes) - 1u;
-    const int fetch = (kDynamicFetch * lanes + 31) / 32;
+    const Stepping how = kFar ? far : kNear;
+    const int fetch = (how.fetch * lanes + 31) / 32;
     int top = kSentinel;
     float ox = 0, oy = 0, oz = 0, tmin = 0, dx = 0, dy = 0, dz = 0, hitT = 0;
     float idx = 0, idy = 0, idz = 0, oodx = 0, oody = 0, oodz = 0;
@@ -230,21 +267,26 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
         // Steps until fewer than `fetch` lanes have work (or none, once there
         // are no rays to fetch).  A lane either descends or tests its leaf; each
         // warp step is one of the two: descent unless the lanes at leaves are
-        // more than half as many (a leaf step is short and frees its lane).
+        // more than half as many (a leaf step is short and frees its lane), or,
+        // in the largest layouts, more.
         const int enough = more ? fetch : 1;
         while (true) {
             const bool leaf = has && leafAddr < 0;
             const bool inner = has && !leaf && nodeAddr != kSentinel;
             const unsigned bi = __ballot_sync(team, inner), bl = __ballot_sync(team, leaf);
             if (__popc(bi | bl) < enough) break;
-            if (__popc(bi) >= kLeafWeight * __popc(bl)) {
+            if (__popc(bi) >= how.weight * __popc(bl)) {
                 // Two steps a vote: most lanes that descend do so again.
                 if (inner) {
                     node_step();
                     if ((unsigned)nodeAddr < (unsigned)kSentinel && leafAddr >= 0) node_step();
                 }
             } else {
-                if (leaf) leaf_step();
+                if (leaf) {
+                    do leaf_step();
+                    while (kFar && leafAddr < 0);
+                }
+                if constexpr (kFar) __syncwarp(team);
             }
         }
         if (has && nodeAddr == kSentinel && leafAddr >= 0) {
@@ -262,10 +304,10 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
     }
 }
 
-template <int kStack, bool kMapped>
+template <int kStack, bool kMapped, bool kFar>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
-                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter) {
-    const int blocks_per_sm = ctx->trace_blocks[kStack > 64][kMapped];
+                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter, const Stepping& how) {
+    const int blocks_per_sm = ctx->trace_blocks[kStack > 64][kMapped][kFar];
     // Rays per warp: the paths of a warp's rays add up as far as they differ, so
     // few rays are spread over as many warps as run at once (1,000 rays through
     // 20,011 triangles: 57 us at one ray a warp, 93 at 32; 50,000 rays: 103 us at
@@ -277,16 +319,21 @@ void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int
     const int64_t need = (n + W * lanes - 1) / (W * lanes);
     int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
     if (need < grid) grid = need;
-    k_trace<kStack, kMapped><<<(unsigned)grid, kTraceThreads, 0, ctx->stream>>>(
-        reinterpret_cast<const float4*>(nodes), woop, tri, map, rays, n, any_hit, res, counter, lanes, ctx->d_error);
+    k_trace<kStack, kMapped, kFar><<<(unsigned)grid, kTraceThreads, 0, ctx->stream>>>(
+        reinterpret_cast<const float4*>(nodes), woop, tri, map, rays, n, any_hit, res, counter, lanes, how, ctx->d_error);
     ctx->launches += 1;
 }
 
 template <int kStack>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
-                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter) {
-    if (map.groups) launch_trace<kStack, true>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter);
-    else launch_trace<kStack, false>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter);
+                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter, const Stepping& how) {
+    auto run = [&](auto mapped, auto far) {
+        launch_trace<kStack, mapped.value, far.value>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, how);
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    if (map.groups) how.whole_leaf ? run(yes, yes) : run(yes, no);
+    else how.whole_leaf ? run(no, yes) : run(no, no);
 }
 
 // Cosine-weighted diffuse bounce per primary hit (the workload of
@@ -340,21 +387,25 @@ __global__ void __launch_bounds__(256) k_bounce(const float4* __restrict__ verts
 // Blocks of each instance that an SM holds (once per context: contexts launch from
 // threads of their own).
 int trace_prepare(atr_ctx* ctx) {
-    auto set = [&](int deep, int mapped, auto kernel) {
-        int* const b = &ctx->trace_blocks[deep][mapped];
+    auto set = [&](int* b, auto kernel) {
         const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(b, kernel, kTraceThreads, 0);
         if (e != cudaSuccess || *b < 1) *b = 1;
         return e;
     };
-    ATR_CUDA(set(0, 0, k_trace<64, false>));
-    ATR_CUDA(set(0, 1, k_trace<64, true>));
-    ATR_CUDA(set(1, 0, k_trace<256, false>));
-    ATR_CUDA(set(1, 1, k_trace<256, true>));
+    auto& b = ctx->trace_blocks;
+    ATR_CUDA(set(&b[0][0][0], k_trace<64, false, false>));
+    ATR_CUDA(set(&b[0][0][1], k_trace<64, false, true>));
+    ATR_CUDA(set(&b[0][1][0], k_trace<64, true, false>));
+    ATR_CUDA(set(&b[0][1][1], k_trace<64, true, true>));
+    ATR_CUDA(set(&b[1][0][0], k_trace<256, false, false>));
+    ATR_CUDA(set(&b[1][0][1], k_trace<256, false, true>));
+    ATR_CUDA(set(&b[1][1][0], k_trace<256, true, false>));
+    ATR_CUDA(set(&b[1][1][1], k_trace<256, true, true>));
     return ATR_OK;
 }
 
 int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
-              int max_depth, const float4* rays, int64_t n, int any_hit, int4* res) {
+              int max_depth, size_t layout_bytes, const float4* rays, int64_t n, int any_hit, int4* res) {
     if (n == 0) return ATR_OK;
     // The ray counter: the context's own, which every launch on its stream
     // leaves at zero.  A captured trace gets one of its own, since its graph may
@@ -369,9 +420,11 @@ int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t
         counter = own;
     }
     int st = ATR_OK;
+    const Stepping how =
+        stepping(layout_bytes, n, (int64_t)ctx->num_sms * ctx->trace_blocks[0][0][0] * kTraceThreads);
     ctx->phase_begin("trace");
-    if (max_depth + 1 < 64) launch_trace<64>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter);
-    else if (max_depth + 1 < 256) launch_trace<256>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter);
+    if (max_depth + 1 < 64) launch_trace<64>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, how);
+    else if (max_depth + 1 < 256) launch_trace<256>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, how);
     else st = ATR_ERR_UNSUPPORTED;
     ctx->phase_end();
     ctx->release(own);
@@ -384,10 +437,10 @@ int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t
 }
 
 int trace_batch(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const uint32_t* ray_off,
-                const uint32_t* group_mesh, const uint32_t* tri_off, uint32_t groups, int max_depth,
+                const uint32_t* group_mesh, const uint32_t* tri_off, uint32_t groups, int max_depth, size_t layout_bytes,
                 const float4* rays, int64_t n, int any_hit, int4* res) {
     const RayMeshMap map{ray_off, group_mesh, tri_off, groups};
-    return trace_run(ctx, nodes, woop, tri, map, max_depth, rays, n, any_hit, res);
+    return trace_run(ctx, nodes, woop, tri, map, max_depth, layout_bytes, rays, n, any_hit, res);
 }
 
 }  // namespace atr
@@ -400,8 +453,8 @@ int atr_trace(atr_ctx* ctx, const atr_compact* cp, const float* rays, int64_t n,
     ATR_REQUIRE(ctx && cp && rays && results, ATR_ERR_INVALID_ARG, "atr_trace: NULL argument");
     ATR_REQUIRE(n >= 0, ATR_ERR_INVALID_ARG, "atr_trace: negative ray count");
     const RayMeshMap map{nullptr, nullptr, nullptr, 0u};
-    return trace_run(ctx, cp->nodes, cp->woop, cp->tri_index, map, cp->max_depth, reinterpret_cast<const float4*>(rays),
-                     n, any_hit, reinterpret_cast<int4*>(results));
+    return trace_run(ctx, cp->nodes, cp->woop, cp->tri_index, map, cp->max_depth,
+                     (size_t)cp->num_nodes * 64 + (size_t)cp->num_woop * 16, reinterpret_cast<const float4*>(rays), n, any_hit, reinterpret_cast<int4*>(results));
 }
 
 int atr_gen_bounce_rays(atr_ctx* ctx, const atr_scene* scene, const float* rays, const int32_t* results, int64_t n,

@@ -222,3 +222,49 @@ def test_deep_stacks_over_several_meshes(ctx):
     batch.trace(rd.data_ptr(), 2 * n, [0, n, 2 * n], [0, 1], res.data_ptr())
     ctx.synchronize()
     assert np.array_equal(res.cpu().numpy()[:, :2], np.concatenate(want)[:, :2])
+
+
+# ---- layouts far beyond L2 -----------------------------------------------------
+
+@pytest.mark.parametrize("n,least,most", [(6_300_000, 600e6, 1100e6), (11_000_000, 1100e6, 2e9)])
+def test_large_layouts(ctx, n, least, most):
+    """The sizes from which warps step otherwise: on the device's own layout the
+    oracle's traversal finds the same, alone and beside another mesh."""
+    import torch
+    v = ab.gen_scene(ab.SCENE_UNIFORM, n, 5)
+    scene = ab.SceneWrapper(ctx, v)
+    mn, mx = scene.bounds()
+    tree = ab.LBVHBuilder().BuildTree(scene)
+    col, _ = ab.BVHTreeCollapser().Collapse(tree)
+    bvh = ab.CudaBVH(col, scene)
+    col.close()
+    tree.close()
+    view = bvh.view()
+    assert least < view.num_nodes * 64 + view.num_woop * 16 < most
+    # More than twice the rays that 148 SMs hold at once (189,440).
+    rays = ab.gen_rays_random(400_009, mn, mx, seed=8).reshape(-1, 8)
+    cp = O.Compact(*bvh.download())
+    rd = torch.from_numpy(rays).cuda()
+    res = torch.full((len(rays), 4), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    want = {}
+    for any_hit in (False, True):
+        bvh.trace(rd.data_ptr(), len(rays), res.data_ptr(), any_hit=any_hit)
+        ctx.synchronize()
+        want[any_hit] = O.trace(cp, rays, any_hit=any_hit)[:, :2]
+        assert np.array_equal(res.cpu().numpy()[:, :2], want[any_hit]), any_hit
+    bvh.close()
+    scene.close()
+    small = O.gen_scene(O.SCENE_UNIFORM, 300, 3)
+    batch = ab.Batch(ctx, np.concatenate([small, v]), np.array([0, 300, 300 + n], np.uint32))
+    batch.build(ab.Batch.NONE)
+    batch.collapse()
+    batch.flatten()
+    m = len(rays) - 1000
+    batch.trace(rd.data_ptr(), len(rays), [0, m, len(rays)], [1, 0], res.data_ptr())
+    ctx.synchronize()
+    got = res.cpu().numpy()[:, :2]
+    assert np.array_equal(got[:m], want[False][:m])
+    few = O.flatten(O.collapse(O.build_lbvh(small, *O.scene_aabb(small))[0]), small)
+    assert np.array_equal(got[m:], O.trace(few, rays[m:])[:, :2])
+    batch.close()
