@@ -86,9 +86,10 @@ struct atr_ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     uint32_t* d_error = nullptr;  // device error bits
-    // Traversal's ray counter and finished-warp counter, zero between launches
-    // (in d_error's allocation).
+    // Traversal's two ray counters (in d_error's allocation) and which of them the
+    // next launch uses: that one is zero.
     unsigned long long* d_trace = nullptr;
+    int trace_turn = 0;
     // Pinned words that small read-backs and the error word are copied to, so
     // that one stream synchronisation covers them.
     static constexpr size_t kStage = 256;

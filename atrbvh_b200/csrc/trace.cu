@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
                                                const int* __restrict__ tri_all, RayMeshMap map,
                                                const float4* __restrict__ rays, int64_t nrays, int any_hit,
                                                int4* __restrict__ results, unsigned long long* __restrict__ counter,
+                                               unsigned long long* __restrict__ other,
                                                int lanes, Stepping far, uint32_t* __restrict__ err) {
     // The stack's top entry is held in a register (top), so a pop does not
     // wait for a load; of the sp entries below it the first kSharedStack are
@@ -119,6 +120,9 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
     // rest in local memory (16 entries take 5 % off incoherent rays; 4 or 8 less).
     __shared__ int s_stack[kSharedStack][kTraceThreads];
     int stack[kStack > kSharedStack ? kStack - kSharedStack : 1];
+    // The launch before this one, which used the other counter, is done; the next
+    // one starts from it.
+    if (other && blockIdx.x == 0 && threadIdx.x == 0) *other = 0ull;
     const int lane = threadIdx.x & 31;
     if (lane >= lanes) return;
     const unsigned team = lanes == 32 ? kFull : (1u << lanes) - 1u;
@@ -297,16 +301,12 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
         }
         if (!more && !__any_sync(team, has)) break;
     }
-    // The last warp leaves both counters at zero for the next launch.
-    if (lane == 0 && atomicAdd(counter + 1, 1ull) == (unsigned long long)gridDim.x * (kTraceThreads / 32) - 1ull) {
-        counter[0] = 0ull;
-        counter[1] = 0ull;
-    }
 }
 
 template <int kStack, bool kMapped, bool kFar>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
-                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter, const Stepping& how) {
+                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter,
+                  unsigned long long* other, const Stepping& how) {
     const int blocks_per_sm = ctx->trace_blocks[kStack > 64][kMapped][kFar];
     // Rays per warp: the paths of a warp's rays add up as far as they differ, so
     // few rays are spread over as many warps as run at once (1,000 rays through
@@ -320,15 +320,17 @@ void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int
     int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
     if (need < grid) grid = need;
     k_trace<kStack, kMapped, kFar><<<(unsigned)grid, kTraceThreads, 0, ctx->stream>>>(
-        reinterpret_cast<const float4*>(nodes), woop, tri, map, rays, n, any_hit, res, counter, lanes, how, ctx->d_error);
+        reinterpret_cast<const float4*>(nodes), woop, tri, map, rays, n, any_hit, res, counter, other, lanes, how,
+        ctx->d_error);
     ctx->launches += 1;
 }
 
 template <int kStack>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
-                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter, const Stepping& how) {
+                  const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter,
+                  unsigned long long* other, const Stepping& how) {
     auto run = [&](auto mapped, auto far) {
-        launch_trace<kStack, mapped.value, far.value>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, how);
+        launch_trace<kStack, mapped.value, far.value>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how);
     };
     const std::true_type yes;
     const std::false_type no;
@@ -407,24 +409,27 @@ int trace_prepare(atr_ctx* ctx) {
 int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
               int max_depth, size_t layout_bytes, const float4* rays, int64_t n, int any_hit, int4* res) {
     if (n == 0) return ATR_OK;
-    // The ray counter: the context's own, which every launch on its stream
-    // leaves at zero.  A captured trace gets one of its own, since its graph may
-    // run on any stream beside others.
-    unsigned long long* counter = ctx->d_trace;
+    // The ray counter: one of the context's two, used in turn; the launch that uses
+    // one clears the other for the next (a count of finished warps that let the last
+    // one clear a single counter cost 4 us a launch).  A captured trace gets one of
+    // its own, since its graph may run on any stream beside others.
+    unsigned long long* counter = ctx->d_trace + ctx->trace_turn;
+    unsigned long long* other = ctx->d_trace + (ctx->trace_turn ^ 1);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     ATR_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
     unsigned long long* own = nullptr;
     if (cap != cudaStreamCaptureStatusNone) {
-        ATR_TRY(ctx->alloc(reinterpret_cast<void**>(&own), 16));
-        cudaMemsetAsync(own, 0, 16, ctx->stream);
+        ATR_TRY(ctx->alloc(reinterpret_cast<void**>(&own), 8));
+        cudaMemsetAsync(own, 0, 8, ctx->stream);
         counter = own;
+        other = nullptr;
     }
     int st = ATR_OK;
     const Stepping how =
         stepping(layout_bytes, n, (int64_t)ctx->num_sms * ctx->trace_blocks[0][0][0] * kTraceThreads);
     ctx->phase_begin("trace");
-    if (max_depth + 1 < 64) launch_trace<64>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, how);
-    else if (max_depth + 1 < 256) launch_trace<256>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, how);
+    if (max_depth + 1 < 64) launch_trace<64>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how);
+    else if (max_depth + 1 < 256) launch_trace<256>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how);
     else st = ATR_ERR_UNSUPPORTED;
     ctx->phase_end();
     ctx->release(own);
@@ -432,7 +437,13 @@ int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t
         set_error("trace: layout depth %d exceeds the traversal stack", max_depth);
         return st;
     }
-    ATR_CUDA(cudaGetLastError());
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        // Whether this launch ran or not, both counters are zero behind it.
+        if (!own) cudaMemsetAsync(ctx->d_trace, 0, 16, ctx->stream);
+        return cuda_fail(e, "k_trace launch", __FILE__, __LINE__);
+    }
+    if (!own) ctx->trace_turn ^= 1;  // the launch uses up its counter and clears the other
     return ATR_OK;
 }
 
