@@ -306,16 +306,19 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
 template <int kStack, bool kMapped, bool kFar>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
                   const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter,
-                  unsigned long long* other, const Stepping& how) {
+                  unsigned long long* other, const Stepping& how, size_t layout_bytes) {
     const int blocks_per_sm = ctx->trace_blocks[kStack > 64][kMapped][kFar];
     // Rays per warp: the paths of a warp's rays add up as far as they differ, so
     // few rays are spread over as many warps as run at once (1,000 rays through
     // 20,011 triangles: 57 us at one ray a warp, 93 at 32; 50,000 rays: 103 us at
-    // 32 or 16, 117 at 8).
+    // 32 or 16, 117 at 8).  Not over a handful of triangles, whose paths are a few
+    // steps and end together (3,072 and 76,800 rays over 12: 12.3 and 14.8 us
+    // spread, 10.4 and 12.6 at 32; random rays over 100 already gain from it).
+    constexpr size_t kFewSteps = 4096;  // bytes of nodes and Woop entries
     constexpr int W = kTraceThreads / 32;
     const int64_t warps = (int64_t)ctx->num_sms * blocks_per_sm * W;
     int lanes = 32;
-    while (lanes > 1 && n <= warps * (lanes / 2)) lanes /= 2;
+    while (layout_bytes > kFewSteps && lanes > 1 && n <= warps * (lanes / 2)) lanes /= 2;
     const int64_t need = (n + W * lanes - 1) / (W * lanes);
     int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
     if (need < grid) grid = need;
@@ -328,9 +331,10 @@ void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int
 template <int kStack>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
                   const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter,
-                  unsigned long long* other, const Stepping& how) {
+                  unsigned long long* other, const Stepping& how, size_t layout_bytes) {
     auto run = [&](auto mapped, auto far) {
-        launch_trace<kStack, mapped.value, far.value>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how);
+        launch_trace<kStack, mapped.value, far.value>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how,
+                                                      layout_bytes);
     };
     const std::true_type yes;
     const std::false_type no;
@@ -428,8 +432,10 @@ int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t
     const Stepping how =
         stepping(layout_bytes, n, (int64_t)ctx->num_sms * ctx->trace_blocks[0][0][0] * kTraceThreads);
     ctx->phase_begin("trace");
-    if (max_depth + 1 < 64) launch_trace<64>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how);
-    else if (max_depth + 1 < 256) launch_trace<256>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how);
+    if (max_depth + 1 < 64)
+        launch_trace<64>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how, layout_bytes);
+    else if (max_depth + 1 < 256)
+        launch_trace<256>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how, layout_bytes);
     else st = ATR_ERR_UNSUPPORTED;
     ctx->phase_end();
     ctx->release(own);
