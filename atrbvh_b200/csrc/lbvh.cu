@@ -22,18 +22,17 @@ namespace atr {
 namespace {
 
 constexpr int kSortThreads = 256;
-// Keys per thread, hence per tile.  Batches use kSortItems; a single sort that
-// fits kTilesWanted tiles (one prefix chunk) of 3 or 6 keys a thread uses those
-// (sort_items): with fewer tiles than the GPU holds at once, a pass costs one
-// block's chain of ranking rounds, which is shorter in smaller tiles.  Codes and
-// sort of 65,536 triangles 65 -> 46 us; past one chunk the prefixes take back
-// what the ranking saves (1,000,003 63-bit keys: 238 us at 12, 252 at 6).
+// Keys per thread, hence per tile.  Batches use kSortItems; a single sort of one
+// prefix chunk uses 3 or 6 (sort_items): with fewer tiles than the GPU holds at
+// once, a pass costs one block's chain of ranking rounds, which is shorter in
+// smaller tiles, until there are too many.  Codes and sort at 3 | 6 | 12 keys, us,
+// 30- and 63-bit: 65,536 70 | 73 | 85, 131 | 141 | 162; 131,072 72 | 74 | 85, 148 |
+// 141 | 170; 196,608 80 | 75 | 88, 156 | 143 | 169; 360,448 100 | 87 | 91, 205 | 168 |
+// 173; 393,216 108 | 92 | 93, 210 | 176 | 173.  Past one chunk the prefixes take back
+// what the ranking saves (1,000,003 63-bit keys: 238 at 12, 252 at 6).
 constexpr int kSortItems = 12;
 constexpr int kSortTile = kSortThreads * kSortItems;
-constexpr uint32_t kTilesWanted = 256;
-inline int sort_items(uint32_t n) {
-    return n <= kTilesWanted * kSortThreads * 3 ? 3 : n <= kTilesWanted * kSortThreads * 6 ? 6 : kSortItems;
-}
+inline int sort_items(uint32_t n) { return n <= 131072 ? 3 : n <= 360448 ? 6 : kSortItems; }
 template <class F>
 auto with_items(int items, F f) {
     if (items == 3) return f(std::integral_constant<int, 3>{});
@@ -376,10 +375,13 @@ __global__ void __launch_bounds__(kSortThreads) k_word_counts(uint32_t n, WordPa
 // tile whose mesh began before its chunk.
 //
 // FOLD: block x walks all the chunks of its 32 digits instead, carrying the
-// sums along, so the counts come out whole and no carry pass follows; used up to
-// kFoldChunks chunks (a chunk takes the walk about 1 us, k_chunk_carry and its
-// launch 4.5 us), and by the word passes, which take each digit's total from here.
-constexpr uint32_t kFoldChunks = 4;
+// sums along, so the counts come out whole and no carry pass follows; used for
+// kFoldChunks chunks, and by the word passes, which take each digit's total from
+// here.  Codes and sort, us, walked | with k_chunk_carry (30-bit; 63-bit): one chunk
+// has no carry pass either way, 163,840 triangles 77 | 74 (155 | 148); two, 786,433
+// 125 | 133 (233 | 249); three, 2,000,003 203 | 198 (396 | 383); four, 3,145,728 262 |
+// 248 (510 | 481).
+constexpr uint32_t kFoldChunks = 2;
 constexpr int kPrefixRuns = 32;
 constexpr int kPrefixRunTiles = 8;
 constexpr uint32_t kPrefixChunk = kPrefixRuns * kPrefixRunTiles;
@@ -1121,7 +1123,7 @@ int sort_pairs(atr_ctx* ctx, const Segs& segs, uint32_t tiles, int items, K** ke
             });
             ctx->launches += 1;
         }
-        if (chunks <= kFoldChunks)
+        if (chunks == kFoldChunks)
             k_tile_prefix<D, true><<<D / 32, 32 * kPrefixRuns, 0, s>>>(segs, tiles, counts, chunk_tot, WordPass{});
         else
             k_tile_prefix<D, false><<<prefix_grid, 32 * kPrefixRuns, 0, s>>>(segs, tiles, counts, chunk_tot,

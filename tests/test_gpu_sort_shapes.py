@@ -26,11 +26,18 @@ def _check_keys(ctx, v, bits):
     scene.close()
 
 
-# One tile (3,072), then tiles of 768, 1,536 and 3,072 keys: at most 256 of the
-# smaller ones; 12 keys a thread fold up to four chunks of 256 tiles.
+# One tile (3,072), then tiles of 768, 1,536 and 3,072 keys; two chunks of 256
+# tiles are walked by the prefixes.
 @pytest.mark.parametrize("bits", [30, 63])
 @pytest.mark.parametrize("n", [2, 31, 3071, 3072, 3073, 196608, 196609, 393216, 393217, 786433])
 def test_lbvh_order_at_tile_boundaries(ctx, n, bits):
+    _check_keys(ctx, O.gen_scene(O.SCENE_CLUSTERED if n % 2 else O.SCENE_UNIFORM, n, n), bits)
+
+
+# Where tiles grow to 1,536 and 3,072 keys, and three chunks: carried.
+@pytest.mark.parametrize("bits", [30, 63])
+@pytest.mark.parametrize("n", [131072, 131073, 360448, 360449, 1572864, 1572865])
+def test_lbvh_order_where_tiles_and_prefixes_change(ctx, n, bits):
     _check_keys(ctx, O.gen_scene(O.SCENE_CLUSTERED if n % 2 else O.SCENE_UNIFORM, n, n), bits)
 
 
