@@ -462,9 +462,11 @@ __global__ void __launch_bounds__(kTrWarps * 32) k_trbvh(TreeRefs g, Segs segs, 
 
 // One climb that restructures treelets as its warps reach them, for trees whose
 // level passes find no memory: 20 bytes of scratch a triangle (counts and nodesSah
-// per node, arrivals) in place of 75 to 82.  Level passes | this, 3 iterations:
-// 20,011 triangles 456 | 499 us, 100,003 615 | 623, 1,000,003 1,783 | 2,716, 16.8M
-// 22.1 | 39.7 ms.
+// per node, arrivals) in place of 75 to 82; and for trees of a few treelets, where
+// it is one launch an iteration in place of the passes'.  Level passes | this, 3
+// iterations, us: 2 triangles 76 | 28, 10 103 | 63, 50 148 | 118, 100 191 | 173, 150
+// 180 | 200, 300 214 | 226, 20,011 456 | 499, 100,003 615 | 623, 1,000,003 1,783 |
+// 2,716, 16.8M 22,100 | 39,700.
 __global__ void __launch_bounds__(kTrWarps * 32) k_tr_tight(TreeRefs g, Segs segs, int32_t* __restrict__ counts,
                                                             float* __restrict__ nsah, uint32_t* __restrict__ counters,
                                                             const uint8_t* __restrict__ seg_iters, int iteration,
@@ -526,6 +528,8 @@ __global__ void __launch_bounds__(kTrWarps * 32) k_tr_tight(TreeRefs g, Segs seg
     }
 }
 
+constexpr uint32_t kTightTriangles = 128;  // up to these the climb is the faster
+
 int trbvh_tight(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_nodes, int iterations,
                 const uint8_t* seg_iters, float ci, float ct) {
     const size_t inner = segs.n - segs.count, b4 = align256(total_nodes * 4);
@@ -580,6 +584,7 @@ int level_scratch(atr_ctx* ctx, void** p, size_t bytes, bool* fits) {
 int trbvh_run(atr_ctx* ctx, const TreeRefs& g, const Segs& segs, size_t total_nodes, int iterations,
               const uint8_t* seg_iters, float ci, float ct, const int2* karras_ranges) {
     if (iterations <= 0) return ATR_OK;
+    if (segs.n <= kTightTriangles) return trbvh_tight(ctx, g, segs, total_nodes, iterations, seg_iters, ci, ct);
     const size_t inner = segs.n - segs.count;
     const LevelScratch ls(segs.n, kTr, auto_levels(segs.n, kTr));
     const size_t b_rec = align256(total_nodes * 16), b_kid = align256(inner * 16), b_ctr = align256(inner * 4);

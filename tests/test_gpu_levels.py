@@ -78,6 +78,20 @@ def test_sizes(ctx, n):
         scene.close()
 
 
+@pytest.mark.parametrize("n", [2, 13, 127, 128, 129])
+def test_small_trees_by_one_climb(ctx, n):
+    """TRBVH of up to 128 triangles takes one climb an iteration."""
+    v = O.gen_scene(O.SCENE_UNIFORM, n, n)
+    mn, mx = O.scene_aabb(v)
+    scene = ab.SceneWrapper(ctx, v, mn, mx)
+    tree = ab.LBVHBuilder().BuildTree(scene)
+    before = ctx.launch_count()
+    ab.TRBVHOptimizer(7, 3).Optimize(tree)
+    assert (ctx.launch_count() - before <= 6) == (n <= 128)
+    ctx.synchronize()
+    _same(ab.BVHTreeInstanceManager().DeviceToHostTree(tree), O.trbvh(O.build_lbvh(v, mn, mx)[0], 7, 3), n)
+
+
 def test_nan_areas_do_not_hang_trbvh(ctx):
     """A triangle with an infinite vertex and a flat axis has a NaN area."""
     v = O.gen_scene(O.SCENE_UNIFORM, 300, 5)
