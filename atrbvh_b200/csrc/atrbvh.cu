@@ -889,7 +889,8 @@ constexpr int kQuadLeaves = 10;  // largest treelet the quad path takes
 // so a lane's reads of areas and distances are in flight together.  The passes
 // are bound by shared-memory wavefronts (71 % of peak on the first level of
 // 4,194,304 triangles), their latency and issue: ATRBVH(9, 2) of 4,194,304
-// triangles 1,889 -> 1,819 us, of 16,777,216 5,464 -> 5,253 against TS = 0.
+// triangles 1,889 -> 1,819 us, of 16,777,216 5,464 -> 5,253 against TS = 0;
+// (5, 2) and (7, 2) of 4,194,304 uniform ones 2,293 -> 2,167 and 2,342 -> 2,267.
 // Measured and not kept: the merge steps unrolled too (5,535 at 16,777,216:
 // instruction fetch), the groups' slots interleaved over the banks (5,750 and
 // more: lanes of a group then share four banks), distances read ahead of their
@@ -1463,7 +1464,7 @@ int atrbvh_run(atr_ctx* ctx, const TreeRefs& g_in, const Segs& segs, size_t tota
                 const bool quads = max_ts <= kQuadLeaves && ctx->atr_quad_min >= 0 && expect >= ctx->atr_quad_min;
                 const bool whole = !quads && max_ts <= kRegTreelet && expect <= (double)ctx->atr_warp_max;
                 if (quads) {
-                    // Sizes of the autotuner's range that have a kernel of their own.
+                    // Sizes that have a kernel of their own, where all meshes share one.
                     const int ts = seg_tsize || warps != 8 ? 0 : tsize;
                     switch (ts) {
                         case 5: k_level_groups<8, 8, true, 5><<<lg, 256, 0, st>>>(g, segs, lv, lev, tsize, nullptr, it, ci, ctx->d_error); break;
