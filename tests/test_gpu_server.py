@@ -191,8 +191,9 @@ def _submit_all(srv, reqs, outs):
     return stamps, [srv.wait(t) for t in tickets]
 
 
-def _joining(n=400000, refits=3):
-    """A build that lasts and, at once, refits of its mesh: one without rays."""
+def _joining(n=1_200_000, refits=3):
+    """A build that lasts (several ms, for the submissions behind it) and, at once,
+    refits of its mesh: one without rays."""
     v = _mesh(n, 21)
     none = np.zeros((0, 8), np.float32)
     reqs = [(ab.REQ_BUILD, 5, v, _rays(v, 6000, 1))]
@@ -234,7 +235,7 @@ def test_server_builds_do_not_wait_for_refits_that_join():
     srv.close()
     assert res[0]["batch_requests"] == len(reqs)
     done = [s + r["latency_ms"] / 1e3 for s, r in zip(stamps, res)]
-    # Seven refits stage 19 MB each, copy it and refit 400,000 triangles.
+    # Seven refits stage 58 MB each, copy it and refit 1,200,000 triangles.
     assert min(done[1:]) - done[0] > 1e-3, [r["latency_ms"] for r in res]
 
 
@@ -254,7 +255,7 @@ def test_server_join_ends_at_the_batch_limit():
 
 def test_server_refits_wait_for_every_build_of_their_mesh():
     """Build, refit, build, refit of one id at once: both refits are of the second build."""
-    a, b = _mesh(300000, 31), _mesh(300000, 32)
+    a, b = _mesh(800000, 31), _mesh(800000, 32)
     r = _rays(a, 5000, 4)
     reqs = [(ab.REQ_BUILD, 9, a, r), (ab.REQ_REFIT, 9, _jitter(b, 1), r),
             (ab.REQ_BUILD, 9, b, r), (ab.REQ_REFIT, 9, _jitter(b, 2), r)]
