@@ -113,7 +113,7 @@ struct atr_ctx {
     int atr_quad_min = 20000;
     int atr_warp_max = 4096;
     int top_ctas = 8;  // cluster size of the ATRBVH top kernel
-    int trace_blocks[2][2][2] = {};  // traversal's blocks per SM: [stack of 256][several meshes][far beyond L2]
+    int trace_blocks[2][2][3] = {};  // traversal's blocks per SM: [stack of 256][several meshes][variant]
     struct Phase {
         std::string name;
         cudaEvent_t a, b;

@@ -47,20 +47,24 @@ namespace {
 constexpr int kSentinel = 0x76543210;
 
 // How a warp steps: lanes with work below which it fetches rays; how many times as
-// many lanes must wait to descend as at leaves for a descent; whether a leaf step
-// runs each lane's leaf to its end.  The near stepping is compiled in (read from
-// arguments it cost up to 0.6 %).
+// many lanes must wait to descend as at leaves for a descent; and the kernel's
+// variant.  kNear's figures are compiled in (read from arguments they cost up to
+// 0.6 %).  kFar: a leaf step runs each lane's leaf to its end.  kClose: as kNear, but
+// while a warp's rays have one origin (a camera's) it fetches below 8 lanes: their
+// paths are short and end together, and a fetch takes as long as several steps.
+enum Variant { kNear = 0, kFar = 1, kClose = 2 };
 struct Stepping {
+    Variant variant;
     int fetch, weight;
-    bool whole_leaf;
 };
-constexpr Stepping kNear = {20, 2, false};
+constexpr Stepping kNearSteps = {kNear, 20, 2};
+constexpr int kCameraFetch = 8;
 // By the bytes of the layout's nodes and Woop entries (126 MB of L2).  Far beyond
 // L2 the fetches' misses bound the trace, and more lanes at work lose more than they
 // hide: a leaf's remaining sectors leave the L1 between two of its lane's steps, and
 // rays in flight push each other's nodes out.  8.4M random rays, closest | any hit,
-// ms, by each lane at its own step (as before the vote) / 20, 2, false / 20, 2, true
-// / 16, 1, true:
+// ms, by each lane at its own step (as before the vote) / kNear / kFar, 20, 2 / kFar,
+// 16, 1:
 //   uniform    62 MB    8.0 / 5.59 / 5.64 / 5.71   | 6.8 / 4.75 / 4.78 / 4.85
 //   uniform   459 MB   13.8 / 10.0 / 9.98 / 9.99   | 7.5 / 5.91 / 5.88 / 5.80
 //   clustered 447 MB    5.6 / 3.46 / 3.44 / 3.75   | 4.7 / 2.80 / 2.82 / 3.04
@@ -74,12 +78,17 @@ constexpr Stepping kNear = {20, 2, false};
 //   uniform  2.63 GB   44.7 / 47.4 / 46.3 / 42.0   | 13.6 / 15.3 / 14.9 / 13.9
 // With at most twice the rays that the GPU holds at once (189,440) rays do not push
 // each other out yet: 16.8M uniform triangles, closest hit of 100,003, 300,007 and
-// 400,009 rays by 20, 2, false / 16, 1, true: 0.80 / 0.79, 1.50 / 1.55, 2.04 / 1.90.
+// 400,009 rays by kNear / kFar, 16, 1: 0.80 / 0.79, 1.50 / 1.55, 2.04 / 1.90.
+// In layouts of up to 4 MB a camera's rays end early: 8.3M pinhole rays, us, kNear /
+// kClose: 1,000 uniform triangles (0.1 MB) 246 / 231, clustered 10,007 (1.2 MB) 282 /
+// 262, 30,011 (3.6 MB) 356 / 332; beyond, clustered 65,536 (7.7 MB) 452 / 414 but
+// uniform 811 / 843.
 Stepping stepping(size_t layout_bytes, int64_t rays, int64_t held) {
-    if (rays <= 2 * held) return kNear;
-    if (layout_bytes >= 1100000000) return {16, 1, true};
-    if (layout_bytes >= 600000000) return {20, 2, true};
-    return kNear;
+    if (layout_bytes <= 4000000 && rays > held) return {kClose, 20, 2};  // else every warp fetches once
+    if (rays <= 2 * held) return kNearSteps;
+    if (layout_bytes >= 1100000000) return {kFar, 16, 1};
+    if (layout_bytes >= 600000000) return {kFar, 20, 2};
+    return kNearSteps;
 }
 
 __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
@@ -106,7 +115,7 @@ __device__ __forceinline__ void ld32(const float4* p, float4& a, float4& b) {
 constexpr int kTraceThreads = 128;
 constexpr int kSharedStack = 16;
 
-template <int kStack, bool kMapped, bool kFar>
+template <int kStack, bool kMapped, Variant kVariant>
 __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restrict__ nodes_all,
                                                const float4* __restrict__ woop_all,
                                                const int* __restrict__ tri_all, RayMeshMap map,
@@ -126,7 +135,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
     const int lane = threadIdx.x & 31;
     if (lane >= lanes) return;
     const unsigned team = lanes == 32 ? kFull : (1u << lanes) - 1u;
-    const Stepping how = kFar ? far : kNear;
+    const Stepping how = kVariant == kFar ? far : kNearSteps;
     const int fetch = (how.fetch * lanes + 31) / 32;
     int top = kSentinel;
     float ox = 0, oy = 0, oz = 0, tmin = 0, dx = 0, dy = 0, dz = 0, hitT = 0;
@@ -273,7 +282,13 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
         // warp step is one of the two: descent unless the lanes at leaves are
         // more than half as many (a leaf step is short and frees its lane), or,
         // in the largest layouts, more.
-        const int enough = more ? fetch : 1;
+        int enough = more ? fetch : 1;
+        if constexpr (kVariant == kClose) {
+            // One origin, but for chance: only the schedule depends on it.
+            const unsigned from = __float_as_uint(ox) ^ 31u * __float_as_uint(oy) ^ 961u * __float_as_uint(oz);
+            const unsigned first = __shfl_sync(team, from, 0);
+            if (__all_sync(team, !has || from == first) && more) enough = (kCameraFetch * lanes + 31) / 32;
+        }
         while (true) {
             const bool leaf = has && leafAddr < 0;
             const bool inner = has && !leaf && nodeAddr != kSentinel;
@@ -288,9 +303,9 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
             } else {
                 if (leaf) {
                     do leaf_step();
-                    while (kFar && leafAddr < 0);
+                    while (kVariant == kFar && leafAddr < 0);
                 }
-                if constexpr (kFar) __syncwarp(team);
+                if constexpr (kVariant == kFar) __syncwarp(team);
             }
         }
         if (has && nodeAddr == kSentinel && leafAddr >= 0) {
@@ -303,11 +318,11 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const float4* __restric
     }
 }
 
-template <int kStack, bool kMapped, bool kFar>
+template <int kStack, bool kMapped, Variant kVariant>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
                   const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter,
                   unsigned long long* other, const Stepping& how, size_t layout_bytes) {
-    const int blocks_per_sm = ctx->trace_blocks[kStack > 64][kMapped][kFar];
+    const int blocks_per_sm = ctx->trace_blocks[kStack > 64][kMapped][kVariant];
     // Rays per warp: the paths of a warp's rays add up as far as they differ, so
     // few rays are spread over as many warps as run at once (1,000 rays through
     // 20,011 triangles: 57 us at one ray a warp, 93 at 32; 50,000 rays: 103 us at
@@ -322,7 +337,7 @@ void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int
     const int64_t need = (n + W * lanes - 1) / (W * lanes);
     int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
     if (need < grid) grid = need;
-    k_trace<kStack, kMapped, kFar><<<(unsigned)grid, kTraceThreads, 0, ctx->stream>>>(
+    k_trace<kStack, kMapped, kVariant><<<(unsigned)grid, kTraceThreads, 0, ctx->stream>>>(
         reinterpret_cast<const float4*>(nodes), woop, tri, map, rays, n, any_hit, res, counter, other, lanes, how,
         ctx->d_error);
     ctx->launches += 1;
@@ -332,14 +347,19 @@ template <int kStack>
 void launch_trace(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t* tri, const RayMeshMap& map,
                   const float4* rays, int64_t n, int any_hit, int4* res, unsigned long long* counter,
                   unsigned long long* other, const Stepping& how, size_t layout_bytes) {
-    auto run = [&](auto mapped, auto far) {
-        launch_trace<kStack, mapped.value, far.value>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how,
-                                                      layout_bytes);
+    auto run = [&](auto mapped, auto variant) {
+        launch_trace<kStack, mapped.value, variant.value>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter,
+                                                          other, how, layout_bytes);
     };
-    const std::true_type yes;
-    const std::false_type no;
-    if (map.groups) how.whole_leaf ? run(yes, yes) : run(yes, no);
-    else how.whole_leaf ? run(no, yes) : run(no, no);
+    auto by_variant = [&](auto mapped) {
+        switch (how.variant) {
+            case kNear: run(mapped, std::integral_constant<Variant, kNear>{}); break;
+            case kFar: run(mapped, std::integral_constant<Variant, kFar>{}); break;
+            case kClose: run(mapped, std::integral_constant<Variant, kClose>{}); break;
+        }
+    };
+    if (map.groups) by_variant(std::true_type{});
+    else by_variant(std::false_type{});
 }
 
 // Cosine-weighted diffuse bounce per primary hit (the workload of
@@ -399,14 +419,18 @@ int trace_prepare(atr_ctx* ctx) {
         return e;
     };
     auto& b = ctx->trace_blocks;
-    ATR_CUDA(set(&b[0][0][0], k_trace<64, false, false>));
-    ATR_CUDA(set(&b[0][0][1], k_trace<64, false, true>));
-    ATR_CUDA(set(&b[0][1][0], k_trace<64, true, false>));
-    ATR_CUDA(set(&b[0][1][1], k_trace<64, true, true>));
-    ATR_CUDA(set(&b[1][0][0], k_trace<256, false, false>));
-    ATR_CUDA(set(&b[1][0][1], k_trace<256, false, true>));
-    ATR_CUDA(set(&b[1][1][0], k_trace<256, true, false>));
-    ATR_CUDA(set(&b[1][1][1], k_trace<256, true, true>));
+    ATR_CUDA(set(&b[0][0][kNear], k_trace<64, false, kNear>));
+    ATR_CUDA(set(&b[0][0][kFar], k_trace<64, false, kFar>));
+    ATR_CUDA(set(&b[0][0][kClose], k_trace<64, false, kClose>));
+    ATR_CUDA(set(&b[0][1][kNear], k_trace<64, true, kNear>));
+    ATR_CUDA(set(&b[0][1][kFar], k_trace<64, true, kFar>));
+    ATR_CUDA(set(&b[0][1][kClose], k_trace<64, true, kClose>));
+    ATR_CUDA(set(&b[1][0][kNear], k_trace<256, false, kNear>));
+    ATR_CUDA(set(&b[1][0][kFar], k_trace<256, false, kFar>));
+    ATR_CUDA(set(&b[1][0][kClose], k_trace<256, false, kClose>));
+    ATR_CUDA(set(&b[1][1][kNear], k_trace<256, true, kNear>));
+    ATR_CUDA(set(&b[1][1][kFar], k_trace<256, true, kFar>));
+    ATR_CUDA(set(&b[1][1][kClose], k_trace<256, true, kClose>));
     return ATR_OK;
 }
 
@@ -430,7 +454,7 @@ int trace_run(atr_ctx* ctx, const int4* nodes, const float4* woop, const int32_t
     }
     int st = ATR_OK;
     const Stepping how =
-        stepping(layout_bytes, n, (int64_t)ctx->num_sms * ctx->trace_blocks[0][0][0] * kTraceThreads);
+        stepping(layout_bytes, n, (int64_t)ctx->num_sms * ctx->trace_blocks[0][0][kNear] * kTraceThreads);
     ctx->phase_begin("trace");
     if (max_depth + 1 < 64)
         launch_trace<64>(ctx, nodes, woop, tri, map, rays, n, any_hit, res, counter, other, how, layout_bytes);

@@ -45,6 +45,27 @@ def test_trace_matches_oracle_at_any_ray_count(ctx, deep, n):
         assert np.array_equal(res.cpu().numpy()[:, :2], want[:, :2])
 
 
+@pytest.mark.parametrize("w,h", [(1, 1), (37, 29), (640, 480)])
+def test_camera_rays_match_oracle(ctx, deep, w, h):
+    """Rays of one origin over a small layout, which are fetched later, and such
+    rays among others."""
+    import torch
+    scene, col, bvh, cp, mn, mx = deep
+    n = w * h
+    assert bvh.view().num_nodes * 64 + bvh.view().num_woop * 16 <= 4_000_000
+    rays = ab.gen_rays_pinhole(w, h).reshape(-1, 8)
+    mixed = rays.copy()
+    mixed[1::3] = ab.gen_rays_random(n, mn, mx, seed=n).reshape(-1, 8)[1::3]
+    for r in (rays, mixed):
+        rd = torch.from_numpy(r).cuda()
+        for any_hit in (False, True):
+            res = torch.full((n, 4), -7, dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            bvh.trace(rd.data_ptr(), n, res.data_ptr(), any_hit=any_hit)
+            ctx.synchronize()
+            assert np.array_equal(res.cpu().numpy()[:, :2], O.trace(cp, r, any_hit=any_hit)[:, :2])
+
+
 def test_captured_trace_replays_beside_direct_ones(ctx, deep):
     """A captured trace keeps a ray counter of its own."""
     import torch
