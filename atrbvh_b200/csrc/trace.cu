@@ -13,8 +13,9 @@
 // same operations.
 //
 // Warps are persistent: lanes whose ray is done wait until fewer than 20 lanes
-// of the warp have work (the reference's dynamic fetch; 16 for the largest
-// layouts), then take new rays from a global counter.  Between two fetches the warp steps as one, every step
+// of the warp have work (the reference's dynamic fetch; 16 in the largest
+// layouts, 8 for a camera's rays in small ones), then take new rays from a global
+// counter.  Between two fetches the warp steps as one, every step
 // either a descent or a leaf test, chosen by vote: left to diverge, the lanes
 // of a warp met again only by chance and an instruction served 6.6 of 32 lanes
 // (1M sorted incoherent rays; 8.8 for pinhole rays); voting serves 11 and 13.
